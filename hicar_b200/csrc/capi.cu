@@ -120,7 +120,6 @@ struct hicarw_handle {
     unsigned int *hscan = nullptr;
     // staging for host pointers
     float *su = nullptr, *sv = nullptr, *sw = nullptr, *sT = nullptr, *srho = nullptr, *sdiv = nullptr;
-    float *sprobe_u = nullptr, *sprobe_v = nullptr, *sprobe_w = nullptr;
     float *swork = nullptr; // cell-sized scratch of balance_uvw (divergence) and smooth_alpha (ping-pong)
     int structure_uploaded = 0, operator_probed = 0, precond_n_sweeps = 2;
     std::map<GraphKey, GraphRec> graphs;
@@ -392,7 +391,7 @@ extern "C" int hicarw_finalize_iter_winds(hicarw_handle *h)
     void *ptrs[] = {h->mjac, h->mju, h->mjv, h->mjw, h->mdzdx, h->mdzdy, h->mdzdx_u, h->mdzdy_v, h->madz, h->mnterr,
                     h->mf[0], h->mf[1], h->mf[2], h->mf[3], h->mf[4], h->dz_if, h->dzdx_surf, h->dzdy_surf, h->adz_col,
                     h->alpha, h->div, h->coef, h->bc, h->st, h->hist, h->partials, h->scan, h->su, h->sv, h->sw,
-                    h->sT, h->srho, h->sdiv, h->sprobe_u, h->sprobe_v, h->sprobe_w, h->swork};
+                    h->sT, h->srho, h->sdiv, h->swork};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (int q = 0; q < NVEC; q++)
@@ -1158,36 +1157,16 @@ extern "C" int hicarw_calibrate_projection_operator(hicarw_handle *h, const floa
     CK(cudaMemcpyAsync(h->alpha, alpha, n_cell(d) * 4, kind, s));
     const float *rho = nullptr;
     if (adv_den && (rc = stage_in(h, density, &h->srho, n_cell(d), mem_kind, s, &rho)) != 0) return rc;
-    // scratch winds (the reference saves u/v/w dqdt, probes in them and restores them;
-    // probing in separate buffers leaves the caller's arrays untouched, same result)
-    if (!h->sprobe_u) {
-        CK(cudaMalloc((void **)&h->sprobe_u, n_u(d) * 4));
-        CK(cudaMalloc((void **)&h->sprobe_v, n_v(d) * 4));
-        CK(cudaMalloc((void **)&h->sprobe_w, n_cell(d) * 4));
-    }
-    if (!h->sT) CK(cudaMalloc((void **)&h->sT, n_cell(d) * 4));
-    if (!h->structure_uploaded) { // the analytic coefficients fill the rows a probe never reaches
-        launch_coefs(d, metrics_of(h), h->alpha, h->coef, 0, s);
+    // the responses of all 27 probes in one pass (k_model.cu); the caller's winds,
+    // which the reference probes in and restores, are not touched
+    if (!h->structure_uploaded) {
         launch_bccol(d, metrics_of(h), h->alpha, h->bc, s);
         h->structure_uploaded = 1;
     }
-    CK(cudaMemsetAsync(h->scan + 3, 0, 4, s));
-    Metrics m = metrics_of(h);
-    for (int cc = 0; cc < 3; cc++)
-        for (int cb = 0; cb < 3; cb++)
-            for (int ca = 0; ca < 3; ca++) {
-                launch_probe_pattern<double>(d, V<double>(h, V_X), ca, cb, cc, s);
-                CK(cudaMemsetAsync(h->sprobe_u, 0, n_u(d) * 4, s));
-                CK(cudaMemsetAsync(h->sprobe_v, 0, n_v(d) * 4, s));
-                CK(cudaMemsetAsync(h->sprobe_w, 0, n_cell(d) * 4, s));
-                launch_winds<double>(d, m, V<double>(h, V_X), h->alpha, rho, h->sprobe_u, h->sprobe_v, h->sprobe_w, adv_den, s);
-                launch_divergence(d, m, h->sprobe_u, h->sprobe_v, h->sprobe_w, rho, h->sT, adv_den, 0, 1, s);
-                launch_probe_record(d, h->sT, h->coef, ca, cb, cc, h->scan + 3, s);
-            }
-    CK(cudaMemcpyAsync(&h->hscan[3], h->scan + 3, 4, cudaMemcpyDeviceToHost, s));
+    launch_calibrate(d, metrics_of(h), h->alpha, rho, adv_den, h->coef, s);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
-    float leak;
-    memcpy(&leak, &h->hscan[3], 4);
+    const float leak = 0.0f; // only stencil neighbours share a face with a cell
     if (max_leak) *max_leak = leak;
     (void)u; (void)v; (void)w;
     return hicarw_probe_finalize(h, leak, stream);
@@ -1216,42 +1195,63 @@ extern "C" int hicarw_get_lambda(hicarw_handle *h, double *lambda, int mem_kind,
     return HICARW_OK;
 }
 
+// The 15 coefficient arrays between the padded layout and the caller's
+// (15, ny, nz, nx): device arrays by one kernel (coalesced along i), host arrays
+// by one strided copy per coefficient.
+__global__ void coefs_copy_kernel(Dims d, float *__restrict__ coef, float *__restrict__ user, int to_user)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, j = blockIdx.z + 1;
+    if (i > d.nx) return;
+    const long long n = (long long)d.nx * d.nz * d.ny, o = kidx(d, i, k, j), c = cidx(d, i, k, j);
+    float v[NCOEF];
+#pragma unroll
+    for (int q = 0; q < NCOEF; q++) v[q] = to_user ? coef[q * d.npad + o] : user[q * n + c];
+#pragma unroll
+    for (int q = 0; q < NCOEF; q++) (to_user ? user[q * n + c] : coef[q * d.npad + o]) = v[q];
+}
+
+static int copy_coefs(hicarw_handle *h, float *user, int to_user, int mem_kind, cudaStream_t s)
+{
+    const Dims &d = h->d;
+    if (mem_kind != HICARW_MEM_HOST) {
+        coefs_copy_kernel<<<dim3((d.nx + 127) / 128, d.nz, d.ny), 128, 0, s>>>(d, h->coef, user, to_user);
+        count_launch(1);
+        CK(cudaGetLastError());
+    } else {
+        for (int c = 0; c < NCOEF; c++) {
+            const cudaPitchedPtr pad = make_cudaPitchedPtr(h->coef + (size_t)c * d.npad + kidx(d, 1, 1, 1),
+                                                           sizeof(float) * d.P, d.nx, d.mz);
+            const cudaPitchedPtr usr = make_cudaPitchedPtr(user + (size_t)c * n_cell(d), sizeof(float) * d.nx, d.nx, d.nz);
+            cudaMemcpy3DParms p = {};
+            p.srcPtr = to_user ? pad : usr;
+            p.dstPtr = to_user ? usr : pad;
+            p.extent = make_cudaExtent(sizeof(float) * d.nx, d.nz, d.ny);
+            p.kind = to_user ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+            CK(cudaMemcpy3DAsync(&p, s));
+        }
+    }
+    CK(cudaStreamSynchronize(s));
+    return HICARW_OK;
+}
+
 extern "C" int hicarw_get_coefs(hicarw_handle *h, float *coefs, int mem_kind, void *stream)
 {
     api_entry();
     if (!h || !coefs) return HICARW_ERR_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    const Dims &d = h->d;
-    cudaMemcpyKind kind = mem_kind == HICARW_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-    for (int c = 0; c < NCOEF; c++) {
-        // interior rows (1..nx, 1..nz, 1..ny) -> (nx, nz, ny)
-        for (int j = 1; j <= d.ny; j++)
-            CK(cudaMemcpy2DAsync(coefs + (size_t)c * n_cell(d) + (size_t)(j - 1) * d.nx * d.nz, sizeof(float) * d.nx,
-                                 h->coef + (size_t)c * d.npad + kidx(d, 1, 1, j), sizeof(float) * d.P,
-                                 sizeof(float) * d.nx, d.nz, kind, s));
-    }
-    CK(cudaStreamSynchronize(s));
-    return HICARW_OK;
+    return copy_coefs(h, coefs, 1, mem_kind, (cudaStream_t)stream);
 }
 
 extern "C" int hicarw_set_coefs(hicarw_handle *h, const float *coefs, int probed, int mem_kind, void *stream)
 {
     api_entry();
     if (!h || !coefs) return HICARW_ERR_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    const Dims &d = h->d;
-    cudaMemcpyKind kind = mem_kind == HICARW_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
-    for (int c = 0; c < NCOEF; c++)
-        for (int j = 1; j <= d.ny; j++)
-            CK(cudaMemcpy2DAsync(h->coef + (size_t)c * d.npad + kidx(d, 1, 1, j), sizeof(float) * d.P,
-                                 coefs + (size_t)c * n_cell(d) + (size_t)(j - 1) * d.nx * d.nz, sizeof(float) * d.nx,
-                                 sizeof(float) * d.nx, d.nz, kind, s));
+    const int rc = copy_coefs(h, const_cast<float *>(coefs), 0, mem_kind, (cudaStream_t)stream);
+    if (rc) return rc;
     h->operator_probed = probed ? 1 : 0;
     h->structure_uploaded = 1;
     h->mg_dirty = h->unet_dirty = 1;
     for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
     h->graphs.clear();
-    CK(cudaStreamSynchronize(s));
     return HICARW_OK;
 }
 

@@ -235,6 +235,161 @@ void launch_probe_record(const Dims &d, const float *T, float *coef, int ca, int
 }
 
 // ---------------------------------------------------------------------------
+// The whole calibration (wind.F90:1010-1099) in one pass.  A cell's divergence
+// reads the corrections of its own six faces, and those read lambda inside the
+// cell's 3 x 3 x 3 neighbourhood, which holds exactly one point of each of the
+// 27 colours; so the response that probe (ca, cb, cc) records at a cell is that
+// of one unit point at one neighbour, and only the 15 neighbours of the stencil
+// share a face with the cell (the other 12 record a response of zero: no
+// leakage).  One thread evaluates the 15 responses of its cell with the
+// statements of winds_kernel and divergence_kernel, the unit point's place
+// known at compile time, terms of untouched faces (exact zeros) left out.
+// What bounds it: the divisions (24 face responses of 8 each), not memory; the
+// 27 probes it replaces wrote and read back lambda, the winds and the
+// divergence in full each time.
+// ---------------------------------------------------------------------------
+// the geometry of one face as the correction and the divergence read it
+struct Face {
+    float half_mf, slope, jac, rho; // 0.5 * map factor, terrain slope, jacobian, correction density
+    float a, b;                     // density factor of the flux: (a + b) / 2 inside, a alone on the outer faces
+    float mf;                       // map factor of the flux
+    bool inner;
+};
+
+// lambda at the relative place (rk, rj, ri) of the unit point at (DK, DJ, DI)
+template <int DK, int DJ, int DI>
+__device__ constexpr float unit(int rk, int rj, int ri)
+{
+    return rk == DK && rj == DJ && ri == DI ? 1.0f : 0.0f;
+}
+
+// the flux through a face of the correction by the unit point; (rj1, ri1) and
+// (rj0, ri0): the cells above and below the face
+template <int DK, int DJ, int DI>
+__device__ __forceinline__ float face_response(const Face &f, int rj1, int ri1, int rj0, int ri0, int k, int nz,
+                                               float dzk1, float dzke, float den, float dx, int adv_den)
+{
+    float dl;
+    const float mean_p = (unit<DK, DJ, DI>(1, rj1, ri1) + unit<DK, DJ, DI>(1, rj0, ri0)) / 2.0f;
+    const float mean_0 = (unit<DK, DJ, DI>(0, rj1, ri1) + unit<DK, DJ, DI>(0, rj0, ri0)) / 2.0f;
+    const float mean_m = (unit<DK, DJ, DI>(-1, rj1, ri1) + unit<DK, DJ, DI>(-1, rj0, ri0)) / 2.0f;
+    if (k == nz) dl = (mean_0 - mean_m) / dzke;
+    else if (k == 1) dl = (mean_p - mean_0) / dzk1;
+    else dl = (mean_p - mean_m) / den;
+    const float grad = (unit<DK, DJ, DI>(0, rj1, ri1) - unit<DK, DJ, DI>(0, rj0, ri0)) / dx - f.slope * (dl) / f.jac;
+    const float u = f.half_mf * grad / (f.rho);
+    if (!adv_den) return u;
+    return f.inner ? u * f.jac * (f.a + f.b) / 2.0f : u * f.jac * f.a;
+}
+
+__global__ void calibrate_kernel(Dims d, Metrics m, const float *__restrict__ alpha, const float *__restrict__ rho,
+                                 int adv_den, float *__restrict__ coef)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, j = blockIdx.z + 1;
+    if (i > d.nx) return;
+    const int nz = d.nz;
+    const float dzk1 = m.dz_if[zidx(d, 1, 2, 1)], dzke = m.dz_if[zidx(d, 1, nz, 1)];
+    const float den = m.dz_if[zidx(d, 1, k + 1, 1)] + m.dz_if[zidx(d, 1, k, 1)];
+    const long long c = cidx(d, i, k, j);
+    auto u_face = [&](int fi) {
+        const long long q = uidx(d, fi, k, j);
+        Face f{0.5f * m.mf_mx_u[i2u(d, fi, j)], m.dzdx_u[q], m.ju[q], 1.0f, 0.0f, 0.0f, m.mf_my_u[i2u(d, fi, j)],
+               fi > 1 && fi <= d.nx};
+        if (adv_den) {
+            if (f.inner) {
+                f.a = rho[cidx(d, fi - 1, k, j)];
+                f.b = rho[cidx(d, fi, k, j)];
+                f.rho = 0.5f * (f.b + f.a);
+            } else {
+                const int e = fi == 1 ? 1 : d.nx, n = fi == 1 ? 2 : d.nx - 1;
+                f.rho = rho[cidx(d, e, k, j)];
+                f.a = 1.5f * f.rho - 0.5f * rho[cidx(d, n, k, j)];
+            }
+        }
+        return f;
+    };
+    auto v_face = [&](int fj) {
+        const long long q = cidx(d, i, k, fj);
+        Face f{0.5f * m.mf_my_v[i2(d, i, fj)], m.dzdy_v[q], m.jv[q], 1.0f, 0.0f, 0.0f, m.mf_mx_v[i2(d, i, fj)],
+               fj > 1 && fj <= d.ny};
+        if (adv_den) {
+            if (f.inner) {
+                f.a = rho[cidx(d, i, k, fj - 1)];
+                f.b = rho[cidx(d, i, k, fj)];
+                f.rho = 0.5f * (f.b + f.a);
+            } else {
+                const int e = fj == 1 ? 1 : d.ny, n = fj == 1 ? 2 : d.ny - 1;
+                f.rho = rho[cidx(d, i, k, e)];
+                f.a = 1.5f * f.rho - 0.5f * rho[cidx(d, i, k, n)];
+            }
+        }
+        return f;
+    };
+    const Face u0 = u_face(i), u1 = u_face(i + 1), v0 = v_face(j), v1 = v_face(j + 1);
+    const float mxy = m.mf_mxy[i2(d, i, j)], adz = m.adz[c], jac = m.jac[c];
+    // the w levels k and k - 1: alpha^2 / 2, the level distance, the jacobian, the density
+    auto w_density = [&](int kk) {
+        if (!adv_den) return 1.0f;
+        const long long q = cidx(d, i, kk, j), qp = cidx(d, i, kk + 1, j);
+        return (rho[q] * m.adz[qp] + rho[qp] * m.adz[q]) / (m.adz[q] + m.adz[qp]);
+    };
+    // flux of the w correction by a lambda difference dlam (level kk + 1 minus kk)
+    auto w_response = [&](int kk, float dlam) {
+        const long long q = cidx(d, i, kk, j);
+        const float a = alpha[q], jw = m.jw[q], rho_w = w_density(kk);
+        const float w = 0.5f * (a * a) * dlam / m.dz_if[zidx(d, i, kk + 1, j)] / jw / rho_w;
+        return adv_den ? w * jw * rho_w : w * jw;
+    };
+    // 2 T from the horizontal sum and the w fluxes of levels k and k - 1
+    auto store = [&](int slot, bool in, float sum, float wk, float wm) {
+        float dv = mxy * sum / d.dx;
+        if (k == 1) dv = dv + wk / (adz);
+        else dv = dv + (wk - wm) / (adz);
+        coef[(long long)slot * d.npad + kidx(d, i, k, j)] = in ? 2.0f * (dv / jac) : 0.0f;
+    };
+#define U1(DK, DJ, DI) face_response<DK, DJ, DI>(u1, 0, 1, 0, 0, k, nz, dzk1, dzke, den, d.dx, adv_den)
+#define U0(DK, DJ, DI) face_response<DK, DJ, DI>(u0, 0, 0, 0, -1, k, nz, dzk1, dzke, den, d.dx, adv_den)
+#define V1(DK, DJ, DI) face_response<DK, DJ, DI>(v1, 1, 0, 0, 0, k, nz, dzk1, dzke, den, d.dx, adv_den)
+#define V0(DK, DJ, DI) face_response<DK, DJ, DI>(v0, 0, 0, -1, 0, k, nz, dzk1, dzke, den, d.dx, adv_den)
+    const bool up = k < nz, dn = k > 1;
+    // the cell's own column: all four side faces and the w levels
+    const float wk_p = up ? w_response(k, 1.0f) : 0.0f, wm_p = dn ? w_response(k - 1, 1.0f) : 0.0f;
+    const float wk_m = up ? w_response(k, -1.0f) : 0.0f, wm_m = dn ? w_response(k - 1, -1.0f) : 0.0f;
+#define OWN(DK) \
+    (U1(DK, 0, 0) / u1.mf - U0(DK, 0, 0) / u0.mf + V1(DK, 0, 0) / v1.mf - V0(DK, 0, 0) / v0.mf)
+    store(CA, true, OWN(0), wk_m, wm_p);
+    store(CB, up, OWN(1), wk_p, 0.0f);
+    store(CC, dn, OWN(-1), 0.0f, wm_m);
+    // the neighbouring columns: the face they share with the cell
+    const bool e = i < d.nx, w = i > 1, n = j < d.ny, s = j > 1;
+    store(CD, e, U1(0, 0, 1) / u1.mf, 0.0f, 0.0f);
+    store(CE, w, -(U0(0, 0, -1) / u0.mf), 0.0f, 0.0f);
+    store(CF, n, V1(0, 1, 0) / v1.mf, 0.0f, 0.0f);
+    store(CG, s, -(V0(0, -1, 0) / v0.mf), 0.0f, 0.0f);
+    store(CH, e && up, U1(1, 0, 1) / u1.mf, 0.0f, 0.0f);
+    store(CI, w && up, -(U0(1, 0, -1) / u0.mf), 0.0f, 0.0f);
+    store(CJ, e && dn, U1(-1, 0, 1) / u1.mf, 0.0f, 0.0f);
+    store(CK, w && dn, -(U0(-1, 0, -1) / u0.mf), 0.0f, 0.0f);
+    store(CL, n && up, V1(1, 1, 0) / v1.mf, 0.0f, 0.0f);
+    store(CM, s && up, -(V0(1, -1, 0) / v0.mf), 0.0f, 0.0f);
+    store(CN, n && dn, V1(-1, 1, 0) / v1.mf, 0.0f, 0.0f);
+    store(CO, s && dn, -(V0(-1, -1, 0) / v0.mf), 0.0f, 0.0f);
+#undef OWN
+#undef U1
+#undef U0
+#undef V1
+#undef V0
+}
+
+void launch_calibrate(const Dims &d, const Metrics &m, const float *alpha, const float *rho, int adv_den, float *coef,
+                      cudaStream_t st)
+{
+    dim3 b(128), g((d.nx + 127) / 128, d.nz, d.ny);
+    calibrate_kernel<<<g, b, 0, st>>>(d, m, alpha, rho, adv_den, coef);
+    count_launch(1);
+}
+
+// ---------------------------------------------------------------------------
 // init_module_vars (:2274-2421): dz_if, dzdx_surf, dzdy_surf, adv_dz_col.
 // ---------------------------------------------------------------------------
 __global__ void module_vars_kernel(Dims d, const float *__restrict__ adz, const float *__restrict__ dzdx,

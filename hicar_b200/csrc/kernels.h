@@ -26,6 +26,8 @@ template <typename V>
 void launch_probe_pattern(const Dims &d, V *x, int ca, int cb, int cc, cudaStream_t st);
 void launch_probe_record(const Dims &d, const float *T, float *coef, int ca, int cb, int cc, unsigned int *leak,
                          cudaStream_t st);
+void launch_calibrate(const Dims &d, const Metrics &m, const float *alpha, const float *rho, int adv_den, float *coef,
+                      cudaStream_t st);
 void launch_w_real(const Dims &d, const Metrics &m, const float *u, const float *v, const float *w_grid, float *w_real,
                    cudaStream_t st);
 void launch_idealized_wgrid(const Dims &d, const Metrics &m, const float *u, const float *v, const float *w_real_field,

@@ -1,0 +1,76 @@
+"""GPU tests of the one-pass calibration (calibrate_kernel) against the
+reference's probe hooks run one colour at a time, and of the coefficient copies
+between the padded and the caller's layout."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from hicar_b200 import _capi, cases
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(autouse=True)
+def _fresh(lib):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from hicar_b200 import wind, wind_iterative
+    wind_iterative.finalize_iter_winds()
+    wind.reset()
+    yield
+    wind_iterative.finalize_iter_winds()
+    wind.reset()
+
+
+def _coefs(dom, host):
+    from hicar_b200 import wind_iterative as wi
+    h, shape = wi.handle(dom.nest_indx), (15, dom.ny, dom.nz, dom.nx)
+    if host:
+        out = np.empty(shape, np.float32)
+        _capi.check(_capi.load().hicarw_get_coefs(h, out.ctypes.data, _capi.MEM_HOST, None), h)
+        return out
+    out = torch.empty(shape, dtype=torch.float32, device="cuda")
+    _capi.check(_capi.load().hicarw_get_coefs(h, C.c_void_p(out.data_ptr()), _capi.MEM_DEVICE, None), h)
+    return out.cpu().numpy()
+
+
+# smallest extents (every face an outer one, nz = 2: no inner level), block edges, odd sizes
+@pytest.mark.parametrize("shape", [(3, 3, 2), (4, 5, 3), (129, 4, 2), (128, 7, 5), (37, 41, 9)])
+@pytest.mark.parametrize("adv", [True, False])
+def test_one_pass_calibration_equals_the_probe_hooks(shape, adv):
+    from hicar_b200 import wind, wind_iterative as wi
+    from hicar_b200.domain import DeviceDomain
+    case = cases.build_case(*shape, seed=11, adv_den=adv, n_hills=3, alpha="smooth")
+    dom = DeviceDomain.from_case(case, "cuda")
+    opt = wi.WindOptions(advect_density=adv)
+    wi.init_iter_winds(dom, opt)
+    leak = wind.calibrate_projection_operator(dom, opt)
+    one = _coefs(dom, host=False)
+    np.testing.assert_array_equal(one, _coefs(dom, host=True))
+    winds = [a.clone() for a in (dom.u_dqdt, dom.v_dqdt, dom.w_dqdt)]
+    div = torch.empty((dom.ny, dom.nz, dom.nx), dtype=torch.float32, device="cuda")
+    leak_hooks = wind.calibrate_projection_operator(dom, opt, div, on_device=False)
+    np.testing.assert_array_equal(one, _coefs(dom, host=False))
+    assert leak == leak_hooks
+    for a, b in zip(winds, (dom.u_dqdt, dom.v_dqdt, dom.w_dqdt)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 2), (130, 5, 3)])
+@pytest.mark.parametrize("host", [True, False])
+def test_coefficients_round_trip(shape, host):
+    from hicar_b200 import wind_iterative as wi
+    from hicar_b200.domain import DeviceDomain
+    case = cases.build_case(*shape, seed=3, adv_den=True, n_hills=3)
+    dom = DeviceDomain.from_case(case, "cuda")
+    wi.init_iter_winds(dom, wi.WindOptions())
+    h, lib = wi.handle(dom.nest_indx), _capi.load()
+    rng = np.random.default_rng(1)
+    a = rng.standard_normal((15, dom.ny, dom.nz, dom.nx)).astype(np.float32)
+    t = torch.from_numpy(a).cuda()
+    src = a.ctypes.data if host else t.data_ptr()
+    _capi.check(lib.hicarw_set_coefs(h, C.c_void_p(src), 1, _capi.MEM_HOST if host else _capi.MEM_DEVICE, None), h)
+    np.testing.assert_array_equal(_coefs(dom, host=True), a)
+    np.testing.assert_array_equal(_coefs(dom, host=False), a)
