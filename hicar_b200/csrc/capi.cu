@@ -199,6 +199,24 @@ static int mg_build_tuned(hicarw_handle *h, cudaStream_t s)
     return 0;
 }
 
+// The V-cycle for the handle's present coefficients and options, built or
+// refreshed where it is not: 1 when anything was made again, 0 when it stood,
+// negative on failure.  Never inside a stream capture.
+static int mg_ensure(hicarw_handle *h, cudaStream_t s)
+{
+    if (h->mg_dirty || !h->mg.ready) {
+        mg_params(h);
+        if (mg_build_tuned(h, s) != 0) {
+            h->err = "multigrid build failed";
+            return HICARW_ERR_CUDA;
+        }
+        h->mg_dirty = 0;
+        return 1;
+    }
+    const int rc = mg_refresh(h->mg, s);
+    return rc < 0 ? HICARW_ERR_CUDA : rc;
+}
+
 static Metrics metrics_of(const hicarw_handle *h)
 {
     Metrics m;
@@ -608,11 +626,7 @@ static int bicgstab_solve(hicarw_handle *h, int sweeps, cudaStream_t s, int allo
 {
     int rc;
     select_precond(h, allow_mg);
-    if (h->use_mg && (h->mg_dirty || !h->mg.ready)) {
-        mg_params(h);
-        if (mg_build_tuned(h, s) != 0) { h->err = "multigrid build failed"; return HICARW_ERR_CUDA; }
-        h->mg_dirty = 0;
-    }
+    if (h->use_mg && (rc = mg_ensure(h, s)) < 0) return rc;
     if (h->opt.solver == HICARW_SOLVER_FGMRES) return fgmres_solve(h, sweeps, s);
     const int solver = h->opt.solver;
     const int prec = prec_in >= 0 ? prec_in : solve_precision(h);
@@ -1315,11 +1329,7 @@ extern "C" int hicarw_apply_precond(hicarw_handle *h, const double *x, double *y
         else h->unet_dirty = 0;
     }
     if (!rc && sweeps <= 0) {
-        if ((h->mg_dirty || !h->mg.ready) && !(learned && h->opt.precond == HICARW_PRECOND_LEARNED)) {
-            mg_params(h);
-            if (mg_build_tuned(h, s) != 0) rc = HICARW_ERR_CUDA;
-            else h->mg_dirty = 0;
-        }
+        if (!(learned && h->opt.precond == HICARW_PRECOND_LEARNED)) rc = std::min(0, mg_ensure(h, s));
         if (!rc) {
             CK(cudaMemsetAsync(by, 0, (size_t)d.npad * 8, s));
             if (learned && h->opt.precond == HICARW_PRECOND_LEARNED) unet_precond(h->unet, opctx(h), bx, by, nullptr, s);
@@ -1419,10 +1429,7 @@ extern "C" int hicarw_profile_iteration(hicarw_handle *h, int reps, char *names,
         if (unet_prepare_operator(h->unet, opctx(h), s) != 0) return HICARW_ERR_ARG;
         h->unet_dirty = 0;
     }
-    if (h->use_mg && (h->mg_dirty || !h->mg.ready)) {
-        if (mg_build_tuned(h, s) != 0) return HICARW_ERR_CUDA;
-        h->mg_dirty = 0;
-    }
+    if (h->use_mg && (rc = mg_ensure(h, s)) < 0) return rc;
     FgmresCtx fg;
     if (solver == HICARW_SOLVER_FGMRES) {
         if ((rc = fgmres_prepare(h, h->precond_n_sweeps, &fg)) != 0) return rc;
@@ -1594,11 +1601,7 @@ extern "C" int hicarw_dist_setup(hicarw_handle *h, const double *rhs, double *to
     cudaStream_t s = (cudaStream_t)stream;
     select_precond(h, 1);
     if (h->use_learned || h->use_mglearned) return HICARW_ERR_STATE;
-    if (h->use_mg && (h->mg_dirty || !h->mg.ready)) {
-        mg_params(h);
-        if (mg_build_tuned(h, s) != 0) return HICARW_ERR_CUDA;
-        h->mg_dirty = 0;
-    }
+    if (h->use_mg && (rc = mg_ensure(h, s)) < 0) return rc;
     if ((rc = ensure_vectors(h, HICARW_KRYLOV_F64)) != 0) return rc;
     if ((rc = put_padded(h, rhs, V<double>(h, V_RHS), mem_kind, s)) != 0) return rc;
     launch_diag<double>(h->d, h->coef, h->dz_if, V<double>(h, V_DINV), h->operator_probed, s);
@@ -1641,6 +1644,7 @@ extern "C" int hicarw_dist_precond(hicarw_handle *h, int which, void *stream)
     SolveState *st = h->st;
     double *r = V<double>(h, V_R), *p = V<double>(h, V_P), *phat = V<double>(h, V_PHAT), *v = V<double>(h, V_V),
            *sv = V<double>(h, V_S), *shat = V<double>(h, V_SHAT), *Dinv = V<double>(h, V_DINV);
+    if (h->use_mg && (rc = mg_ensure(h, s)) < 0) return rc;
     if (which == 0) {
         launch_iteration_begin(st, s);
         if (h->use_mg) mg_apply<double>(h->mg, p, phat, st, s);
@@ -1994,12 +1998,10 @@ static int batch_run(hicarw_batch *b, const hicarw_batch_item *items, int adv_de
         hicarw_handle *h = b->hs[i];
         h->launches_at_call = g_launches.load();
         select_precond(h, 1);
-        if (h->use_mg && (h->mg_dirty || !h->mg.ready)) {
-            mg_params(h);
-            if (mg_build_tuned(h, s) != 0)
+        if (h->use_mg) {
+            if ((rc = mg_ensure(h, s)) < 0)
                 return batch_fail(HICARW_ERR_CUDA, "multigrid build of subdomain " + std::to_string(i) + ": " + h->err);
-            h->mg_dirty = 0;
-            rebuild = true;
+            if (rc) rebuild = true;
         }
         if (h->opt.solver == HICARW_SOLVER_FGMRES) {
             const bool dirty = (h->use_learned || h->use_mglearned) && h->unet_dirty;

@@ -1236,6 +1236,207 @@ __global__ void __launch_bounds__(MG_FUSE_THREADS) coarse_cycle_kernel(const __g
 }
 
 // ---------------------------------------------------------------------------
+// Dense coarse cycle.  From a level of at most MG_DENSE_MAX unknowns down, the
+// cycle (its pre-smoothing, W repeats and post-smoothings included) is a fixed
+// linear map of that level's right-hand side, so the build tabulates it as one
+// n x n matrix and a visit is one matrix-vector product: two short launches
+// (restriction, product) in the place of a chain of 8 to 44 dependent steps on
+// levels too small to hide a memory latency.  The columns are the cycle applied
+// to the unit vectors, in FP64 with the levels' FP32 coefficients and Thomas
+// factors, rounded once to FP32; the product accumulates in FP32, 32 partial
+// sums per row.
+// What bounds it: the launch and one L2 round trip (n = 1024: 4 MB of matrix,
+// read once per visit by rows spread over the whole chip).  n <= 2048 keeps
+// the matrix at 16 MB, a few us from L2 or HBM.  A solve to 1e-9 (B200): 64x64x20
+// 8.29 -> 2.92 ms, 181x157x33 17.7 -> 9.7 ms, 512x512x48 52.5 -> 45.3 ms.
+// ---------------------------------------------------------------------------
+constexpr int MG_DENSE_MAX = 2048;
+constexpr int DN_THREADS = 128;
+
+__device__ __forceinline__ int dense_index(const Dims &d, int i, int k, int j)
+{
+    return ((j - 1) * d.nz + k - 1) * d.nx + i - 1;
+}
+
+// rd = R^T (r_f - A_f x1_f) of the dense level's cells, compact order; four
+// lanes per coarse cell, one per child, every operand straight from memory so
+// that all of a thread's loads are in flight together.
+template <typename TR, bool NOX>
+__global__ void __launch_bounds__(DN_THREADS) dense_restrict_kernel(Dims f, const float *__restrict__ coef_f,
+                                                                    const TR *__restrict__ r_f,
+                                                                    const float *__restrict__ x1_f, Dims dc, int n,
+                                                                    float *__restrict__ rd, const SolveState *gate)
+{
+    if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
+    const int t = blockIdx.x * DN_THREADS + threadIdx.x, cell = t >> 2, child = t & 3;
+    double acc = 0.0;
+    if (cell < n) {
+        const int I = cell % dc.nx + 1, row = cell / dc.nx, k = row % dc.nz + 1, J = row / dc.nz + 1;
+        const int i = 2 * I - 1 + (child & 1), j = 2 * J - 1 + (child >> 1);
+        if (i <= f.nx && j <= f.ny) {
+            const long long o = kidx(f, i, k, j);
+            if (NOX) {
+                acc = (double)r_f[o];
+            } else {
+                float cv[15], xv[15];
+                load_coefs(coef_f, f.npad, o, cv);
+#pragma unroll
+                for (int q = 0; q < 15; q++)
+                    xv[q] = inside(f, i + off_i(q), k + off_k(q), j + off_j(q))
+                                ? x1_f[o + off_i(q) + off_k(q) * (long long)f.P + off_j(q) * f.plane]
+                                : 0.0f;
+                float y = 0.0f;
+#pragma unroll
+                for (int q = 0; q < 15; q++) y = fmaf(cv[q], xv[q], y);
+                acc = (double)r_f[o] - (double)y;
+            }
+        }
+    }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+    if (cell < n && child == 0) rd[cell] = (float)acc;
+}
+
+// x = S rd, one warp per row (ld: row length in floats, a multiple of 128; the
+// padding of S and rd is zero), x in the level's padded layout.
+__global__ void __launch_bounds__(DN_THREADS) dense_apply_kernel(const float *__restrict__ S, int n, int ld,
+                                                                 const float *__restrict__ rd, Dims d,
+                                                                 float *__restrict__ x, const SolveState *gate)
+{
+    if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
+    const int row = blockIdx.x * (DN_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= n) return;
+    const float4 *sr = reinterpret_cast<const float4 *>(S + (size_t)row * ld), *rr = reinterpret_cast<const float4 *>(rd);
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    constexpr int U = 8; // 1024 columns in flight
+    for (int b = lane; b < ld / 4; b += 32 * U) {
+        float4 a[U], v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) a[u] = b + 32 * u < ld / 4 ? __ldg(sr + b + 32 * u) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = b + 32 * u < ld / 4 ? rr[b + 32 * u] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            acc.x = fmaf(a[u].x, v[u].x, acc.x);
+            acc.y = fmaf(a[u].y, v[u].y, acc.y);
+            acc.z = fmaf(a[u].z, v[u].z, acc.z);
+            acc.w = fmaf(a[u].w, v[u].w, acc.w);
+        }
+    }
+    float y = (acc.x + acc.y) + (acc.z + acc.w);
+    for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    if (lane == 0) x[kidx(d, row % d.nx + 1, row / d.nx % d.nz + 1, row / (d.nx * d.nz) + 1)] = y;
+}
+
+// ---- tabulating the matrix: the cycle's steps on n right-hand sides at once,
+// FP64, vectors as [cell][right-hand side] (coalesced over the right-hand
+// sides), x = nullptr standing for zero and r = nullptr for the unit vectors ----
+__device__ __forceinline__ double table_at(const double *x, const Dims &d, int i, int k, int j, int n, int q)
+{
+    return x && inside(d, i, k, j) ? x[(size_t)dense_index(d, i, k, j) * n + q] : 0.0;
+}
+
+// rc = R^T (r - A x), one thread per (coarse cell, right-hand side)
+__global__ void table_restrict_kernel(Dims f, const float *__restrict__ coef, const double *__restrict__ r,
+                                      const double *__restrict__ x, Dims dc, double *__restrict__ rc, int n)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, cell = blockIdx.y;
+    if (q >= n) return;
+    const int I = cell % dc.nx + 1, row = cell / dc.nx, k = row % dc.nz + 1, J = row / dc.nz + 1;
+    double acc = 0.0;
+    for (int child = 0; child < 4; child++) {
+        const int i = 2 * I - 1 + (child & 1), j = 2 * J - 1 + (child >> 1);
+        if (i > f.nx || j > f.ny) continue;
+        const int fc = dense_index(f, i, k, j);
+        double y = r ? r[(size_t)fc * n + q] : (fc == q ? 1.0 : 0.0);
+        const long long o = kidx(f, i, k, j);
+#pragma unroll
+        for (int s = 0; s < 15; s++)
+            y -= (double)coef[(long long)s * f.npad + o] * table_at(x, f, i + off_i(s), k + off_k(s), j + off_j(s), n, q);
+        acc += y;
+    }
+    rc[(size_t)cell * n + q] = acc;
+}
+
+// res = r - A x2 with x2 = x + cs P xc, one thread per (cell, right-hand side)
+__global__ void table_residual_kernel(Dims d, const float *__restrict__ coef, const double *__restrict__ r,
+                                      const double *__restrict__ x, Dims dc, const double *__restrict__ xc, double cs,
+                                      double *__restrict__ res, int n)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, cell = blockIdx.y;
+    if (q >= n) return;
+    const int i = cell % d.nx + 1, row = cell / d.nx, k = row % d.nz + 1, j = row / d.nz + 1;
+    double y = r ? r[(size_t)cell * n + q] : (cell == q ? 1.0 : 0.0);
+    const long long o = kidx(d, i, k, j);
+#pragma unroll
+    for (int s = 0; s < 15; s++) {
+        const int ii = i + off_i(s), kk = k + off_k(s), jj = j + off_j(s);
+        if (!inside(d, ii, kk, jj)) continue;
+        y -= (double)coef[(long long)s * d.npad + o] *
+             (table_at(x, d, ii, kk, jj, n, q) + cs * table_at(xc, dc, (ii + 1) >> 1, kk, (jj + 1) >> 1, n, q));
+    }
+    res[(size_t)cell * n + q] = y;
+}
+
+// out = x2 + w T^-1 res (x2 as above, zero where x and xc are null), one thread
+// per (column, right-hand side); the operands of TABLE_U levels are read ahead
+constexpr int TABLE_U = 8;
+__global__ void table_columns_kernel(Dims d, const float *__restrict__ coef, const float *__restrict__ cp,
+                                     const float *__restrict__ minv, const double *__restrict__ res,
+                                     const double *__restrict__ x, Dims dc, const double *__restrict__ xc, double cs,
+                                     double omega, double *out, int n)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y % d.nx + 1, j = blockIdx.y / d.nx + 1;
+    if (q >= n) return;
+    double dp = 0.0;
+    for (int k0 = 1; k0 <= d.nz; k0 += TABLE_U) {
+        double rv[TABLE_U];
+        float cv[TABLE_U], mv[TABLE_U];
+#pragma unroll
+        for (int u = 0; u < TABLE_U; u++) {
+            const int k = k0 + u;
+            const bool in = k <= d.nz;
+            const int cell = dense_index(d, i, in ? k : d.nz, j);
+            const long long o = kidx(d, i, in ? k : d.nz, j);
+            rv[u] = res ? res[(size_t)cell * n + q] : (cell == q ? 1.0 : 0.0);
+            cv[u] = k > 1 ? coef[(long long)CC * d.npad + o] : 0.0f;
+            mv[u] = minv[o];
+        }
+#pragma unroll
+        for (int u = 0; u < TABLE_U; u++)
+            if (k0 + u <= d.nz) {
+                dp = (rv[u] - (double)cv[u] * dp) * (double)mv[u];
+                out[(size_t)dense_index(d, i, k0 + u, j) * n + q] = dp;
+            }
+    }
+    double y = 0.0;
+    for (int k0 = d.nz; k0 >= 1; k0 -= TABLE_U) {
+        double rv[TABLE_U], bv[TABLE_U];
+        float pv[TABLE_U];
+#pragma unroll
+        for (int u = 0; u < TABLE_U; u++) {
+            const int k = max(k0 - u, 1);
+            rv[u] = out[(size_t)dense_index(d, i, k, j) * n + q];
+            pv[u] = cp[kidx(d, i, k, j)];
+            bv[u] = table_at(x, d, i, k, j, n, q) + cs * table_at(xc, dc, (i + 1) >> 1, k, (j + 1) >> 1, n, q);
+        }
+#pragma unroll
+        for (int u = 0; u < TABLE_U; u++)
+            if (k0 - u >= 1) {
+                y = rv[u] - (double)pv[u] * y;
+                out[(size_t)dense_index(d, i, k0 - u, j) * n + q] = bv[u] + omega * y;
+            }
+    }
+}
+
+// S = x rounded to FP32, rows padded to ld
+__global__ void table_store_kernel(const double *__restrict__ x, int n, int ld, float *__restrict__ S)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y;
+    if (q < ld) S[(size_t)row * ld + q] = q < n ? (float)x[(size_t)row * n + q] : 0.0f;
+}
+
+// ---------------------------------------------------------------------------
 static Dims level_dims(int nx, int ny, int nz, float dx)
 {
     Dims d;
@@ -1246,6 +1447,14 @@ static Dims level_dims(int nx, int ny, int nz, float dx)
     d.npad = d.plane * d.my;
     d.dx = dx;
     return d;
+}
+
+static void dense_free(Mg &mg)
+{
+    if (mg.dense) cudaFree(mg.dense);
+    if (mg.dense_r) cudaFree(mg.dense_r);
+    mg.dense = mg.dense_r = nullptr;
+    mg.dense_level = 0;
 }
 
 void mg_free(Mg &mg)
@@ -1266,12 +1475,14 @@ void mg_free(Mg &mg)
     mg.err = nullptr;
     if (mg.coef0h) cudaFree(mg.coef0h);
     mg.coef0h = nullptr;
+    dense_free(mg);
 }
 
 static int sm_count();
 static int smem_optin();
 static int smem_per_sm();
 static void fused_setup(Mg &mg);
+static bool dense_setup(Mg &mg, cudaStream_t s);
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 
 __global__ void bf16_copy_kernel(const float *__restrict__ in, __nv_bfloat16 *__restrict__ out, size_t n)
@@ -1355,7 +1566,8 @@ int mg_build(Mg &mg, const Dims &fine, const float *fine_coef, cudaStream_t s)
         mg.coef0h = nullptr;
     }
     const cudaError_t e = cudaGetLastError();
-    fused_setup(mg);
+    mg.fuse_level = mg.cluster_n = 0;
+    if (!dense_setup(mg, s)) fused_setup(mg);
     mg.ready = 1;
     return e == cudaSuccess ? 0 : -1;
 }
@@ -1850,6 +2062,131 @@ static bool launch_fused(const Mg &mg, int l, const SolveState *gate, cudaStream
     return true;
 }
 
+// ---- dense coarse cycle: where it starts, tabulation, launches ----
+static dim3 table_grid(int n, int y) { return dim3((n + 127) / 128, y); }
+
+// The cycle of level l (its pre-smoothed iterate in x1) on the unit vectors;
+// returns the buffer that holds its result.
+static double *tabulate(const Mg &mg, int l, double *const *r, double *const *x1, double *const *x3, double *res, int n,
+                        cudaStream_t s)
+{
+    if (l == mg.nlev - 1) return x1[l];
+    const MgLevel &F = mg.lev[l], &C = mg.lev[l + 1];
+    const bool last = l + 1 == mg.nlev - 1;
+    const int cells = F.d.nx * F.d.ny * F.d.nz, ccells = C.d.nx * C.d.ny * C.d.nz;
+    double *cur = x1[l], *other = x3[l];
+    for (int rep = 0; rep < ((mg.wmask >> l) & 1 ? 2 : 1); rep++) {
+        table_restrict_kernel<<<table_grid(n, ccells), 128, 0, s>>>(F.d, F.coef, r[l], cur, C.d, r[l + 1], n);
+        table_columns_kernel<<<table_grid(n, C.d.nx * C.d.ny), 128, 0, s>>>(
+            C.d, C.coef, C.cp, C.minv, r[l + 1], nullptr, C.d, nullptr, 0.0, last ? 1.0 : (double)mg.omega, x1[l + 1], n);
+        const double *xc = tabulate(mg, l + 1, r, x1, x3, res, n, s);
+        table_residual_kernel<<<table_grid(n, cells), 128, 0, s>>>(F.d, F.coef, r[l], cur, C.d, xc, (double)mg.cscale,
+                                                                   res, n);
+        table_columns_kernel<<<table_grid(n, F.d.nx * F.d.ny), 128, 0, s>>>(F.d, F.coef, F.cp, F.minv, res, cur, C.d, xc,
+                                                                            (double)mg.cscale, (double)mg.omega, other, n);
+        count_launch(4);
+        std::swap(cur, other);
+    }
+    return cur;
+}
+
+// Tabulate the cycle from mg.dense_level down into mg.dense with the present
+// cycle parameters; false when there is no memory for it.
+static bool dense_fill(Mg &mg, cudaStream_t s)
+{
+    const int l0 = mg.dense_level, n = mg.dense_n;
+    double *r[MG_MAX_LEVELS] = {}, *x1[MG_MAX_LEVELS] = {}, *x3[MG_MAX_LEVELS] = {}, *buf = nullptr;
+    size_t total = 0;
+    auto size = [&](int l) { return (size_t)mg.lev[l].d.nx * mg.lev[l].d.ny * mg.lev[l].d.nz * n; };
+    for (int l = l0; l < mg.nlev; l++) total += size(l) * (l == l0 ? 2 : 3);
+    total += size(l0); // residuals
+    if (cudaMallocAsync((void **)&buf, total * sizeof(double), s) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    double *p = buf;
+    for (int l = l0; l < mg.nlev; l++) {
+        if (l > l0) { r[l] = p; p += size(l); }
+        x1[l] = p; p += size(l);
+        x3[l] = p; p += size(l);
+    }
+    const MgLevel &T = mg.lev[l0];
+    table_columns_kernel<<<table_grid(n, T.d.nx * T.d.ny), 128, 0, s>>>(
+        T.d, T.coef, T.cp, T.minv, nullptr, nullptr, T.d, nullptr, 0.0, l0 == mg.nlev - 1 ? 1.0 : (double)mg.omega, x1[l0], n);
+    const double *x = tabulate(mg, l0, r, x1, x3, p, n, s);
+    table_store_kernel<<<dim3((mg.dense_ld + 127) / 128, n), 128, 0, s>>>(x, n, mg.dense_ld, mg.dense);
+    count_launch(2);
+    cudaFreeAsync(buf, s);
+    mg.dense_omega = mg.omega;
+    mg.dense_cscale = mg.cscale;
+    mg.dense_wmask = mg.wmask;
+    return cudaGetLastError() == cudaSuccess;
+}
+
+// The coarse part as a dense matrix (the default; HICARW_MG_FUSE set in the
+// environment selects the step-by-step forms below).  False when it does not
+// apply: no level has few enough unknowns, or no memory.
+static bool dense_setup(Mg &mg, cudaStream_t s)
+{
+    int l0 = 0;
+    if (!getenv("HICARW_MG_FUSE"))
+        for (int l = 1; l < mg.nlev && !l0; l++)
+            if ((long long)mg.lev[l].d.nx * mg.lev[l].d.ny * mg.lev[l].d.nz <= MG_DENSE_MAX) l0 = l;
+    // a level cut off by MG_MAX_LEVELS is not a single column: the step-by-step forms handle it
+    if (mg.lev[mg.nlev - 1].d.nx != 1 || mg.lev[mg.nlev - 1].d.ny != 1) l0 = 0;
+    if (l0 != mg.dense_level) dense_free(mg);
+    if (!l0) return false;
+    mg.dense_n = mg.lev[l0].d.nx * mg.lev[l0].d.ny * mg.lev[l0].d.nz;
+    mg.dense_ld = (mg.dense_n + 127) / 128 * 128;
+    mg.dense_level = l0;
+    if (!mg.dense) {
+        if (cudaMalloc((void **)&mg.dense, (size_t)mg.dense_n * mg.dense_ld * sizeof(float)) != cudaSuccess ||
+            cudaMalloc((void **)&mg.dense_r, mg.dense_ld * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            dense_free(mg);
+            return false;
+        }
+        cudaMemsetAsync(mg.dense_r, 0, mg.dense_ld * sizeof(float), s);
+    }
+    if (dense_fill(mg, s)) return true;
+    dense_free(mg);
+    return false;
+}
+
+// Before the launches of a cycle are enqueued: the dense matrix belongs to the
+// cycle's present parameters.  1: it was tabulated again, 0: it stands, -1: error.
+int mg_refresh(Mg &mg, cudaStream_t s)
+{
+    if (!mg.ready || !mg.dense_level ||
+        (mg.dense_omega == mg.omega && mg.dense_cscale == mg.cscale && mg.dense_wmask == mg.wmask))
+        return 0;
+    return dense_fill(mg, s) ? 1 : -1;
+}
+
+static const char *kDenseName[MG_MAX_LEVELS] = {
+    "mg_dense_l0", "mg_dense_l1", "mg_dense_l2",  "mg_dense_l3",  "mg_dense_l4",  "mg_dense_l5",  "mg_dense_l6", "mg_dense_l7",
+    "mg_dense_l8", "mg_dense_l9", "mg_dense_l10", "mg_dense_l11", "mg_dense_l12", "mg_dense_l13", "mg_dense_l14", "mg_dense_l15"};
+
+// Level C = mg.dense_level's result from level F's residual (x1 zero with nox).
+template <typename TR>
+static const float *dense_visit(const Mg &mg, const MgLevel &F, const TR *r, const SolveState *gate, cudaStream_t s,
+                                bool nox)
+{
+    const MgLevel &C = mg.lev[mg.dense_level];
+    const double N = (double)F.d.nx * F.d.ny * F.d.nz;
+    const int n = mg.dense_n, g = (4 * n + DN_THREADS - 1) / DN_THREADS, rows = DN_THREADS / 32;
+    {
+        ProfScope ps_(kLevelName[2][mg.dense_level], nox ? sizeof(TR) * N + 4.0 * n : (60.0 + sizeof(TR) + 4.0) * N, s);
+        if (nox) dense_restrict_kernel<TR, true><<<g, DN_THREADS, 0, s>>>(F.d, F.coef, r, F.x1, C.d, n, mg.dense_r, gate);
+        else dense_restrict_kernel<TR, false><<<g, DN_THREADS, 0, s>>>(F.d, F.coef, r, F.x1, C.d, n, mg.dense_r, gate);
+        count_launch(1);
+    }
+    ProfScope ps_(kDenseName[mg.dense_level], 4.0 * n * (mg.dense_ld + 2.0), s);
+    dense_apply_kernel<<<(n + rows - 1) / rows, DN_THREADS, 0, s>>>(mg.dense, n, mg.dense_ld, mg.dense_r, C.d, C.x3, gate);
+    count_launch(1);
+    return C.x3;
+}
+
 // Coarse part of the cycle below level l >= 1, whose right-hand side r and
 // first iterate x1 (pre-smoothed from zero by the restriction kernel) are in
 // place; returns the buffer that holds level l's result.  A level whose bit
@@ -1872,9 +2209,12 @@ static const float *coarse_cycle(const Mg &mg, int l, const SolveState *gate, cu
     for (int rep = 0; rep < reps; rep++) {
         MgLevel Fi = F;
         Fi.x1 = cur; // the iterate whose residual is restricted and which the post-smoother corrects
-        launch_restrict_pre<float>(Fi, F.r, C, l + 1, last ? C.x3 : C.x1, last ? 1.0f : mg.omega, gate, s);
         MgLevel Cr = C;
-        Cr.x3 = const_cast<float *>(coarse_cycle(mg, l + 1, gate, s));
+        if (l + 1 == mg.dense_level) Cr.x3 = const_cast<float *>(dense_visit<float>(mg, Fi, F.r, gate, s, false));
+        else {
+            launch_restrict_pre<float>(Fi, F.r, C, l + 1, last ? C.x3 : C.x1, last ? 1.0f : mg.omega, gate, s);
+            Cr.x3 = const_cast<float *>(coarse_cycle(mg, l + 1, gate, s));
+        }
         launch_post<float, float>(Fi, l, F.r, Cr, other, mg.omega, mg.cscale, gate, mg.use_tma, mg.err, s);
         std::swap(cur, other);
     }
@@ -1896,9 +2236,12 @@ void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStr
     const MgLevel &F = mg.lev[0];
     const MgLevel &C = mg.lev[1];
     const bool last = L == 2;
-    launch_restrict_pre<V>(F, in, C, 1, last ? C.x3 : C.x1, last ? 1.0f : w, gate, s, !mg.pre0);
     MgLevel Cr = C;
-    Cr.x3 = const_cast<float *>(coarse_cycle(mg, 1, gate, s));
+    if (mg.dense_level == 1) Cr.x3 = const_cast<float *>(dense_visit<V>(mg, F, in, gate, s, !mg.pre0));
+    else {
+        launch_restrict_pre<V>(F, in, C, 1, last ? C.x3 : C.x1, last ? 1.0f : w, gate, s, !mg.pre0);
+        Cr.x3 = const_cast<float *>(coarse_cycle(mg, 1, gate, s));
+    }
     launch_post<V, V>(F, 0, in, Cr, out, w, mg.cscale, gate, mg.use_tma, mg.err, s,
                       mg.pre0 ? nullptr : mg.coef0h, !mg.pre0);
 }

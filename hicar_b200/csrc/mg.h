@@ -31,6 +31,11 @@ struct Mg {
     int fuse_level = 0;  // first level of the coarse part run by one thread-block cluster (0: every level its own
                          // launches; HICARW_MG_FUSE=0 at build time)
     int cluster_n = 0;   // CTAs of that cluster
+    int dense_level = 0; // level (>= 1) from which the cycle is one matrix-vector product (0: none)
+    int dense_n = 0, dense_ld = 0;  // its unknowns and the matrix's row length
+    float *dense = nullptr, *dense_r = nullptr; // the matrix and the compact right-hand side of a visit
+    float dense_omega = 0.0f, dense_cscale = 0.0f; // the parameters that the matrix was tabulated with
+    int dense_wmask = 0;
     int bf16 = 0;        // the finest level's smoother coefficients in BF16 (V(0,1) cycles; factors of the rounded
                          // tridiagonal)
     __nv_bfloat16 *coef0h = nullptr; // those coefficients (15 * npad)
@@ -40,6 +45,7 @@ struct Mg {
 
 int mg_build(Mg &mg, const Dims &fine, const float *fine_coef, cudaStream_t s);
 void mg_free(Mg &mg);
+int mg_refresh(Mg &mg, cudaStream_t s); // after a change of omega, cscale or wmask: 1 when the dense matrix was made again
 long long mg_tma_posts(); // post-smoother launches enqueued through the tensor-copy kernel
 template <typename V>
 void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStream_t s);

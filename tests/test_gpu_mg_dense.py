@@ -1,0 +1,62 @@
+"""GPU tests of the dense coarse cycle: the V-cycle whose coarse levels are one
+tabulated matrix against the numpy restatement, at the sizes where the choice of
+the dense level changes, and after a change of the cycle's parameters."""
+import numpy as np
+import pytest
+
+from hicar_b200 import _capi, cases
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(autouse=True)
+def _fresh(lib, monkeypatch):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from hicar_b200 import wind, wind_iterative
+    monkeypatch.delenv("HICARW_MG_FUSE", raising=False)
+    wind_iterative.finalize_iter_winds()
+    wind.reset()
+    yield
+    wind_iterative.finalize_iter_winds()
+    wind.reset()
+
+
+def _apply(h, x):
+    y = np.empty_like(x)
+    _capi.check(_capi.load().hicarw_apply_precond(h, x.ctypes.data, y.ctypes.data, 0, _capi.MEM_HOST, None), h)
+    return y
+
+
+# dense level 1 with few, with an odd number of and with many unknowns; a lower level; rows of one aggregate
+@pytest.mark.parametrize("shape", [(6, 4, 3), (9, 7, 5), (32, 32, 8), (63, 65, 4), (33, 31, 9), (3, 40, 24), (70, 50, 33)])
+def test_dense_coarse_cycle_against_the_restatement(shape):
+    """Tolerance: the restatement runs the levels in FP32 as the per-level kernels
+    do; 1e-5 is the bar of those kernels' own tests."""
+    import mg_ref
+    from hicar_b200 import wind, wind_iterative as wi
+    from hicar_b200.domain import DeviceDomain
+    nx, ny, nz = shape
+    case = cases.build_case(nx, ny, nz, seed=31, adv_den=True, n_hills=6)
+    dom = DeviceDomain.from_case(case, "cuda")
+    wi.init_iter_winds(dom, wi.WindOptions())
+    wind.calibrate_projection_operator(dom, wi.WindOptions())
+    h = wi.handle(dom.nest_indx)
+    coefs = np.empty((15, ny, nz, nx), np.float32)
+    _capi.check(_capi.load().hicarw_get_coefs(h, coefs.ctypes.data, _capi.MEM_HOST, None), h)
+    rng = np.random.default_rng(41)
+    x = np.zeros((ny + 2, nz + 2, nx + 2))
+    x[1:-1, 1:-1, 1:-1] = rng.standard_normal((ny, nz, nx))
+    first = None
+    # the matrix belongs to the parameters of the call: change them and change them back
+    for omega, wlev, scale, skip in ((0.8, (), 1.35, False), (1.0, (2, 3, 4), 1.35, True), (1.0, (1, 2), 1.1, True),
+                                     (0.8, (), 1.35, False)):
+        wi.set_options(wi.WindOptions(mg_omega=omega, mg_w_levels=wlev, mg_coarse_scale=scale, mg_skip_fine_presmooth=skip))
+        y = _apply(h, x)
+        ref = mg_ref.VCycle(coefs, omega, scale, fine_presmooth=not skip, wlevels=wlev)(x[1:-1, 1:-1, 1:-1])
+        got = y[1:-1, 1:-1, 1:-1]
+        assert np.linalg.norm(got - ref) < 1e-5 * np.linalg.norm(ref), (omega, wlev)
+        assert not y[0].any() and not y[-1].any() and not y[:, 0].any() and not y[:, :, -1].any()
+        first = y if first is None else first
+    np.testing.assert_array_equal(y, first)
