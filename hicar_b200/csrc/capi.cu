@@ -2,10 +2,9 @@
 // calc_iter_winds (wind_iterative.F90:295-532), probing (:1096-1248,
 // wind.F90:1010-1099) and the device-driven BiCGStab loop.
 //
-// The loop: one CUDA graph holds `check_every` BiCGStab iterations (the kernel
-// schedule of k_krylov.cu).  The host
-// replays it and, one graph behind, reads the device-side `stop` flag through
-// pinned memory, so the GPU never waits for the host inside a solve.  Kernels
+// The loop: one CUDA graph whose WHILE node repeats a few BiCGStab iterations
+// (the kernel schedule of k_krylov.cu) until the device-side `stop` flag is set,
+// so neither the GPU nor the host waits for the other inside a solve.  Kernels
 // of an ended solve return immediately.
 #include <cuda_runtime.h>
 #include <stdio.h>
@@ -74,7 +73,7 @@ ProfScope::~ProfScope()
 static thread_local std::string g_err_noh;
 
 struct GraphKey {
-    int prec, sweeps, chunk, solver, replace, precond;
+    int prec, sweeps, chunk, solver, bodies, precond;
     bool operator<(const GraphKey &o) const
     {
         if (precond != o.precond) return precond < o.precond;
@@ -82,7 +81,7 @@ struct GraphKey {
         if (sweeps != o.sweeps) return sweeps < o.sweeps;
         if (chunk != o.chunk) return chunk < o.chunk;
         if (solver != o.solver) return solver < o.solver;
-        return replace < o.replace;
+        return bodies < o.bodies;
     }
 };
 struct GraphRec {
@@ -109,8 +108,8 @@ struct hicarw_handle {
     void *vec[NVEC] = {};
     SolveState *st = nullptr;
     SolveState *hst = nullptr; // pinned host mirror
-    int *hflag = nullptr;      // pinned stop flags (2 slots)
-    cudaEvent_t ev[2] = {nullptr, nullptr};
+    int *hflag = nullptr;      // pinned stop flag
+    int loop_nodes = 0, loop_first = 0; // kernels of a pass through the loop's body; passes counted at its launches
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     double *hist = nullptr;
     int hist_cap = 0;
@@ -367,8 +366,6 @@ extern "C" int hicarw_init_iter_winds(const hicarw_grid *g, const hicarw_options
         return HICARW_ERR_CUDA;
     }
     cudaStreamCreateWithFlags(&h->cap, cudaStreamNonBlocking);
-    cudaEventCreateWithFlags(&h->ev[0], cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&h->ev[1], cudaEventDisableTiming);
     cudaEventCreate(&h->t0);
     cudaEventCreate(&h->t1);
     cudaMemcpyKind kind = mem_kind == HICARW_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
@@ -417,8 +414,6 @@ extern "C" int hicarw_finalize_iter_winds(hicarw_handle *h)
     if (h->hst) cudaFreeHost(h->hst);
     if (h->hflag) cudaFreeHost(h->hflag);
     if (h->hscan) cudaFreeHost(h->hscan);
-    for (int q = 0; q < 2; q++)
-        if (h->ev[q]) cudaEventDestroy(h->ev[q]);
     if (h->dist_buf) cudaFree(h->dist_buf);
     if (h->t0) cudaEventDestroy(h->t0);
     if (h->t1) cudaEventDestroy(h->t1);
@@ -535,52 +530,90 @@ static void enqueue_true_residual_prec(hicarw_handle *h, int prec, int mode, cud
                                             mode ? V<float>(h, V_RHAT) : nullptr, h->st, mode, rb, s);
 }
 
-static int get_graph(hicarw_handle *h, int prec, int sweeps, int chunk, GraphRec **out)
+// Keeps a solve's device-side loop running: until the solve state stops, or for
+// `bodies` more passes through its body.
+__global__ void loop_cond_kernel(cudaGraphConditionalHandle hc, SolveState *st, int bodies)
 {
-    GraphKey key{prec, sweeps, chunk, h->opt.solver, h->opt.replace_every, h->use_mg};
+    const int n = st->bodies + 1;
+    st->passes++;
+    const int more = !st->stop && n < bodies;
+    st->bodies = more ? n : 0;
+    cudaGraphSetConditional(hc, more ? 1u : 0u);
+}
+
+// The Krylov loop as one graph: a WHILE node whose body holds `chunk` iterations,
+// repeated on the device until the solve stops or for `bodies` passes.
+static int get_graph(hicarw_handle *h, int prec, int sweeps, int chunk, int bodies, GraphRec **out)
+{
+    GraphKey key{prec, sweeps, chunk, h->opt.solver, bodies, h->use_mg};
     auto it = h->graphs.find(key);
     if (it != h->graphs.end()) { *out = &it->second; return 0; }
     cudaGraph_t graph;
-    g_capturing = 1;
+    CK(cudaGraphCreate(&graph, 0));
+    cudaGraphConditionalHandle hc;
+    cudaGraphNode_t node;
+    cudaGraphNodeParams p{};
+    cudaError_t e = cudaGraphConditionalHandleCreate(&hc, graph, 1, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess) {
+        p.type = cudaGraphNodeTypeConditional;
+        p.conditional.handle = hc;
+        p.conditional.type = cudaGraphCondTypeWhile;
+        p.conditional.size = 1;
+        e = cudaGraphAddNode(&node, graph, nullptr, 0, &p);
+    }
     g_capture_nodes = 0;
-    CK(cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal));
-    for (int q = 0; q < chunk; q++) enqueue_iteration_prec(h, prec, sweeps, h->cap);
-    cudaError_t e = cudaStreamEndCapture(h->cap, &graph);
-    g_capturing = 0;
-    if (e != cudaSuccess) { set_err(h, "cudaStreamEndCapture", e); return HICARW_ERR_CUDA; }
+    if (e == cudaSuccess) {
+        cudaGraph_t body = p.conditional.phGraph_out[0];
+        g_capturing = 1;
+        e = cudaStreamBeginCaptureToGraph(h->cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) {
+            for (int q = 0; q < chunk; q++) enqueue_iteration_prec(h, prec, sweeps, h->cap);
+            loop_cond_kernel<<<1, 1, 0, h->cap>>>(hc, h->st, bodies);
+            count_launch(1);
+            e = cudaStreamEndCapture(h->cap, &body);
+        }
+        g_capturing = 0;
+    }
     GraphRec rec;
     rec.nodes = g_capture_nodes;
-    e = cudaGraphInstantiate(&rec.exec, graph, 0);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&rec.exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (e != cudaSuccess) { set_err(h, "cudaGraphInstantiate", e); return HICARW_ERR_CUDA; }
+    if (e != cudaSuccess) { set_err(h, "Krylov loop graph", e); return HICARW_ERR_CUDA; }
     auto res = h->graphs.emplace(key, rec);
     *out = &res.first->second;
     return 0;
 }
 
+// Iterations per pass through the loop's body: a pass costs one more launch and
+// the loop's own turn, a stopped solve up to LOOP_BODY - 1 iterations of kernels
+// that return at once.  One, two, four: 1.82, 1.81, 1.87 ms a solve at 64x64x20,
+// 8.25, 8.24, 8.40 at 181x157x33 (13 and 16 iterations).
+constexpr int LOOP_BODY = 2;
+
 // Run the BiCGStab loop until the device says stop.  Returns the reference
 // status (0/1/2) in h->hst after the call.
 static int run_loop(hicarw_handle *h, int prec, int sweeps, cudaStream_t s)
 {
-    GraphRec *g = nullptr;
-    int chunk = h->opt.check_every;
-    int rc = get_graph(h, prec, sweeps, chunk, &g);
-    if (rc) return rc;
-    const int max_chunks = (h->opt.max_iters + chunk - 1) / chunk + 2;
     // FP32 Krylov vectors: the recurrence residual is replaced by the FP64 true
-    // residual of the FP64 solution every replace_every iterations (rounded to graphs)
-    const int rep = prec != HICARW_KRYLOV_F64 && h->opt.replace_every > 0 ? std::max(1, h->opt.replace_every / chunk) : 0;
-    h->hflag[0] = h->hflag[1] = 0;
-    for (int n = 0; n < max_chunks; n++) {
+    // residual of the FP64 solution every replace_every iterations, rounded to
+    // multiples of check_every
+    const int chunk = h->opt.check_every;
+    const int rep = prec != HICARW_KRYLOV_F64 && h->opt.replace_every > 0 ? std::max(1, h->opt.replace_every / chunk) * chunk : 0;
+    const int body = rep > 0 && rep % LOOP_BODY ? 1 : LOOP_BODY;
+    const int all = (h->opt.max_iters + body - 1) / body + 2, bodies = rep > 0 ? rep / body : all;
+    GraphRec *g = nullptr;
+    int rc = get_graph(h, prec, sweeps, body, bodies, &g);
+    if (rc) return rc;
+    for (int n = 0; n < all; n += bodies) {
         CK(cudaGraphLaunch(g->exec, s));
         g_launches += g->nodes;
-        if (rep && (n + 1) % rep == 0) enqueue_true_residual_prec(h, prec, 1, s);
-        CK(cudaMemcpyAsync(&h->hflag[n & 1], &h->st->stop, sizeof(int), cudaMemcpyDeviceToHost, s));
-        CK(cudaEventRecord(h->ev[n & 1], s));
-        if (n >= 1) {
-            CK(cudaEventSynchronize(h->ev[(n - 1) & 1]));
-            if (h->hflag[(n - 1) & 1]) break;
-        }
+        h->loop_nodes = g->nodes;
+        h->loop_first++;
+        if (!rep) break; // the loop itself ended the solve
+        CK(cudaMemcpyAsync(h->hflag, &h->st->stop, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (h->hflag[0]) break;
+        enqueue_true_residual_prec(h, prec, 1, s);
     }
     return 0;
 }
@@ -628,7 +661,6 @@ static int bicgstab_solve(hicarw_handle *h, int sweeps, cudaStream_t s, int allo
     select_precond(h, allow_mg);
     if (h->use_mg && (rc = mg_ensure(h, s)) < 0) return rc;
     if (h->opt.solver == HICARW_SOLVER_FGMRES) return fgmres_solve(h, sweeps, s);
-    const int solver = h->opt.solver;
     const int prec = prec_in >= 0 ? prec_in : solve_precision(h);
     rc = ensure_vectors(h, prec);
     if (rc) return rc;
@@ -637,7 +669,7 @@ static int bicgstab_solve(hicarw_handle *h, int sweeps, cudaStream_t s, int allo
     launch_state_reset(h->st, h->opt.tol_rel, h->opt.tol_abs, h->opt.max_iters,
                        h->use_mg ? h->opt.stall_iters : 0, s);
     CK(cudaEventRecord(h->t0, s));
-    (void)solver;
+    h->loop_first = 0;
     enqueue_setup_prec(h, prec, c, rb, s, 0);
     rc = run_loop(h, prec, sweeps, s);
     if (rc) return rc;
@@ -659,7 +691,9 @@ static int bicgstab_solve(hicarw_handle *h, int sweeps, cudaStream_t s, int allo
     CK(cudaEventRecord(h->t1, s));
     // final FP64 true residual of the solution (diagnostic; reference has none)
     enqueue_true_residual_prec(h, prec, 0, s);
-    return fetch_state(h, s);
+    if ((rc = fetch_state(h, s)) != 0) return rc;
+    g_launches += (long long)h->loop_nodes * (h->hst->passes - h->loop_first); // the passes after each launch's first
+    return 0;
 }
 
 // ---- flexible GMRES ------------------------------------------------------------

@@ -84,6 +84,8 @@ struct SolveState {
     int dist;       // decomposed solve: reductions publish their local totals in dist_tot and the
                     // host applies the scalar steps to the totals summed over all ranks
     double dist_tot[5];
+    int bodies;      // passes through the present loop graph's body so far
+    int passes;      // ... of all its launches in this solve
     double mr_theta; // composite learned preconditioner: the minimal-residual step along the U-Net's correction
 };
 

@@ -677,6 +677,7 @@ __global__ void state_reset_kernel(SolveState *s, double tol_rel, double tol_abs
     s->err = 0;
     s->profile = 0;
     s->dist = 0;
+    s->bodies = s->passes = 0;
 }
 
 void launch_state_reset(SolveState *stt, double tol_rel, double tol_abs, int max_iters, int stall_k, cudaStream_t st)
