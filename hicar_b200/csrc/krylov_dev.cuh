@@ -265,7 +265,7 @@ __device__ __forceinline__ void march_rows(const OpCtx &c, const V *__restrict__
 
 namespace hw {
 
-// ---- float4 column-marching rows of y = A x (probed operator, nx % 4 == 0) ----
+// ---- float4 column-marching rows of y = A x (probed operator) ----
 // A lane owns four consecutive interior columns i0 .. i0+3 (i0 = 1 + 4g: a
 // 16-byte aligned group in the padded layout), a warp a strip of 128 columns
 // of one j row, and it marches k upwards over a chunk of at most M4_KC levels
@@ -304,20 +304,18 @@ __device__ __forceinline__ void st4v(double *__restrict__ p, const double (&v)[4
     *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
 }
 
-__host__ __device__ __forceinline__ bool march4_ok(const Dims &d) { return d.nx % 4 == 0 && d.nx >= 4; }
 __host__ __device__ __forceinline__ int march4_kc(const OpCtx &c) { return c.kc > 0 ? c.kc : M4_KC; }
-__host__ __device__ __forceinline__ long long march4_items(const OpCtx &c)
+__host__ __device__ __forceinline__ long long march4_items(const Dims &d, int KC)
 {
-    const Dims &d = c.d;
-    const int KC = march4_kc(c), G = d.nx / 4, nsx = (G + 31) / 32, nkc = (d.mz + KC - 1) / KC;
+    const int G = (d.nx + 3) / 4, nsx = (G + 31) / 32, nkc = (d.mz + KC - 1) / KC;
     return (long long)d.my * nsx * nkc;
 }
 
-template <typename V, typename F4, typename F1>
+template <typename V, bool RAG, typename F4, typename F1>
 __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict__ x, F4 &&f4, F1 &&f1)
 {
     const Dims &d = c.d;
-    const int KC = march4_kc(c), G = d.nx / 4, nsx = (G + 31) / 32, nkc = (d.mz + KC - 1) / KC;
+    const int KC = march4_kc(c), G = (d.nx + 3) / 4, nsx = (G + 31) / 32, nkc = (d.mz + KC - 1) / KC;
     const long long items = (long long)d.my * nsx * nkc;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     const long long P = d.P, PL = d.plane, N = d.npad;
@@ -331,6 +329,15 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
         const long long ob = (long long)j * PL + 1 + XO + 4LL * g; // group start at k = 0
         const long long oc = (long long)j * PL + XO;                // column i = 0 at k = 0
         const bool first = live && g == 0, lastg = live && g == G - 1;
+        const int nv = RAG && lastg ? d.nx - 4 * (G - 1) : 4; // interior columns of the group
+        auto put = [&](long long o, const double (&y)[4]) {
+            if (!RAG || nv == 4) f4(o, y);
+            else {
+#pragma unroll
+                for (int e = 0; e < 3; e++)
+                    if (e < nv) f1(o + e, y[e]);
+            }
+        };
         // lateral columns i = 0 and i = mx - 1: identity rows
         if (first)
             for (int k = k0; k <= k1; k++) f1(oc + k * P, (double)x[oc + k * P]);
@@ -342,11 +349,11 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
                     V xv[4];
                     ld4v(x + ob + k * P, xv);
                     const double y[4] = {(double)xv[0], (double)xv[1], (double)xv[2], (double)xv[3]};
-                    f4(ob + k * P, y);
+                    put(ob + k * P, y);
                 }
             continue;
         }
-        const bool west = live && lane == 0, east = live && (lane == 31 || g == G - 1);
+        const bool west = live && lane == 0, east = live && (lane == 31 || lastg) && nv == 4;
         // windows at k-1 (m), k (0) of the own row (c), the rows j-1 (s) and j+1 (n); the outer columns
         V c_m[4] = {}, c_0[4] = {}, s_m[4] = {}, s_0[4] = {}, n_m[4] = {}, n_0[4] = {};
         V w_m = 0, w_0 = 0, e_m = 0, e_0 = 0;
@@ -422,7 +429,7 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
                         y[e] = v;
                     }
                 }
-                f4(o, y);
+                put(o, y);
             }
 #pragma unroll
             for (int e = 0; e < 4; e++) {
