@@ -41,15 +41,14 @@ __device__ __forceinline__ bool inside(const Dims &d, int i, int k, int j)
 }
 
 // Programmatic dependent launch (the small levels' kernels, launched with the
-// programmatic-serialization attribute): wait until every earlier kernel of the
-// stream has completed and its writes are visible (a no-op for an ordinary
-// launch), then let the next kernel be launched while this one runs; the next
-// kernel reads nothing before its own wait.
-__device__ __forceinline__ void pdl_prologue()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// programmatic-serialization attribute).  pdl_trigger lets the next kernel be
+// launched while this one runs; pdl_wait waits until every earlier kernel of the
+// stream has completed and its writes are visible (both no-ops for an ordinary
+// launch).  Between the two a kernel loads what no kernel of the cycle writes:
+// its coefficients and factors.  Every path through such a kernel passes
+// pdl_wait, so that a kernel's completion implies that of all before it.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 
 // offsets (dk, dj, di) of the 15 coefficients A..O
@@ -129,51 +128,64 @@ __global__ void factor_kernel(Dims d, const float *__restrict__ coef, float *__r
 
 // Thomas recurrences of one column held in shared memory ([k][c] layout, stride tc):
 // res <- T^-1 res, with T = tridiag(C, 1/m-form factors) and couplings to the ghost planes dropped.
-// The operands of THOMAS_U levels are read ahead into registers, so that only
-// the multiply-add chain is serial (the same operations in the same order as
-// a level-by-level loop).
+// The operands of THOMAS_U levels are read into registers while the levels
+// before them are computed, so that only the multiply-add chain is serial (the
+// same operations in the same order as a level-by-level loop).
 constexpr int THOMAS_U = 8;
 
 __device__ __forceinline__ void thomas_column(float *s_res, const float *s_c, const float *s_m, const float *s_cp,
                                               int c, int tc, int nz)
 {
     float dprev = 0.0f;
-    int k = 0;
-    for (; k + THOMAS_U <= nz; k += THOMAS_U) {
-        float rv[THOMAS_U], cv[THOMAS_U], mv[THOMAS_U];
+    const int full = nz / THOMAS_U * THOMAS_U;
+    float rv[THOMAS_U], cv[THOMAS_U], mv[THOMAS_U], rn[THOMAS_U], cn[THOMAS_U], mn[THOMAS_U];
+    auto down = [&](int k, float (&r)[THOMAS_U], float (&cc)[THOMAS_U], float (&m)[THOMAS_U]) {
+        if (k >= full) return;
 #pragma unroll
         for (int u = 0; u < THOMAS_U; u++) {
-            int t = (k + u) * tc + c;
-            rv[u] = s_res[t]; cv[u] = s_c[t]; mv[u] = s_m[t];
+            const int t = (k + u) * tc + c;
+            r[u] = s_res[t]; cc[u] = s_c[t]; m[u] = s_m[t];
         }
+    };
+    down(0, rv, cv, mv);
+    for (int k = 0; k < full; k += THOMAS_U) {
+        down(k + THOMAS_U, rn, cn, mn);
 #pragma unroll
         for (int u = 0; u < THOMAS_U; u++) {
             dprev = (rv[u] - cv[u] * dprev) * mv[u];
             s_res[(k + u) * tc + c] = dprev;
         }
+#pragma unroll
+        for (int u = 0; u < THOMAS_U; u++) { rv[u] = rn[u]; cv[u] = cn[u]; mv[u] = mn[u]; }
     }
-    for (; k < nz; k++) {
-        int t = k * tc + c;
+    for (int k = full; k < nz; k++) {
+        const int t = k * tc + c;
         dprev = (s_res[t] - s_c[t] * dprev) * s_m[t];
         s_res[t] = dprev;
     }
     float y = 0.0f;
-    k = nz - 1;
-    for (; k + 1 >= THOMAS_U; k -= THOMAS_U) {
-        float rv[THOMAS_U], pv[THOMAS_U];
+    const int rest = nz - full;
+    auto up = [&](int k, float (&r)[THOMAS_U], float (&p)[THOMAS_U]) {
+        if (k < rest) return;
 #pragma unroll
         for (int u = 0; u < THOMAS_U; u++) {
-            int t = (k - u) * tc + c;
-            rv[u] = s_res[t]; pv[u] = s_cp[t];
+            const int t = (k - u) * tc + c;
+            r[u] = s_res[t]; p[u] = s_cp[t];
         }
+    };
+    up(nz - 1, rv, cv);
+    for (int k = nz - 1; k >= rest; k -= THOMAS_U) {
+        up(k - THOMAS_U, rn, cn);
 #pragma unroll
         for (int u = 0; u < THOMAS_U; u++) {
-            y = rv[u] - pv[u] * y;
+            y = rv[u] - cv[u] * y;
             s_res[(k - u) * tc + c] = y;
         }
+#pragma unroll
+        for (int u = 0; u < THOMAS_U; u++) { rv[u] = rn[u]; cv[u] = cn[u]; }
     }
-    for (; k >= 0; k--) {
-        int t = k * tc + c;
+    for (int k = rest - 1; k >= 0; k--) {
+        const int t = k * tc + c;
         y = s_res[t] - s_cp[t] * y;
         s_res[t] = y;
     }
@@ -262,7 +274,6 @@ __global__ void __launch_bounds__(MG_THREADS) pre_kernel(Dims d, const float *__
                                                          const TR *__restrict__ r, float *__restrict__ out,
                                                          float omega, const SolveState *gate)
 {
-    pdl_prologue();
     if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
     constexpr int TC = TX * TY;
     extern __shared__ float sm[];
@@ -337,6 +348,36 @@ __device__ __forceinline__ void stage_window(const Dims &d, const float *__restr
     }
 }
 
+// The same with loads through L2 (a kernel that may start before its
+// predecessor's end does not read the predecessor's results through the
+// read-only path).
+template <int SX, int SY>
+__device__ __forceinline__ void stage_window_l2(const Dims &d, const float *x1, const Dims &dc, const float *xc, int ia,
+                                                int ja, float *s_x, float cs = 1.0f)
+{
+    constexpr int SP = SX * SY;
+    const int nst = SP * (d.nz + 2);
+    for (int base = threadIdx.x; base < nst; base += MG_THREADS * MG_BATCH) {
+        float a[MG_BATCH], b[MG_BATCH];
+#pragma unroll
+        for (int u = 0; u < MG_BATCH; u++) {
+            const int t = base + u * MG_THREADS;
+            const int lx = t % SX, ly = (t / SX) % SY, k = t / SP;
+            const int i = ia + lx, j = ja + ly;
+            a[u] = b[u] = 0.0f;
+            if (t < nst && inside(d, i, k, j)) {
+                a[u] = __ldcg(x1 + kidx(d, i, k, j));
+                if (xc) b[u] = __ldcg(xc + kidx(dc, (i + 1) >> 1, k, (j + 1) >> 1));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < MG_BATCH; u++) {
+            const int t = base + u * MG_THREADS;
+            if (t < nst) s_x[t] = xc ? a[u] + cs * b[u] : a[u];
+        }
+    }
+}
+
 // Post-smoothing: out = x2 + w T^-1 (r - A x2) with x2 = x1 + P xc, x2 of the
 // tile and its one-column ring staged in shared memory first.
 constexpr int POST_CELLS = 4; // (column, level) residuals per thread in flight; 3 CTAs per SM by registers
@@ -349,7 +390,6 @@ __global__ void __launch_bounds__(MG_THREADS, 3) post_kernel(Dims d, const CT *_
                                                           const float *__restrict__ xc, TO *__restrict__ out,
                                                           float omega, float cscale, const SolveState *gate)
 {
-    pdl_prologue();
     if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
     constexpr int TC = TX * TY, SX = TX + 2, SY = TY + 2, SP = SX * SY;
     extern __shared__ float sm[];
@@ -914,7 +954,6 @@ __global__ void __launch_bounds__(MG_THREADS, 3) restrict_pre_kernel(
     const float *__restrict__ coef_c, const float *__restrict__ cp_c, const float *__restrict__ minv_c,
     float *__restrict__ r_c, float *__restrict__ out_c, float omega, const SolveState *gate)
 {
-    pdl_prologue();
     if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
     constexpr int TC = TX * TY, FX = 2 * TX + 2, FY = 2 * TY + 2, FP = FX * FY;
     extern __shared__ float sm[];
@@ -974,6 +1013,180 @@ __global__ void __launch_bounds__(MG_THREADS, 3) restrict_pre_kernel(
         int I = I0 + c % TX, J = J0 + c / TX;
         if (I > dc.nx || J > dc.ny) continue;
         out_c[kidx(dc, I, k, J)] = omega * s_res[t];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The small levels' restriction and post-smoothing (column tiles of 4 or 8).
+// Their time is a chain of latencies: launch, operands, column recurrences,
+// store.  They load the operands that the cycle does not write (coefficients,
+// Thomas factors) before they wait for the kernel before them, so that these
+// loads and the launch overlap its run, and take the right-hand side and the
+// window in one further round trip.  The arithmetic of a cell is that of
+// restrict_pre_kernel and post_kernel.  A solve to 1e-9 against the kernels that
+// waited first (B200): 64x64x20 1.81 -> 1.62 ms, 181x157x33 8.24 -> 7.29 ms,
+// 512x512x48 39.7 -> 37.0 ms; without the programmatic launch 1.67, 7.63, 38.7.
+// ---------------------------------------------------------------------------
+constexpr int SM_POST_U = 2;     // cells per thread loaded ahead (8 columns x 64 levels: all)
+constexpr int SM_RESTRICT_U = 3; // fine cells per thread loaded ahead (4 coarse columns x 48 levels: all)
+
+template <typename TR, typename TO, int TX, int TY, typename CT>
+__global__ void __launch_bounds__(MG_THREADS) post_small_kernel(Dims d, const CT *__restrict__ coef,
+                                                                const float *__restrict__ cp,
+                                                                const float *__restrict__ minv, const TR *r,
+                                                                const float *x1, Dims dc, const float *xc, TO *out,
+                                                                float omega, float cscale, const SolveState *gate)
+{
+    pdl_trigger();
+    constexpr int TC = TX * TY, SX = TX + 2, SY = TY + 2, SP = SX * SY;
+    extern __shared__ float sm[];
+    const int nz = d.nz, n = TC * nz;
+    float *s_res = sm, *s_c = sm + n, *s_m = sm + 2 * n, *s_cp = sm + 3 * n, *s_x = sm + 4 * n;
+    const int i0 = blockIdx.x * TX + 1, j0 = blockIdx.y * TY + 1;
+    auto offset = [&](int t, long long &o) { // the cell of item t; false outside the level
+        const int c = t % TC, i = i0 + c % TX, j = j0 + c / TX;
+        o = kidx(d, i, t / TC + 1, j);
+        return t < n && i <= d.nx && j <= d.ny;
+    };
+    float cv[SM_POST_U][15], vm[SM_POST_U], vp[SM_POST_U];
+    auto load = [&](int u, int t) {
+        long long o;
+        vm[u] = vp[u] = 0.0f;
+        if (offset(t, o)) {
+            load_coefs(coef, d.npad, o, cv[u]);
+            vm[u] = __ldg(minv + o);
+            vp[u] = __ldg(cp + o);
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < SM_POST_U; u++) load(u, threadIdx.x + u * MG_THREADS);
+    pdl_wait();
+    if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
+    TR rv[SM_POST_U];
+    auto load_r = [&](int u, int t) {
+        long long o;
+        rv[u] = offset(t, o) ? r[o] : (TR)0;
+    };
+#pragma unroll
+    for (int u = 0; u < SM_POST_U; u++) load_r(u, threadIdx.x + u * MG_THREADS);
+    stage_window_l2<SX, SY>(d, x1, dc, xc, i0 - 1, j0 - 1, s_x, cscale);
+    __syncthreads();
+    for (int base = threadIdx.x; base < n; base += MG_THREADS * SM_POST_U) {
+#pragma unroll
+        for (int u = 0; u < SM_POST_U; u++) {
+            const int t = base + u * MG_THREADS;
+            if (base >= MG_THREADS) {
+                load(u, t);
+                load_r(u, t);
+            }
+            long long o;
+            float res = 0.0f, vc = 0.0f;
+            const int c = t % TC, k = t / TC + 1;
+            if (offset(t, o)) {
+                res = post_residual<SX, SP>((double)rv[u], cv[u], s_x + k * SP + (c / TX + 1) * SX + (c % TX + 1));
+                vc = k > 1 ? cv[u][CC] : 0.0f;
+            }
+            if (t < n) { s_res[t] = res; s_c[t] = vc; s_m[t] = vm[u]; s_cp[t] = vp[u]; }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < TC) {
+        const int c = threadIdx.x;
+        if (i0 + c % TX <= d.nx && j0 + c / TX <= d.ny) thomas_column(s_res, s_c, s_m, s_cp, c, TC, nz);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < n; t += MG_THREADS) {
+        long long o;
+        const int c = t % TC, k = t / TC + 1;
+        if (offset(t, o))
+            out[o] = (TO)((double)s_x[k * SP + (c / TX + 1) * SX + (c % TX + 1)] + (double)omega * (double)s_res[t]);
+    }
+}
+
+// Four lanes per coarse cell, one per child; their residuals are summed in the
+// order of restrict_pre_kernel.
+template <typename TR, int TX, int TY, bool NOX>
+__global__ void __launch_bounds__(MG_THREADS) restrict_small_kernel(
+    Dims f, const float *__restrict__ coef_f, const TR *r_f, const float *x1_f, Dims dc,
+    const float *__restrict__ coef_c, const float *__restrict__ cp_c, const float *__restrict__ minv_c, float *r_c,
+    float *out_c, float omega, const SolveState *gate)
+{
+    pdl_trigger();
+    constexpr int TC = TX * TY, FX = 2 * TX + 2, FY = 2 * TY + 2, FP = FX * FY, U = SM_RESTRICT_U;
+    extern __shared__ float sm[];
+    const int nz = f.nz, n = TC * nz, items = 4 * n;
+    float *s_res = sm, *s_c = sm + n, *s_m = sm + 2 * n, *s_cp = sm + 3 * n, *s_x = sm + 4 * n;
+    const int I0 = blockIdx.x * TX + 1, J0 = blockIdx.y * TY + 1;
+    // item t: child t & 3 of the tile's coarse cell t >> 2; the fine cell's offset, false outside the level
+    auto fine = [&](int t, long long &o) {
+        const int cell = t >> 2, c = cell % TC, i = 2 * (I0 + c % TX) - 1 + (t & 1), j = 2 * (J0 + c / TX) - 1 + ((t >> 1) & 1);
+        o = kidx(f, i, cell / TC + 1, j);
+        return t < items && i <= f.nx && j <= f.ny;
+    };
+    float cv[U][15];
+    if (!NOX) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            long long o;
+            if (fine(threadIdx.x + u * MG_THREADS, o)) load_coefs(coef_f, f.npad, o, cv[u]);
+        }
+    }
+    for (int t = threadIdx.x; t < n; t += MG_THREADS) {
+        const int c = t % TC, k = t / TC + 1, I = I0 + c % TX, J = J0 + c / TX;
+        if (I > dc.nx || J > dc.ny) continue;
+        const long long oc = kidx(dc, I, k, J);
+        s_c[t] = k > 1 ? __ldg(coef_c + (long long)CC * dc.npad + oc) : 0.0f;
+        s_m[t] = __ldg(minv_c + oc);
+        s_cp[t] = __ldg(cp_c + oc);
+    }
+    pdl_wait();
+    if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
+    TR rv[U];
+    auto load_r = [&](int u, int t) {
+        long long o;
+        rv[u] = fine(t, o) ? r_f[o] : (TR)0;
+    };
+#pragma unroll
+    for (int u = 0; u < U; u++) load_r(u, threadIdx.x + u * MG_THREADS);
+    if (!NOX) {
+        stage_window_l2<FX, FY>(f, x1_f, f, nullptr, 2 * I0 - 2, 2 * J0 - 2, s_x);
+        __syncthreads();
+    }
+    // every lane of a warp takes the same number of turns (the shuffles below)
+    for (int base = 0; base < items; base += MG_THREADS * U) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int t = base + u * MG_THREADS + threadIdx.x;
+            long long o;
+            const bool in = fine(t, o);
+            if (base > 0) {
+                if (!NOX && in) load_coefs(coef_f, f.npad, o, cv[u]);
+                load_r(u, t);
+            }
+            double v = (double)rv[u];
+            const int cell = t >> 2, c = cell % TC, k = cell / TC + 1;
+            if (!NOX && in)
+                v = restrict_residual<FX, FP>(v, cv[u], s_x + k * FP + (2 * (c / TX) + ((t >> 1) & 1) + 1) * FX +
+                                                            (2 * (c % TX) + (t & 1) + 1));
+            const double v1 = __shfl_down_sync(0xffffffffu, v, 1), v2 = __shfl_down_sync(0xffffffffu, v, 2),
+                         v3 = __shfl_down_sync(0xffffffffu, v, 3);
+            const int I = I0 + c % TX, J = J0 + c / TX;
+            if ((t & 3) == 0 && t < items && I <= dc.nx && J <= dc.ny) {
+                const float rc = (float)(((v + v1) + v2) + v3); // a missing child adds zero
+                r_c[kidx(dc, I, k, J)] = rc;
+                s_res[cell] = rc;
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < TC) {
+        const int c = threadIdx.x;
+        if (I0 + c % TX <= dc.nx && J0 + c / TX <= dc.ny) thomas_column(s_res, s_c, s_m, s_cp, c, TC, nz);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < n; t += MG_THREADS) {
+        const int c = t % TC, k = t / TC + 1, I = I0 + c % TX, J = J0 + c / TX;
+        if (I <= dc.nx && J <= dc.ny) out_c[kidx(dc, I, k, J)] = omega * s_res[t];
     }
 }
 
@@ -1263,33 +1476,32 @@ __device__ __forceinline__ int dense_index(const Dims &d, int i, int k, int j)
 // that all of a thread's loads are in flight together.
 template <typename TR, bool NOX>
 __global__ void __launch_bounds__(DN_THREADS) dense_restrict_kernel(Dims f, const float *__restrict__ coef_f,
-                                                                    const TR *__restrict__ r_f,
-                                                                    const float *__restrict__ x1_f, Dims dc, int n,
-                                                                    float *__restrict__ rd, const SolveState *gate)
+                                                                    const TR *r_f, const float *x1_f, Dims dc, int n,
+                                                                    float *rd, const SolveState *gate)
 {
-    if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
+    pdl_trigger();
     const int t = blockIdx.x * DN_THREADS + threadIdx.x, cell = t >> 2, child = t & 3;
+    const int I = cell % dc.nx + 1, row = cell / dc.nx, k = row % dc.nz + 1, J = row / dc.nz + 1;
+    const int i = 2 * I - 1 + (child & 1), j = 2 * J - 1 + (child >> 1);
+    const bool in = cell < n && i <= f.nx && j <= f.ny;
+    const long long o = kidx(f, i, k, j);
+    float cv[15], xv[15];
+    if (in && !NOX) load_coefs(coef_f, f.npad, o, cv);
+    pdl_wait();
+    if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
     double acc = 0.0;
-    if (cell < n) {
-        const int I = cell % dc.nx + 1, row = cell / dc.nx, k = row % dc.nz + 1, J = row / dc.nz + 1;
-        const int i = 2 * I - 1 + (child & 1), j = 2 * J - 1 + (child >> 1);
-        if (i <= f.nx && j <= f.ny) {
-            const long long o = kidx(f, i, k, j);
-            if (NOX) {
-                acc = (double)r_f[o];
-            } else {
-                float cv[15], xv[15];
-                load_coefs(coef_f, f.npad, o, cv);
+    if (in) {
+        acc = (double)r_f[o];
+        if (!NOX) {
 #pragma unroll
-                for (int q = 0; q < 15; q++)
-                    xv[q] = inside(f, i + off_i(q), k + off_k(q), j + off_j(q))
-                                ? x1_f[o + off_i(q) + off_k(q) * (long long)f.P + off_j(q) * f.plane]
-                                : 0.0f;
-                float y = 0.0f;
+            for (int q = 0; q < 15; q++)
+                xv[q] = inside(f, i + off_i(q), k + off_k(q), j + off_j(q))
+                            ? x1_f[o + off_i(q) + off_k(q) * (long long)f.P + off_j(q) * f.plane]
+                            : 0.0f;
+            float y = 0.0f;
 #pragma unroll
-                for (int q = 0; q < 15; q++) y = fmaf(cv[q], xv[q], y);
-                acc = (double)r_f[o] - (double)y;
-            }
+            for (int q = 0; q < 15; q++) y = fmaf(cv[q], xv[q], y);
+            acc -= (double)y;
         }
     }
     acc += __shfl_xor_sync(0xffffffffu, acc, 1);
@@ -1300,21 +1512,27 @@ __global__ void __launch_bounds__(DN_THREADS) dense_restrict_kernel(Dims f, cons
 // x = S rd, one warp per row (ld: row length in floats, a multiple of 128; the
 // padding of S and rd is zero), x in the level's padded layout.
 __global__ void __launch_bounds__(DN_THREADS) dense_apply_kernel(const float *__restrict__ S, int n, int ld,
-                                                                 const float *__restrict__ rd, Dims d,
-                                                                 float *__restrict__ x, const SolveState *gate)
+                                                                 const float *rd, Dims d, float *x,
+                                                                 const SolveState *gate)
 {
+    pdl_trigger();
+    constexpr int U = 8; // 1024 columns in flight, the first ones before the wait
+    const int row = blockIdx.x * (DN_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31, nq = ld / 4;
+    const float4 *sr = reinterpret_cast<const float4 *>(S + (size_t)min(row, n - 1) * ld), *rr = reinterpret_cast<const float4 *>(rd);
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 a[U], acc = zero;
+#pragma unroll
+    for (int u = 0; u < U; u++) a[u] = lane + 32 * u < nq ? __ldg(sr + lane + 32 * u) : zero;
+    pdl_wait();
     if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
-    const int row = blockIdx.x * (DN_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const float4 *sr = reinterpret_cast<const float4 *>(S + (size_t)row * ld), *rr = reinterpret_cast<const float4 *>(rd);
-    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    constexpr int U = 8; // 1024 columns in flight
-    for (int b = lane; b < ld / 4; b += 32 * U) {
-        float4 a[U], v[U];
+    for (int b = lane; b < nq; b += 32 * U) {
+        float4 v[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) a[u] = b + 32 * u < ld / 4 ? __ldg(sr + b + 32 * u) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int u = 0; u < U; u++) v[u] = b + 32 * u < nq ? rr[b + 32 * u] : zero;
+        if (b >= 32 * U) {
 #pragma unroll
-        for (int u = 0; u < U; u++) v[u] = b + 32 * u < ld / 4 ? rr[b + 32 * u] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int u = 0; u < U; u++) a[u] = b + 32 * u < nq ? __ldg(sr + b + 32 * u) : zero;
+        }
 #pragma unroll
         for (int u = 0; u < U; u++) {
             acc.x = fmaf(a[u].x, v[u].x, acc.x);
@@ -1325,7 +1543,7 @@ __global__ void __launch_bounds__(DN_THREADS) dense_apply_kernel(const float *__
     }
     float y = (acc.x + acc.y) + (acc.z + acc.w);
     for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-    if (lane == 0) x[kidx(d, row % d.nx + 1, row / d.nx % d.nz + 1, row / (d.nx * d.nz) + 1)] = y;
+    if (lane == 0 && row < n) x[kidx(d, row % d.nx + 1, row / d.nx % d.nz + 1, row / (d.nx * d.nz) + 1)] = y;
 }
 
 // ---- tabulating the matrix: the cycle's steps on n right-hand sides at once,
@@ -1613,38 +1831,32 @@ static void set_smem(F *kernel, size_t smem)
     raise_smem((const void *)kernel, smem);
 }
 
-// HICARW_MG_PDL=1 in the environment launches the small levels' kernels (2 x 2
-// column tiles) with programmatic stream serialization: each may be launched
-// while the kernel before it runs and waits in its prologue (pdl_prologue) for
-// that kernel's results.  Off by default: inside the solve's CUDA graph it
-// measured no faster (1024x1024x64: 8.28 against 8.33 solves/s).  Read once.
+// Launch of a kernel that opens with pdl_trigger / pdl_wait: with programmatic
+// stream serialization (HICARW_MG_PDL=0 in the environment: an ordinary launch).
+// Read once.
 static bool mg_pdl()
 {
     static const bool on = [] {
         const char *e = getenv("HICARW_MG_PDL");
-        return e && e[0] == '1';
+        return !(e && e[0] == '0');
     }();
     return on;
 }
 
-template <typename K, typename... A>
-static void launch_mg(bool small, K *kernel, dim3 g, size_t smem, cudaStream_t s, A... args)
+template <typename... P, typename... A>
+static void launch_pdl(void (*kernel)(P...), dim3 g, int threads, size_t smem, cudaStream_t s, A... args)
 {
-    if (!(small && mg_pdl())) {
-        kernel<<<g, MG_THREADS, smem, s>>>(args...);
-        return;
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = g;
-    cfg.blockDim = dim3(MG_THREADS);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
+    cfg.numAttrs = mg_pdl() ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 template <typename TR, int TX, int TY>
@@ -1653,8 +1865,7 @@ static void pre_t(const MgLevel &L, const TR *r, float *out, float omega, const 
     dim3 g((L.d.nx + TX - 1) / TX, (L.d.ny + TY - 1) / TY);
     size_t smem = (size_t)4 * TX * TY * L.d.nz * sizeof(float);
     set_smem(pre_kernel<TR, TX, TY>, smem);
-    launch_mg(TX == 2 && TY == 2, pre_kernel<TR, TX, TY>, g, smem, s, L.d, (const float *)L.coef,
-              (const float *)L.cp, (const float *)L.minv, r, out, omega, gate);
+    pre_kernel<TR, TX, TY><<<g, MG_THREADS, smem, s>>>(L.d, L.coef, L.cp, L.minv, r, out, omega, gate);
 }
 
 template <typename TR>
@@ -1674,9 +1885,15 @@ static void post_t(const MgLevel &L, const CT *coef, const TR *r, const MgLevel 
 {
     dim3 g((L.d.nx + TX - 1) / TX, (L.d.ny + TY - 1) / TY);
     size_t smem = ((size_t)4 * TX * TY * L.d.nz + (size_t)(TX + 2) * (TY + 2) * (L.d.nz + 2)) * sizeof(float);
-    set_smem(post_kernel<TR, TO, TX, TY, CT>, smem);
-    launch_mg(TX * TY <= 8, post_kernel<TR, TO, TX, TY, CT>, g, smem, s, L.d, coef, (const float *)L.cp,
-              (const float *)L.minv, r, (const float *)L.x1, C.d, (const float *)C.x3, out, omega, cscale, gate);
+    if constexpr (TX * TY <= 8) {
+        set_smem(post_small_kernel<TR, TO, TX, TY, CT>, smem);
+        launch_pdl(post_small_kernel<TR, TO, TX, TY, CT>, g, MG_THREADS, smem, s, L.d, coef, L.cp, L.minv, r, L.x1, C.d,
+                   C.x3, out, omega, cscale, gate);
+    } else {
+        set_smem(post_kernel<TR, TO, TX, TY, CT>, smem);
+        post_kernel<TR, TO, TX, TY, CT><<<g, MG_THREADS, smem, s>>>(L.d, coef, L.cp, L.minv, r, L.x1, C.d, C.x3, out,
+                                                                    omega, cscale, gate);
+    }
 }
 
 static std::atomic<long long> g_tma_posts{0};
@@ -1861,10 +2078,15 @@ static void restrict_t(const MgLevel &F, const TR *r, const MgLevel &C, float *o
     dim3 g((C.d.nx + TX - 1) / TX, (C.d.ny + TY - 1) / TY);
     size_t smem = ((size_t)4 * TX * TY * C.d.nz + (NOX ? 0 : (size_t)(2 * TX + 2) * (2 * TY + 2) * (C.d.nz + 2))) *
                   sizeof(float);
-    set_smem(restrict_pre_kernel<TR, TX, TY, NOX>, smem);
-    launch_mg(TX * TY <= 8, restrict_pre_kernel<TR, TX, TY, NOX>, g, smem, s, F.d, (const float *)F.coef, r,
-              (const float *)F.x1, C.d, (const float *)C.coef, (const float *)C.cp, (const float *)C.minv, C.r, out,
-              omega, gate);
+    if constexpr (TX * TY <= 8) {
+        set_smem(restrict_small_kernel<TR, TX, TY, NOX>, smem);
+        launch_pdl(restrict_small_kernel<TR, TX, TY, NOX>, g, MG_THREADS, smem, s, F.d, F.coef, r, F.x1, C.d, C.coef, C.cp,
+                   C.minv, C.r, out, omega, gate);
+    } else {
+        set_smem(restrict_pre_kernel<TR, TX, TY, NOX>, smem);
+        restrict_pre_kernel<TR, TX, TY, NOX><<<g, MG_THREADS, smem, s>>>(F.d, F.coef, r, F.x1, C.d, C.coef, C.cp, C.minv,
+                                                                         C.r, out, omega, gate);
+    }
 }
 
 // nox: level f was not pre-smoothed (its x1 is zero): restrict r_f alone.
@@ -2177,12 +2399,13 @@ static const float *dense_visit(const Mg &mg, const MgLevel &F, const TR *r, con
     const int n = mg.dense_n, g = (4 * n + DN_THREADS - 1) / DN_THREADS, rows = DN_THREADS / 32;
     {
         ProfScope ps_(kLevelName[2][mg.dense_level], nox ? sizeof(TR) * N + 4.0 * n : (60.0 + sizeof(TR) + 4.0) * N, s);
-        if (nox) dense_restrict_kernel<TR, true><<<g, DN_THREADS, 0, s>>>(F.d, F.coef, r, F.x1, C.d, n, mg.dense_r, gate);
-        else dense_restrict_kernel<TR, false><<<g, DN_THREADS, 0, s>>>(F.d, F.coef, r, F.x1, C.d, n, mg.dense_r, gate);
+        launch_pdl(nox ? dense_restrict_kernel<TR, true> : dense_restrict_kernel<TR, false>, g, DN_THREADS, 0, s, F.d, F.coef,
+                   r, F.x1, C.d, n, mg.dense_r, gate);
         count_launch(1);
     }
     ProfScope ps_(kDenseName[mg.dense_level], 4.0 * n * (mg.dense_ld + 2.0), s);
-    dense_apply_kernel<<<(n + rows - 1) / rows, DN_THREADS, 0, s>>>(mg.dense, n, mg.dense_ld, mg.dense_r, C.d, C.x3, gate);
+    launch_pdl(dense_apply_kernel, (n + rows - 1) / rows, DN_THREADS, 0, s, mg.dense, n, mg.dense_ld, mg.dense_r, C.d, C.x3,
+               gate);
     count_launch(1);
     return C.x3;
 }
