@@ -212,8 +212,7 @@ static int mg_ensure(hicarw_handle *h, cudaStream_t s)
         h->mg_dirty = 0;
         return 1;
     }
-    const int rc = mg_refresh(h->mg, s);
-    return rc < 0 ? HICARW_ERR_CUDA : rc;
+    return mg_refresh(h->mg, s);
 }
 
 static Metrics metrics_of(const hicarw_handle *h)

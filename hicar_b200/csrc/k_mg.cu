@@ -1449,7 +1449,7 @@ __global__ void __launch_bounds__(MG_FUSE_THREADS) coarse_cycle_kernel(const __g
 }
 
 // ---------------------------------------------------------------------------
-// Dense coarse cycle.  From a level of at most MG_DENSE_MAX unknowns down, the
+// Dense coarse cycle.  From a level of a few thousand unknowns down, the
 // cycle (its pre-smoothing, W repeats and post-smoothings included) is a fixed
 // linear map of that level's right-hand side, so the build tabulates it as one
 // n x n matrix and a visit is one matrix-vector product: two short launches
@@ -1459,11 +1459,17 @@ __global__ void __launch_bounds__(MG_FUSE_THREADS) coarse_cycle_kernel(const __g
 // factors, rounded once to FP32; the product accumulates in FP32, 32 partial
 // sums per row.
 // What bounds it: the launch and one L2 round trip (n = 1024: 4 MB of matrix,
-// read once per visit by rows spread over the whole chip).  n <= 2048 keeps
-// the matrix at 16 MB, a few us from L2 or HBM.  A solve to 1e-9 (B200): 64x64x20
+// read once per visit by rows spread over the whole chip).  How large: the
+// product costs about 4.5 us plus the matrix at HBM rate (n = 2048: 3 us, 3072:
+// 6, 4096: 10), one level further down about 12 us a visit, twice that on a
+// level that corrects twice.  So n <= 3072, 4096 on a level with repeats, where
+// the next level down would take over otherwise (with n <= 2048 / 4096 on every
+// level: 181x157x33, n = 3960 with repeats, 7.29 / 6.10 ms a solve; 512x512x48,
+// n = 3072 without, 37.0 / 35.0; 1024x1024x64, n = 4096 without, 155.8 / 165.7).
+// A solve to 1e-9 (B200): 64x64x20
 // 8.29 -> 2.92 ms, 181x157x33 17.7 -> 9.7 ms, 512x512x48 52.5 -> 45.3 ms.
 // ---------------------------------------------------------------------------
-constexpr int MG_DENSE_MAX = 2048;
+constexpr int MG_DENSE_MAX = 3072, MG_DENSE_MAX_W = 4096; // unknowns, without and with repeats
 constexpr int DN_THREADS = 128;
 
 __device__ __forceinline__ int dense_index(const Dims &d, int i, int k, int j)
@@ -2353,7 +2359,9 @@ static bool dense_setup(Mg &mg, cudaStream_t s)
     int l0 = 0;
     if (!getenv("HICARW_MG_FUSE"))
         for (int l = 1; l < mg.nlev && !l0; l++)
-            if ((long long)mg.lev[l].d.nx * mg.lev[l].d.ny * mg.lev[l].d.nz <= MG_DENSE_MAX) l0 = l;
+            if ((long long)mg.lev[l].d.nx * mg.lev[l].d.ny * mg.lev[l].d.nz <=
+                ((mg.wmask >> l) & 1 ? MG_DENSE_MAX_W : MG_DENSE_MAX))
+                l0 = l;
     // a level cut off by MG_MAX_LEVELS is not a single column: the step-by-step forms handle it
     if (mg.lev[mg.nlev - 1].d.nx != 1 || mg.lev[mg.nlev - 1].d.ny != 1) l0 = 0;
     if (l0 != mg.dense_level) dense_free(mg);
@@ -2376,13 +2384,14 @@ static bool dense_setup(Mg &mg, cudaStream_t s)
 }
 
 // Before the launches of a cycle are enqueued: the dense matrix belongs to the
-// cycle's present parameters.  1: it was tabulated again, 0: it stands, -1: error.
+// cycle's present parameters.  1: the launches changed, 0: they stand.
 int mg_refresh(Mg &mg, cudaStream_t s)
 {
     if (!mg.ready || !mg.dense_level ||
         (mg.dense_omega == mg.omega && mg.dense_cscale == mg.cscale && mg.dense_wmask == mg.wmask))
         return 0;
-    return dense_fill(mg, s) ? 1 : -1;
+    if (!dense_setup(mg, s)) fused_setup(mg); // the level may move with the repeats
+    return 1;
 }
 
 static const char *kDenseName[MG_MAX_LEVELS] = {

@@ -45,7 +45,7 @@ struct Mg {
 
 int mg_build(Mg &mg, const Dims &fine, const float *fine_coef, cudaStream_t s);
 void mg_free(Mg &mg);
-int mg_refresh(Mg &mg, cudaStream_t s); // after a change of omega, cscale or wmask: 1 when the dense matrix was made again
+int mg_refresh(Mg &mg, cudaStream_t s); // after a change of omega, cscale or wmask: 1 when the cycle's launches changed
 long long mg_tma_posts(); // post-smoother launches enqueued through the tensor-copy kernel
 template <typename V>
 void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStream_t s);
