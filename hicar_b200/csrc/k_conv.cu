@@ -3,17 +3,21 @@
 // used by the learned preconditioner.
 //
 // Forward (and data-gradient, with the flipped/transposed weight image) as an
-// implicit GEMM: one 128-cell x-tile at (j, k) is D[128 x COUT] =
-// sum over 27 taps and CIN/16 channel chunks of A_tap[128 x 16] * B_tap[COUT x 16]^T.
-// The 9 neighbouring x-lines (dj, dk) of the tile, 130 cells each (one halo
-// cell per side), are bulk-copied into shared memory with one 2080-byte copy per
-// (line, channel group); in that no-swizzle K-major layout a tap's A operand is
-// the line's matrix descriptor with the start address moved by (di+1) rows of
-// 16 bytes, so the three x-shifts of a line share one copy.  The weight image is
-// stored in global memory exactly as the B operands' shared-memory image and is
-// bulk-copied once per CTA.  Persistent CTAs of 128 threads (one TMEM lane per
-// thread) double-buffer the line stages: the copies of the next tile are in
-// flight while the current tile's MMAs and epilogue run.
+// implicit GEMM.  A persistent CTA takes blocks of one 128-cell x-tile, four
+// output lines in j and KC levels, and marches through the block's input levels:
+// six x-lines of 130 cells (one halo cell per side) per level, bulk-copied with
+// one 2080-byte copy per (line, channel group).  In that no-swizzle K-major
+// layout a tap's A operand is the line's matrix descriptor with the start address
+// moved by (di+1) rows of 16 bytes.  One MMA multiplies a line by the stacked
+// weights of the taps dj = 1, 0, -1 (N = 3 cout): the accumulators of the four
+// output lines of a level lie side by side in tensor memory, so the three
+// products land in neighbouring columns.  Four accumulator levels rotate (three
+// being summed, one in the epilogue).  A copy warp, an MMA thread and four
+// epilogue warps run side by side, tied by mbarriers.
+// What bounds it: an MMA with N <= 64 takes as long as reading its A operand (4
+// KB), so the taps are merged in N (13.5 MMAs per 128-cell tile and 16 input
+// channels instead of 27), and a line is fetched 1.5 times instead of 9.  B200,
+// 16 -> 16 channels at 512x512x48: 0.84 -> 0.34 ms; 32 -> 32 at 64x64x48: 91 -> 46 us.
 //
 // Weight gradient: dW_tap[CIN x COUT] = sum over cells of X(v + tap)^T dY(v):
 // the reduction runs over cells (the MMA's K), both operands MN-major straight
@@ -23,7 +27,10 @@
 // three x-shifts are three accumulators.  Each persistent CTA accumulates all of
 // its tiles in TMEM and adds its partial sums to the FP32 gradient at the end.
 #include <cuda_bf16.h>
+#include <limits.h>
 #include <stdio.h>
+
+#include <algorithm>
 
 #include "kernels.h"
 #include "tc05.cuh"
@@ -64,30 +71,66 @@ __device__ __forceinline__ uint4 pack8(const float *f)
 template <int CIN, int COUT>
 struct FwdCfg {
     static constexpr int GI = CIN / 8, GO = COUT / 8;
-    static constexpr int WB = 27 * GI * COUT * 16; // weight image bytes
-    static constexpr int STAGE = 9 * GI * LG;      // one tile's line images
-    static constexpr int NCOL = 2 * COUT <= 32 ? 32 : (2 * COUT <= 64 ? 64 : 128);
-    static constexpr int SMEM = WB + 2 * STAGE + 64;
-    static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 128, "channel counts");
+    static constexpr int TJ = 4, NL = TJ + 2;       // output and input lines of a block in j
+    static constexpr int SLOTS = 4;                 // accumulator levels: three in the making, one in the epilogue
+    static constexpr int WB = 27 * GI * COUT * 16;  // weight image bytes
+    static constexpr int STAGE = NL * GI * LG;      // one input level's line images
+    static constexpr int NCOL = SLOTS * TJ * COUT;  // 256 or 512
+    static constexpr int NS = 3;                    // input levels in flight
+    static constexpr int SMEM = WB + NS * STAGE + 128;
+    static constexpr int PER_SM = NCOL <= 256 && SMEM <= 113 * 1024 ? 2 : 1;
+    static_assert(CIN % 16 == 0 && COUT % 16 == 0 && NCOL <= 512 && 3 * COUT <= 256, "channel counts");
     static_assert(SMEM <= 232448, "shared memory");
 };
 
+// How a launch splits the grid: blocks of one x-tile, TJ output lines in j and
+// KC output levels, nkb of them in k, njb in j (k fastest).
+struct ConvSplit {
+    int KC, nkb, njb, units;
+};
+
+struct ConvBlock {
+    int tx, j0, k0, nj, nk; // first output line and level, how many of each
+    int lo, hi;             // input levels read (the halo levels are zero and left out)
+};
+
+__device__ __forceinline__ ConvBlock conv_block(const ActDims &d, const ConvSplit &p, int TJ, int u)
+{
+    ConvBlock b;
+    b.k0 = u % p.nkb * p.KC;
+    b.j0 = u / p.nkb % p.njb * TJ;
+    b.tx = u / (p.nkb * p.njb);
+    b.nj = min(TJ, d.ny - b.j0);
+    b.nk = min(p.KC, d.nz - b.k0);
+    b.lo = max(b.k0 - 1, 0);
+    b.hi = min(b.k0 + b.nk, d.nz - 1);
+    return b;
+}
+
+constexpr int CONV_THREADS = 192; // warps 0-3 epilogue (TMEM lanes 32 w .. 32 w + 31), 4 copies, 5 MMAs
+
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) conv3_fwd_kernel(ConvArgs a)
+__global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, ConvSplit p)
 {
     using C = FwdCfg<CIN, COUT>;
+    constexpr int NS = C::NS, TJ = C::TJ, SLOTS = C::SLOTS;
     if (conv_gated(a.gate)) return;
     extern __shared__ __align__(128) uint8_t sm[];
-    uint8_t *wsm = sm;
-    uint8_t *stg0 = sm + C::WB, *stg1 = sm + C::WB + C::STAGE;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + C::WB + 2 * C::STAGE); // copy[0], copy[1], mma[0], mma[1]
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 4);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    uint8_t *wsm = sm, *stg = sm + C::WB;
+    uint64_t *full = reinterpret_cast<uint64_t *>(stg + NS * C::STAGE), *empty = full + NS, *tfull = empty + NS,
+             *tempty = tfull + SLOTS;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(tempty + SLOTS);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const ActDims di = a.din, dd = a.dout;
-    const int ntx = (di.nx + TILE - 1) / TILE;
-    const int ntiles = ntx * di.nz * di.ny;
     if (tid == 0) {
-        for (int q = 0; q < 4; q++) tc::mbar_init(&bars[q], 1);
+        for (int q = 0; q < NS; q++) {
+            tc::mbar_init(&full[q], 1);
+            tc::mbar_init(&empty[q], 1);
+        }
+        for (int q = 0; q < SLOTS; q++) {
+            tc::mbar_init(&tfull[q], 1);
+            tc::mbar_init(&tempty[q], 4);
+        }
         tc::mbar_fence_init();
     }
     if (warp == 0) tc::tmem_alloc(tslot, C::NCOL);
@@ -95,122 +138,169 @@ __global__ void __launch_bounds__(128) conv3_fwd_kernel(ConvArgs a)
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = *tslot;
-    const char *inb = reinterpret_cast<const char *>(a.in);
-
-    // called by all lanes of warp 0: lane 0 posts the byte count, then the lanes
-    // issue one bulk copy each
-    auto issue = [&](int tile, int s, bool with_w) {
-        const int tx = tile % ntx, r = tile / ntx, k = r % di.nz, j = r / di.nz;
-        const int lane = tid & 31;
-        uint8_t *dst = s ? stg1 : stg0;
-        if (lane == 0) tc::mbar_expect_tx(&bars[s], C::STAGE + (with_w ? C::WB : 0));
-        __syncwarp();
-        if (with_w && lane == 31) tc::bulk_g2s(wsm, a.w, C::WB, &bars[s]);
-        for (int q = lane; lane < 31 && q < 9 * C::GI; q += 31) { // lanes 0..30: the line images
-            const int sl = q / C::GI, g = q % C::GI;
-            const long long L = (long long)(j + sl / 3) * (di.nz + 2) + (k + sl % 3); // line (j+dj+1, k+dk+1)
-            tc::bulk_g2s(dst + (sl * C::GI + g) * LG, inb + ((L * C::GI + g) * di.PX + (long long)tx * TILE) * 16, LG,
-                         &bars[s]);
+    bool ok = true;
+    auto wait = [&](uint64_t *bar, int use) { // the use-th completion (from 0); on time-out: no more waits
+        if (ok && !tc::mbar_wait(bar, use & 1)) {
+            if (lane == 0) atomicExch(a.err, 1);
+            ok = false;
         }
     };
 
-    constexpr uint32_t IDESC = tc::idesc_bf16(128, COUT, 0, 0);
-    // Pipeline: in iteration `it` the MMAs of tile `it` (TMEM buffer it&1) run
-    // while the epilogue of tile it-1 (buffer (it-1)&1) reads the other buffer,
-    // and the copies of tile it+1 go into the line stage that tile it-1 used,
-    // issued as soon as its MMAs have completed.  mbarriers: [0], [1] line
-    // stages, [2], [3] MMA completion per TMEM buffer.
-    bool ok = true;
-    int it = 0, tile = blockIdx.x, prev = -1;
-    if (warp == 0 && tile < ntiles) issue(tile, 0, true);
-    for (;; it++) {
-        const bool have = tile < ntiles;
-        const int s = it & 1;
-        if (have) {
-            const bool got = tc::mbar_wait(&bars[s], (it >> 1) & 1);
-            if (!__syncthreads_and(got)) { ok = false; break; }
-            if (tid == 0) {
+    if (warp == 4) { // ---- copies: one input level per stage, one bulk copy per (line, channel group) ----
+        const char *inb = reinterpret_cast<const char *>(a.in);
+        int it = 0;
+        for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+            const ConvBlock b = conv_block(di, p, TJ, u);
+            for (int kk = b.lo; kk <= b.hi; kk++, it++) {
+                const int s = it % NS;
+                if (it >= NS) wait(&empty[s], it / NS - 1);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const int n = (b.nj + 2) * C::GI;
+                if (lane == 0) tc::mbar_expect_tx(&full[s], n * LG + (it == 0 ? C::WB : 0));
+                __syncwarp();
+                if (it == 0 && lane == 31) tc::bulk_g2s(wsm, a.w, C::WB, &full[s]);
+                for (int q = lane; q < n; q += 32) {
+                    const int l = q / C::GI, g = q % C::GI; // input line j0 - 1 + l, level kk
+                    const long long L = (long long)(b.j0 + l) * (di.nz + 2) + (kk + 1);
+                    tc::bulk_g2s(stg + s * C::STAGE + q * LG, inb + ((L * C::GI + g) * di.PX + (long long)b.tx * TILE) * 16,
+                                 LG, &full[s]);
+                }
+            }
+            if (!ok) break;
+        }
+        // nothing in flight at the end: the last stages landed and were read
+        for (int q = it > NS ? it - NS : 0; q < it; q++) {
+            if (!tc::mbar_wait(&full[q % NS], (q / NS) & 1) && lane == 0) atomicExch(a.err, 1);
+            wait(&empty[q % NS], q / NS);
+        }
+    } else if (warp == 5) { // ---- MMAs, one thread ----
+        if (lane == 0) {
+            // descriptors of the stage / weight bases; operands are byte offsets from them (start field = address >> 4)
+            const uint64_t b0 = tc::sdesc(tc::smem_u32(wsm), 3 * COUT * 16, 128);
+            int it = 0, n0 = 0; // n0: output levels of the blocks before
+            for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+                const ConvBlock b = conv_block(di, p, TJ, u);
+                for (int kk = b.lo; kk <= b.hi; kk++, it++) {
+                    const int s = it % NS;
+                    wait(&full[s], it / NS);
+                    // output levels first touched here: their slots must be read out
+                    for (int k = kk == b.lo ? b.k0 : kk + 1; k <= kk + 1 && k < b.k0 + b.nk; k++) {
+                        const int n = n0 + k - b.k0;
+                        if (n >= SLOTS) wait(&tempty[n % SLOTS], n / SLOTS - 1);
+                    }
+                    if (!ok) continue;
+                    tc::fence_after();
+                    const uint64_t a0 = tc::sdesc(tc::smem_u32(stg + s * C::STAGE), LG, 128);
+                    for (int dk = 2; dk >= 0; dk--) { // tap dk - 1: output level k = kk - (dk - 1)
+                        const int k = kk + 1 - dk;
+                        if (k < b.k0 || k >= b.k0 + b.nk) continue;
+                        const bool fresh = kk == max(k - 1, b.lo);
+                        const uint32_t d0 = tmem + (uint32_t)((n0 + k - b.k0) % SLOTS * TJ * COUT);
+#pragma unroll
+                        for (int dil = 0; dil < 3; dil++)
+#pragma unroll
+                            for (int c = 0; c < C::GI / 2; c++) {
+                                const uint64_t bt = b0 + (uint64_t)((((dk * 3 + dil) * C::GI + 2 * c) * 3 * COUT * 16) >> 4);
+                                const bool first = fresh && dil == 0 && c == 0;
+#pragma unroll
+                                for (int l = 0; l < C::NL; l++) {
+                                    // line l feeds the output lines l - 2 .. l with the taps dj = 1, 0, -1
+                                    if (l >= b.nj + 2) break;
+                                    const int o0 = l - 2 > 0 ? l - 2 : 0;
+                                    const int o1 = min(l, b.nj - 1), old = first ? min(l - 1, o1) : o1;
+                                    const uint64_t ad = a0 + (uint64_t)(((l * C::GI + 2 * c) * LG + dil * 16) >> 4);
+                                    const int skip = o0 - (l - 2); // taps of lines outside the block
+                                    if (old >= o0)
+                                        tc::mma_bf16(d0 + o0 * COUT, ad, bt + (uint64_t)(skip * COUT),
+                                                     tc::idesc_bf16(128, 0, 0, 0) | ((uint32_t)((old - o0 + 1) * COUT / 8) << 17), 1u);
+                                    if (first && o1 == l) // output line l gets its first product
+                                        tc::mma_bf16(d0 + l * COUT, ad, bt + (uint64_t)(2 * COUT),
+                                                     tc::idesc_bf16(128, COUT, 0, 0), 0u);
+                                }
+                            }
+                    }
+                    tc::mma_commit(&empty[s]);
+                    if (kk - 1 >= b.k0) tc::mma_commit(&tfull[(n0 + kk - 1 - b.k0) % SLOTS]);
+                    if (kk == b.hi && kk < b.k0 + b.nk) tc::mma_commit(&tfull[(n0 + kk - b.k0) % SLOTS]);
+                }
+                n0 += b.nk;
+            }
+        }
+        __syncwarp();
+    } else { // ---- epilogue: thread = cell of the x-tile ----
+        float bias[COUT];
+#pragma unroll
+        for (int c = 0; c < COUT; c++) bias[c] = a.bias ? __ldg(a.bias + c) : 0.0f;
+        int n = 0;
+        for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+            const ConvBlock b = conv_block(di, p, TJ, u);
+            const int i = b.tx * TILE + tid;
+            for (int k = b.k0; k < b.k0 + b.nk; k++, n++) {
+                const int slot = n % SLOTS;
+                wait(&tfull[slot], n / SLOTS);
                 tc::fence_after();
-                // descriptors of the stage / weight bases; every operand is a
-                // compile-time byte offset from them (start field = address >> 4)
-                const uint64_t a0 = tc::sdesc(tc::smem_u32(s ? stg1 : stg0), LG, 128);
-                const uint64_t b0 = tc::sdesc(tc::smem_u32(wsm), COUT * 16, 128);
+                for (int o = 0; o < b.nj; o++) {
+                    const int j = b.j0 + o;
+                    uint32_t r[COUT / 16][16];
 #pragma unroll
-                for (int t = 0; t < 27; t++) {
+                    for (int q = 0; q < COUT / 16; q++)
+                        tc::tmem_ld16_async(tmem + ((uint32_t)(warp * 32) << 16) +
+                                                (uint32_t)((slot * TJ + o) * COUT + q * 16),
+                                            r[q]);
+                    const bool live = i < di.nx;
+                    uint4 sk[C::GO], mk[C::GO];
+                    if (live && a.skip) {
 #pragma unroll
-                    for (int c = 0; c < C::GI / 2; c++) {
-                        const uint64_t ad = a0 + (uint64_t)((((t / 3) * C::GI + 2 * c) * LG + (t % 3) * 16) >> 4);
-                        const uint64_t bd = b0 + (uint64_t)(((t * C::GI + 2 * c) * COUT * 16) >> 4);
-                        tc::mma_bf16(tmem + s * COUT, ad, bd, IDESC, (t | c) ? 1u : 0u);
+                        for (int g = 0; g < C::GO; g++) sk[g] = a.skip[act_unit(dd, i, k, j, g)];
                     }
+                    if (live && a.mask) {
+#pragma unroll
+                        for (int g = 0; g < C::GO; g++) mk[g] = a.mask[act_unit(dd, i, k, j, g)];
+                    }
+                    float v[COUT];
+#pragma unroll
+                    for (int q = 0; q < COUT / 16; q++) {
+                        tc::tmem_ld_wait(r[q]);
+#pragma unroll
+                        for (int e = 0; e < 16; e++) v[q * 16 + e] = __uint_as_float(r[q][e]) + bias[q * 16 + e];
+                    }
+                    if (o == b.nj - 1) { // the slot is read out
+                        tc::fence_before();
+                        __syncwarp();
+                        if (lane == 0) tc::mbar_arrive(&tempty[slot]);
+                    }
+                    if (!live) continue;
+                    if (a.skip) {
+#pragma unroll
+                        for (int g = 0; g < C::GO; g++) {
+                            float f[8];
+                            unpack8(sk[g], f);
+#pragma unroll
+                            for (int e = 0; e < 8; e++) v[g * 8 + e] += f[e];
+                        }
+                    }
+                    if (a.relu) {
+#pragma unroll
+                        for (int c = 0; c < COUT; c++) v[c] = fmaxf(v[c], 0.0f);
+                    }
+                    if (a.mask) {
+#pragma unroll
+                        for (int g = 0; g < C::GO; g++) {
+                            float f[8];
+                            unpack8(mk[g], f);
+#pragma unroll
+                            for (int e = 0; e < 8; e++) v[g * 8 + e] = f[e] > 0.0f ? v[g * 8 + e] : 0.0f;
+                        }
+                    }
+                    if (a.out) {
+#pragma unroll
+                        for (int g = 0; g < C::GO; g++) a.out[act_unit(dd, i, k, j, g)] = pack8(v + g * 8);
+                    }
+                    if (a.out0) a.out0[((long long)j * dd.nz + k) * dd.nx + i] = v[0];
                 }
-                tc::mma_commit(&bars[2 + s]);
             }
         }
-        const int nxt = have ? tile + (int)gridDim.x : ntiles;
-        if (it == 0) {
-            if (warp == 0 && nxt < ntiles) issue(nxt, s ^ 1, false); // stage 1 not used yet
-        } else {
-            // tile it-1: its MMAs done -> its line stage is free, its accumulator readable
-            const bool done = tc::mbar_wait(&bars[2 + (s ^ 1)], ((it - 1) >> 1) & 1);
-            if (!__syncthreads_and(done)) { ok = false; break; }
-            if (warp == 0 && nxt < ntiles) issue(nxt, s ^ 1, false);
-            tc::fence_after();
-            const int tx = prev % ntx, r = prev / ntx, k = r % di.nz, j = r / di.nz;
-            const int i = tx * TILE + tid;
-            const uint32_t acc_col = (uint32_t)((s ^ 1) * COUT);
-            float v[COUT];
-#pragma unroll
-            for (int q = 0; q < COUT / 16; q++) {
-                float t16[16];
-                tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + acc_col + (uint32_t)(q * 16), t16);
-#pragma unroll
-                for (int e = 0; e < 16; e++) v[q * 16 + e] = t16[e];
-            }
-            if (i < di.nx) {
-                if (a.bias) {
-#pragma unroll
-                    for (int c = 0; c < COUT; c++) v[c] += __ldg(a.bias + c);
-                }
-                if (a.skip) {
-#pragma unroll
-                    for (int g = 0; g < C::GO; g++) {
-                        float f[8];
-                        unpack8(a.skip[act_unit(dd, i, k, j, g)], f);
-#pragma unroll
-                        for (int e = 0; e < 8; e++) v[g * 8 + e] += f[e];
-                    }
-                }
-                if (a.relu) {
-#pragma unroll
-                    for (int c = 0; c < COUT; c++) v[c] = fmaxf(v[c], 0.0f);
-                }
-                if (a.mask) {
-#pragma unroll
-                    for (int g = 0; g < C::GO; g++) {
-                        float f[8];
-                        unpack8(a.mask[act_unit(dd, i, k, j, g)], f);
-#pragma unroll
-                        for (int e = 0; e < 8; e++) v[g * 8 + e] = f[e] > 0.0f ? v[g * 8 + e] : 0.0f;
-                    }
-                }
-                if (a.out) {
-#pragma unroll
-                    for (int g = 0; g < C::GO; g++) a.out[act_unit(dd, i, k, j, g)] = pack8(v + g * 8);
-                }
-                if (a.out0) a.out0[((long long)j * dd.nz + k) * dd.nx + i] = v[0];
-            }
-        }
-        tc::fence_before();
-        __syncthreads();
-        if (!have) break;
-        prev = tile;
-        tile = nxt;
-    }
-    if (!ok && tid == 0) {
-        atomicExch(a.err, 1);
-        // bounded waits for the copies and MMAs this CTA may still have in flight
-        for (int q = 0; q < 4; q++) tc::mbar_wait(&bars[q], (uint32_t)(q < 2 ? (it >> 1) & 1 : (it & 1)), 100000000ull);
     }
     tc::fence_before();
     __syncthreads();
@@ -361,12 +451,20 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
 }
 
 // ---------------------------------------------------------------------------
+// Element (t, ci, co) of the weight image of a conv cin -> cout: per (dk, di) and
+// group of 8 input channels a column of 3 cout rows of 16 bytes, the taps dj = 1,
+// 0, -1 below one another (the order of the output lines that they feed).
+__device__ __forceinline__ int wimage_at(int t, int ci, int co, int cin, int cout)
+{
+    return ((t % 9 * (cin / 8) + ci / 8) * 3 * cout + (2 - t / 9) * cout + co) * 8 + (ci & 7);
+}
+
 __global__ void conv_pack_fwd_kernel(const float *__restrict__ W, int cin, int cout, __nv_bfloat16 *__restrict__ img)
 {
     const int n = 27 * cin * cout;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         const int t = q / (cin * cout), r = q % (cin * cout), ci = r / cout, co = r % cout;
-        img[(((long long)t * (cin / 8) + ci / 8) * cout + co) * 8 + (ci & 7)] = __float2bfloat16_rn(W[q]);
+        img[wimage_at(t, ci, co, cin, cout)] = __float2bfloat16_rn(W[q]);
     }
 }
 
@@ -377,8 +475,7 @@ __global__ void conv_pack_bwd_kernel(const float *__restrict__ W, int cin, int c
     const int n = 27 * cin * cout;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         const int t = q / (cin * cout), r = q % (cin * cout), ci = r / cout, co = r % cout;
-        const int tf = 26 - t;
-        img[(((long long)tf * (cout / 8) + co / 8) * cin + ci) * 8 + (co & 7)] = __float2bfloat16_rn(W[q]);
+        img[wimage_at(26 - t, co, ci, cout, cin)] = __float2bfloat16_rn(W[q]);
     }
 }
 
@@ -408,6 +505,25 @@ static int sm_count()
     return n;
 }
 
+// Levels per block: as few rounds of `resident` blocks, each of KC levels and
+// about three more in halo levels, fill and drain, as any split of nz gives.
+static ConvSplit conv_split(const ActDims &d, int TJ, int resident)
+{
+    ConvSplit best{};
+    long long cost = -1;
+    const long long cols = (long long)((d.nx + TILE - 1) / TILE) * ((d.ny + TJ - 1) / TJ);
+    for (int n = 1; n <= d.nz; n++) {
+        const int KC = (d.nz + n - 1) / n, nkb = (d.nz + KC - 1) / KC;
+        const long long units = cols * nkb, c = (units + resident - 1) / resident * (KC + 3);
+        if (units > INT_MAX) break;
+        if (cost < 0 || c < cost) {
+            cost = c;
+            best = ConvSplit{KC, nkb, (d.ny + TJ - 1) / TJ, (int)units};
+        }
+    }
+    return best;
+}
+
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
 template <int CI, int CO>
@@ -421,15 +537,14 @@ static int launch_fwd(const ConvArgs &a, cudaStream_t s)
             return -1;
         attr = true;
     }
-    const long long ntiles = (long long)((a.din.nx + TILE - 1) / TILE) * a.din.nz * a.din.ny;
-    const int per_sm = C::SMEM <= 113 * 1024 ? 2 : 1;
-    const int grid = (int)(ntiles < (long long)sm_count() * per_sm ? ntiles : (long long)sm_count() * per_sm);
+    const ConvSplit p = conv_split(a.din, C::TJ, sm_count() * C::PER_SM);
+    const int grid = std::min(p.units, sm_count() * C::PER_SM);
     if (grid <= 0) return 0;
     char name[32];
     snprintf(name, sizeof(name), "conv3_fwd_%dx%d", CI, CO);
     const double cells = (double)a.din.nx * a.din.ny * a.din.nz;
     ProfScope ps_(name, cells * 2.0 * (CI + CO), s);
-    conv3_fwd_kernel<CI, CO><<<grid, 128, C::SMEM, s>>>(a);
+    conv3_fwd_kernel<CI, CO><<<grid, CONV_THREADS, C::SMEM, s>>>(a, p);
     count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -1,0 +1,35 @@
+"""GPU tests of the blocked tensor-core convolution where its blocks end: output
+lines in fours, levels per block, 128-cell x-tiles, grids with fewer and with more
+blocks than CTAs."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+F = torch.nn.functional
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 16)])
+@pytest.mark.parametrize("nx,ny,nz", [(1, 1, 1), (128, 4, 2), (129, 5, 1), (40, 3, 9), (127, 8, 33), (257, 6, 5),
+                                      (20, 330, 7), (130, 61, 40)])
+def test_blocks_against_fp64(lib, cin, cout, nx, ny, nz):
+    """Channel 0 in FP32 against FP64 conv3d of the same BF16 values: 27 cin products
+    summed in FP32, 1e-4 of the largest value as in the kernel's other tests; the
+    BF16 outputs within BF16 rounding plus that; the halo stays zero."""
+    from hicar_b200 import learned as L
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    g = torch.Generator().manual_seed(nx + 7 * ny + nz)
+    bf = lambda t: t.to(torch.bfloat16).double()  # noqa: E731
+    x = bf(torch.randn((cin, ny, nz, nx), generator=g))
+    w = bf(torch.randn((27, cin, cout), generator=g) * 0.1)
+    b = torch.randn((cout,), generator=g)
+    wt = w.reshape(3, 3, 3, cin, cout).permute(4, 3, 0, 1, 2)
+    ref = F.conv3d(x[None], wt, b.double(), padding=1)[0]
+    out, out0 = L.conv3(L.to_act(x), w.float().cuda(), b.cuda(), nx, ny, nz, cin, cout, want_out0=True)
+    top = float(ref.abs().max())
+    assert float((out0.double().cpu() - ref[0]).abs().max()) <= 1e-4 * top
+    got = L.from_act(out, nx).double().cpu()
+    assert bool(((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-3 * top).all())
+    o = out.float()
+    o[1:-1, 1:-1, :, 1:nx + 1] = 0
+    assert not bool(o.any())
