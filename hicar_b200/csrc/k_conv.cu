@@ -42,6 +42,10 @@ constexpr int TILE = 128;
 constexpr int LROWS = TILE + 2;
 constexpr int LG = LROWS * 16; // bytes of one (line, channel group) image with halo
 constexpr int YG = TILE * 16;  // bytes of one (line, channel group) image without halo
+constexpr int SG = 17 * 128;   // pitch of the images in a forward stage, which start SGO past a multiple of 128 bytes,
+constexpr int SGO = 112;       // so that the core matrices of the unshifted taps are whole 128-byte lines (the other
+                               // shifts straddle two: an MMA's operand read takes twice as long)
+constexpr int up128(int b) { return (b + 127) / 128 * 128; }
 
 __device__ __forceinline__ bool conv_gated(const SolveState *g)
 {
@@ -74,10 +78,10 @@ struct FwdCfg {
     static constexpr int TJ = 4, NL = TJ + 2;       // output and input lines of a block in j
     static constexpr int SLOTS = 4;                 // accumulator levels: three in the making, one in the epilogue
     static constexpr int WB = 27 * GI * COUT * 16;  // weight image bytes
-    static constexpr int STAGE = NL * GI * LG;      // one input level's line images
+    static constexpr int STAGE = NL * GI * SG;      // one input level's line images
     static constexpr int NCOL = SLOTS * TJ * COUT;  // 256 or 512
     static constexpr int NS = 3;                    // input levels in flight
-    static constexpr int SMEM = WB + NS * STAGE + 128;
+    static constexpr int SMEM = up128(WB) + NS * STAGE + 256;
     static constexpr int PER_SM = NCOL <= 256 && SMEM <= 113 * 1024 ? 2 : 1;
     static_assert(CIN % 16 == 0 && COUT % 16 == 0 && NCOL <= 512 && 3 * COUT <= 256, "channel counts");
     static_assert(SMEM <= 232448, "shared memory");
@@ -109,6 +113,39 @@ __device__ __forceinline__ ConvBlock conv_block(const ActDims &d, const ConvSpli
 
 constexpr int CONV_THREADS = 192; // warps 0-3 epilogue (TMEM lanes 32 w .. 32 w + 31), 4 copies, 5 MMAs
 
+// One input level's MMAs of the taps dk into one output level's accumulators d0
+// (NJ output lines, or nj where NJ is 0): line l feeds the output lines l - 2 .. l
+// with the taps dj = 1, 0, -1; fresh: the accumulators get their first products.
+template <int CIN, int COUT, int NJ>
+__device__ __forceinline__ void issue_taps(int nj, uint64_t a0, uint64_t b0, uint32_t d0, int dk, bool fresh)
+{
+    using C = FwdCfg<CIN, COUT>;
+    const int lines = NJ ? NJ : nj;
+    const uint64_t bk = b0 + (uint64_t)((dk * 3 * C::GI * 3 * COUT * 16) >> 4);
+#pragma unroll
+    for (int dil = 0; dil < 3; dil++)
+#pragma unroll
+        for (int c = 0; c < C::GI / 2; c++) {
+            const uint64_t bt = bk + (uint64_t)(((dil * C::GI + 2 * c) * 3 * COUT * 16) >> 4);
+#pragma unroll
+            for (int l = 0; l < C::NL; l++) {
+                if (l >= lines + 2) break;
+                const int o0 = l - 2 > 0 ? l - 2 : 0, o1 = l < lines - 1 ? l : lines - 1;
+                const uint64_t ad = a0 + (uint64_t)(((l * C::GI + 2 * c) * SG + dil * 16) >> 4);
+                const uint64_t bd = bt + (uint64_t)((o0 - (l - 2)) * COUT); // without the taps of lines outside the block
+                const uint32_t all = tc::idesc_bf16(128, 0, 0, 0) | ((uint32_t)((o1 - o0 + 1) * COUT / 8) << 17);
+                if (dil == 0 && c == 0 && fresh) {
+                    const int old = l - 1 < o1 ? l - 1 : o1;
+                    if (old >= o0)
+                        tc::mma_bf16(d0 + o0 * COUT, ad, bd,
+                                     tc::idesc_bf16(128, 0, 0, 0) | ((uint32_t)((old - o0 + 1) * COUT / 8) << 17), 1u);
+                    if (o1 == l) // output line l gets its first product
+                        tc::mma_bf16(d0 + l * COUT, ad, bt + (uint64_t)(2 * COUT), tc::idesc_bf16(128, COUT, 0, 0), 0u);
+                } else tc::mma_bf16(d0 + o0 * COUT, ad, bd, all, 1u);
+            }
+        }
+}
+
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, ConvSplit p)
 {
@@ -116,8 +153,8 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
     constexpr int NS = C::NS, TJ = C::TJ, SLOTS = C::SLOTS;
     if (conv_gated(a.gate)) return;
     extern __shared__ __align__(128) uint8_t sm[];
-    uint8_t *wsm = sm, *stg = sm + C::WB;
-    uint64_t *full = reinterpret_cast<uint64_t *>(stg + NS * C::STAGE), *empty = full + NS, *tfull = empty + NS,
+    uint8_t *wsm = sm, *stg = sm + up128(C::WB) + SGO;
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + up128(C::WB) + NS * C::STAGE + 128), *empty = full + NS, *tfull = empty + NS,
              *tempty = tfull + SLOTS;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(tempty + SLOTS);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -163,7 +200,7 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
                 for (int q = lane; q < n; q += 32) {
                     const int l = q / C::GI, g = q % C::GI; // input line j0 - 1 + l, level kk
                     const long long L = (long long)(b.j0 + l) * (di.nz + 2) + (kk + 1);
-                    tc::bulk_g2s(stg + s * C::STAGE + q * LG, inb + ((L * C::GI + g) * di.PX + (long long)b.tx * TILE) * 16,
+                    tc::bulk_g2s(stg + s * C::STAGE + q * SG, inb + ((L * C::GI + g) * di.PX + (long long)b.tx * TILE) * 16,
                                  LG, &full[s]);
                 }
             }
@@ -191,34 +228,16 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
                     }
                     if (!ok) continue;
                     tc::fence_after();
-                    const uint64_t a0 = tc::sdesc(tc::smem_u32(stg + s * C::STAGE), LG, 128);
+                    const uint64_t a0 = tc::sdesc(tc::smem_u32(stg + s * C::STAGE), SG, 128);
                     for (int dk = 2; dk >= 0; dk--) { // tap dk - 1: output level k = kk - (dk - 1)
                         const int k = kk + 1 - dk;
                         if (k < b.k0 || k >= b.k0 + b.nk) continue;
                         const bool fresh = kk == max(k - 1, b.lo);
                         const uint32_t d0 = tmem + (uint32_t)((n0 + k - b.k0) % SLOTS * TJ * COUT);
-#pragma unroll
-                        for (int dil = 0; dil < 3; dil++)
-#pragma unroll
-                            for (int c = 0; c < C::GI / 2; c++) {
-                                const uint64_t bt = b0 + (uint64_t)((((dk * 3 + dil) * C::GI + 2 * c) * 3 * COUT * 16) >> 4);
-                                const bool first = fresh && dil == 0 && c == 0;
-#pragma unroll
-                                for (int l = 0; l < C::NL; l++) {
-                                    // line l feeds the output lines l - 2 .. l with the taps dj = 1, 0, -1
-                                    if (l >= b.nj + 2) break;
-                                    const int o0 = l - 2 > 0 ? l - 2 : 0;
-                                    const int o1 = min(l, b.nj - 1), old = first ? min(l - 1, o1) : o1;
-                                    const uint64_t ad = a0 + (uint64_t)(((l * C::GI + 2 * c) * LG + dil * 16) >> 4);
-                                    const int skip = o0 - (l - 2); // taps of lines outside the block
-                                    if (old >= o0)
-                                        tc::mma_bf16(d0 + o0 * COUT, ad, bt + (uint64_t)(skip * COUT),
-                                                     tc::idesc_bf16(128, 0, 0, 0) | ((uint32_t)((old - o0 + 1) * COUT / 8) << 17), 1u);
-                                    if (first && o1 == l) // output line l gets its first product
-                                        tc::mma_bf16(d0 + l * COUT, ad, bt + (uint64_t)(2 * COUT),
-                                                     tc::idesc_bf16(128, COUT, 0, 0), 0u);
-                                }
-                            }
+                        // whole blocks with the line count known at compile time: the issuing thread
+                        // then only adds constants to its descriptors
+                        if (b.nj == TJ) issue_taps<CIN, COUT, TJ>(TJ, a0, b0, d0, dk, fresh);
+                        else issue_taps<CIN, COUT, 0>(b.nj, a0, b0, d0, dk, fresh);
                     }
                     tc::mma_commit(&empty[s]);
                     if (kk - 1 >= b.k0) tc::mma_commit(&tfull[(n0 + kk - 1 - b.k0) % SLOTS]);
@@ -236,28 +255,30 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
         for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
             const ConvBlock b = conv_block(di, p, TJ, u);
             const int i = b.tx * TILE + tid;
+            const bool live = i < di.nx;
+            const long long js = (long long)(dd.nz + 2) * C::GO * dd.PX; // from one line to the next in j
             for (int k = b.k0; k < b.k0 + b.nk; k++, n++) {
                 const int slot = n % SLOTS;
+                const long long base = act_unit(dd, i, k, b.j0, 0);
+                // what the epilogue reads, fetched while the accumulators are still being summed
+                const uint4 *extra = a.skip ? a.skip : a.mask;
+                uint4 ex[TJ][C::GO];
+#pragma unroll
+                for (int o = 0; o < TJ; o++)
+#pragma unroll
+                    for (int g = 0; g < C::GO; g++)
+                        ex[o][g] = extra && live && o < b.nj ? extra[base + o * js + g * dd.PX] : make_uint4(0, 0, 0, 0);
                 wait(&tfull[slot], n / SLOTS);
                 tc::fence_after();
-                for (int o = 0; o < b.nj; o++) {
-                    const int j = b.j0 + o;
+#pragma unroll
+                for (int o = 0; o < TJ; o++) {
+                    if (o >= b.nj) break;
                     uint32_t r[COUT / 16][16];
 #pragma unroll
                     for (int q = 0; q < COUT / 16; q++)
                         tc::tmem_ld16_async(tmem + ((uint32_t)(warp * 32) << 16) +
                                                 (uint32_t)((slot * TJ + o) * COUT + q * 16),
                                             r[q]);
-                    const bool live = i < di.nx;
-                    uint4 sk[C::GO], mk[C::GO];
-                    if (live && a.skip) {
-#pragma unroll
-                        for (int g = 0; g < C::GO; g++) sk[g] = a.skip[act_unit(dd, i, k, j, g)];
-                    }
-                    if (live && a.mask) {
-#pragma unroll
-                        for (int g = 0; g < C::GO; g++) mk[g] = a.mask[act_unit(dd, i, k, j, g)];
-                    }
                     float v[COUT];
 #pragma unroll
                     for (int q = 0; q < COUT / 16; q++) {
@@ -271,11 +292,12 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
                         if (lane == 0) tc::mbar_arrive(&tempty[slot]);
                     }
                     if (!live) continue;
+                    const long long at = base + o * js;
                     if (a.skip) {
 #pragma unroll
                         for (int g = 0; g < C::GO; g++) {
                             float f[8];
-                            unpack8(sk[g], f);
+                            unpack8(ex[o][g], f);
 #pragma unroll
                             for (int e = 0; e < 8; e++) v[g * 8 + e] += f[e];
                         }
@@ -288,16 +310,16 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
 #pragma unroll
                         for (int g = 0; g < C::GO; g++) {
                             float f[8];
-                            unpack8(mk[g], f);
+                            unpack8(a.skip ? a.mask[at + g * dd.PX] : ex[o][g], f);
 #pragma unroll
                             for (int e = 0; e < 8; e++) v[g * 8 + e] = f[e] > 0.0f ? v[g * 8 + e] : 0.0f;
                         }
                     }
                     if (a.out) {
 #pragma unroll
-                        for (int g = 0; g < C::GO; g++) a.out[act_unit(dd, i, k, j, g)] = pack8(v + g * 8);
+                        for (int g = 0; g < C::GO; g++) a.out[at + g * dd.PX] = pack8(v + g * 8);
                     }
-                    if (a.out0) a.out0[((long long)j * dd.nz + k) * dd.nx + i] = v[0];
+                    if (a.out0) a.out0[((long long)(b.j0 + o) * dd.nz + k) * dd.nx + i] = v[0];
                 }
             }
         }
