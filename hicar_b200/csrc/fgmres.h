@@ -21,7 +21,8 @@ struct GmresState {
     double h1[FG_MAXM + 1], h2[FG_MAXM + 1];
 };
 
-typedef void (*PrecondFn)(void *ctx, const double *in, double *out, cudaStream_t s);
+// out = M^-1 in; true when it also left A out in w
+typedef bool (*PrecondFn)(void *ctx, const double *in, double *out, double *w, cudaStream_t s);
 
 struct FgmresCtx {
     OpCtx op;
@@ -30,12 +31,14 @@ struct FgmresCtx {
     double *V, *Z, *W;  // (m+1) basis vectors, m preconditioned vectors, work vector (padded layout)
     double *partials;
     int red_blocks, dot_blocks;
+    const SolveState *st; // the mirror of the stop flag, gates the kernels shared with BiCGStab
     GmresState *g;
     const double *g_h1, *g_h2, *g_hnext; // device addresses inside *g
     PrecondFn precond;
     void *pctx;
 };
 
+bool fgmres_init(); // once before the first launch (false: an attribute was refused)
 void fgmres_reset(GmresState *g, int m, double tol_rel, double tol_abs, int max_iters, double *hist, SolveState *mirror,
                   cudaStream_t s);
 void fgmres_set_profile(GmresState *g, int on, cudaStream_t s);

@@ -132,13 +132,13 @@ __global__ void __launch_bounds__(ROWT, m4_ctas<V>()) spmv_m4_kernel(OpCtx c, co
     if (gated(gate)) return;
     march4_rows<V, RAG>(
         c, x,
-        [&](long long o, const double (&v)[4]) {
+        [&](long long o, const double (&v)[4], bool) {
             V t[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) t[e] = (V)v[e];
             st4v(y + o, t);
         },
-        [&](long long o, double v) { y[o] = (V)v; });
+        [&](long long o, double v, bool) { y[o] = (V)v; });
 }
 
 template <typename V, bool RAG>
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(ROWT, M4_CTAS_DOT5) setup_m4_kernel(OpCtx c, c
     double acc[3] = {0.0, 0.0, 0.0};
     march4_rows<X, RAG>(
         c, x,
-        [&](long long o, const double (&y)[4]) {
+        [&](long long o, const double (&y)[4], bool) {
             V b[4], rv[4];
             ld4v(rhs + o, b);
 #pragma unroll
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(ROWT, M4_CTAS_DOT5) setup_m4_kernel(OpCtx c, c
             st4v(rhat + o, rv);
             st4v(p + o, rv);
         },
-        [&](long long o, double y) {
+        [&](long long o, double y, bool) {
             const double bd = (double)rhs[o];
             const V rv = (V)(bd - y);
             r[o] = rhat[o] = p[o] = rv;
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(ROWT, m4_ctas<V>()) spmv_sigma_m4_kernel(OpCtx
     double acc[1] = {0.0};
     march4_rows<V, RAG>(
         c, phat,
-        [&](long long o, const double (&y)[4]) {
+        [&](long long o, const double (&y)[4], bool) {
             V vv[4], rh[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) vv[e] = (V)y[e];
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(ROWT, m4_ctas<V>()) spmv_sigma_m4_kernel(OpCtx
 #pragma unroll
             for (int e = 0; e < 4; e++) acc[0] += (double)rh[e] * (double)vv[e];
         },
-        [&](long long o, double y) {
+        [&](long long o, double y, bool) {
             const V vv = (V)y;
             v[o] = vv;
             acc[0] += (double)rhat[o] * (double)vv;
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(ROWT, M4_CTAS_DOT5) spmv_dot5_m4_kernel(OpCtx 
     };
     march4_rows<V, RAG>(
         c, shat,
-        [&](long long o, const double (&y)[4]) {
+        [&](long long o, const double (&y)[4], bool) {
             V tv[4], s4[4], r4[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) tv[e] = (V)y[e];
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(ROWT, M4_CTAS_DOT5) spmv_dot5_m4_kernel(OpCtx 
 #pragma unroll
             for (int e = 0; e < 4; e++) add((double)tv[e], (double)s4[e], (double)r4[e]);
         },
-        [&](long long o, double y) {
+        [&](long long o, double y, bool) {
             const V tv = (V)y;
             t[o] = tv;
             add((double)tv, (double)sv[o], (double)rhat[o]);
@@ -533,6 +533,119 @@ void launch_spmv_dot5(const OpCtx &c, const V *shat, V *t, const V *s, const V *
         spmv_dot5_march_kernel<V><<<march_grid(spmv_dot5_march_kernel<V>, c.d, rb.blocks), ROWT, 0, st>>>(
             c, shat, t, s, rhat, stt, hist, rb.partials);
     else spmv_dot5_kernel<V><<<rb.blocks, ROWT, 0, st>>>(c, shat, t, s, rhat, stt, hist, rb.partials);
+    count_launch(1);
+}
+
+// ---- composite learned preconditioner: the passes between the V-cycle and the network ----
+// res = r - A z and its interior rms, left in scal (rms, 1 / rms) by the last CTA
+// (the network scales its input by it): the operator, the difference and the norm in one pass.
+template <bool RAG>
+__global__ void __launch_bounds__(ROWT, M4_CTAS_DOT5) mgl_residual_kernel(OpCtx c, const double *__restrict__ z,
+                                                                          const double *__restrict__ r,
+                                                                          double *__restrict__ res, float *scal,
+                                                                          SolveState *stt, double *partials,
+                                                                          const SolveState *gate)
+{
+    if (gated(gate)) return;
+    double acc[1] = {0.0};
+    march4_rows<double, RAG>(
+        c, z,
+        [&](long long o, const double (&y)[4], bool in) {
+            double rv[4], e[4];
+            ld4v(r + o, rv);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                e[q] = rv[q] - y[q];
+                if (in) acc[0] += e[q] * e[q];
+            }
+            st4v(res + o, e);
+        },
+        [&](long long o, double y, bool in) {
+            const double e = r[o] - y;
+            res[o] = e;
+            if (in) acc[0] += e * e;
+        });
+    double tot[1];
+    if (!grid_reduce<1>(acc, partials, &stt->ticket[4], tot)) return;
+    if (threadIdx.x == 0) {
+        const double rms = sqrt(tot[0] / ((double)c.d.nx * c.d.ny * c.d.nz));
+        scal[0] = (float)rms;
+        scal[1] = rms > 0.0 ? (float)(1.0 / rms) : 0.0f;
+    }
+}
+
+// au = A u and theta = <res, au> / <au, au> (0 when A u = 0), left in stt->mr_theta by the last CTA
+template <bool RAG>
+__global__ void __launch_bounds__(ROWT, M4_CTAS_DOT5) mgl_step_kernel(OpCtx c, const double *__restrict__ u,
+                                                                      const double *__restrict__ res,
+                                                                      double *__restrict__ au, SolveState *stt,
+                                                                      double *partials, const SolveState *gate)
+{
+    if (gated(gate)) return;
+    double acc[2] = {0.0, 0.0};
+    march4_rows<double, RAG>(
+        c, u,
+        [&](long long o, const double (&y)[4], bool) {
+            double rv[4];
+            ld4v(res + o, rv);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                acc[0] += rv[q] * y[q];
+                acc[1] += y[q] * y[q];
+            }
+            st4v(au + o, y);
+        },
+        [&](long long o, double y, bool) {
+            acc[0] += res[o] * y;
+            acc[1] += y * y;
+            au[o] = y;
+        });
+    double tot[2];
+    if (!grid_reduce<2>(acc, partials, &stt->ticket[5], tot)) return;
+    if (threadIdx.x == 0) stt->mr_theta = tot[1] > 0.0 ? tot[0] / tot[1] : 0.0;
+}
+
+// z += theta u; with w also w = A z of the result, from what is at hand: A M(r) = r - res and A u = au
+__global__ void mgl_add_kernel(long long n, const double *__restrict__ u, double *__restrict__ z, const SolveState *st,
+                               const double *__restrict__ r, const double *__restrict__ res,
+                               const double *__restrict__ au, double *__restrict__ w, const SolveState *gate)
+{
+    if (gated(gate)) return;
+    const double theta = st->mr_theta;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        z[q] += theta * u[q];
+        if (w) w[q] = (r[q] - res[q]) + theta * au[q];
+    }
+}
+
+void launch_mgl_residual(const OpCtx &c, const double *z, const double *r, double *res, float *scal, SolveState *stt,
+                         const RedBuf &rb, const SolveState *gate, cudaStream_t st)
+{
+    ProfScope ps_("mgl_residual", coef_bytes(c.d) + rows(c.d) * 24.0, st);
+    OpCtx m = c;
+    auto *kernel = c.d.nx % 4 ? mgl_residual_kernel<true> : mgl_residual_kernel<false>;
+    const int g = march4_grid(kernel, m, rb.blocks);
+    kernel<<<g, ROWT, 0, st>>>(m, z, r, res, scal, stt, rb.partials, gate);
+    count_launch(1);
+}
+
+void launch_mgl_step(const OpCtx &c, const double *u, const double *res, double *au, SolveState *stt, const RedBuf &rb,
+                     const SolveState *gate, cudaStream_t st)
+{
+    ProfScope ps_("mgl_step", coef_bytes(c.d) + rows(c.d) * 24.0, st);
+    OpCtx m = c;
+    auto *kernel = c.d.nx % 4 ? mgl_step_kernel<true> : mgl_step_kernel<false>;
+    const int g = march4_grid(kernel, m, rb.blocks);
+    kernel<<<g, ROWT, 0, st>>>(m, u, res, au, stt, rb.partials, gate);
+    count_launch(1);
+}
+
+static int ew_grid(long long n);
+void launch_mgl_add(const Dims &d, const double *u, double *z, const SolveState *stt, const double *r, const double *res,
+                    const double *au, double *w, const SolveState *gate, cudaStream_t st)
+{
+    ProfScope ps_("mgl_add", rows(d) * (w ? 56.0 : 24.0), st);
+    mgl_add_kernel<<<ew_grid(d.npad), 256, 0, st>>>(d.npad, u, z, stt, r, res, au, w, gate);
     count_launch(1);
 }
 
@@ -825,13 +938,13 @@ __global__ void __launch_bounds__(ROWT, M4_CTAS_DOT5) true_residual_m4_kernel(Op
     };
     march4_rows<X, RAG>(
         c, x,
-        [&](long long o, const double (&y)[4]) {
+        [&](long long o, const double (&y)[4], bool) {
             V b[4];
             ld4v(rhs + o, b);
 #pragma unroll
             for (int e = 0; e < 4; e++) one(o + e, (double)b[e] - y[e]);
         },
-        [&](long long o, double y) { one(o, (double)rhs[o] - y); });
+        [&](long long o, double y, bool) { one(o, (double)rhs[o] - y); });
     double tot[2];
     if (grid_reduce<2>(acc, partials, &stt->ticket[3], tot)) true_residual_finish(stt, tot, mode);
 }

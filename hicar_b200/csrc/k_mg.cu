@@ -1790,8 +1790,8 @@ int mg_build(Mg &mg, const Dims &fine, const float *fine_coef, cudaStream_t s)
         mg.coef0h = nullptr;
     }
     const cudaError_t e = cudaGetLastError();
-    mg.fuse_level = mg.cluster_n = 0;
-    if (!dense_setup(mg, s)) fused_setup(mg);
+    dense_setup(mg, s);
+    fused_setup(mg);
     mg.ready = 1;
     return e == cudaSuccess ? 0 : -1;
 }
@@ -2390,7 +2390,7 @@ int mg_refresh(Mg &mg, cudaStream_t s)
     if (!mg.ready || !mg.dense_level ||
         (mg.dense_omega == mg.omega && mg.dense_cscale == mg.cscale && mg.dense_wmask == mg.wmask))
         return 0;
-    if (!dense_setup(mg, s)) fused_setup(mg); // the level may move with the repeats
+    dense_setup(mg, s); // the level may move with the repeats
     return 1;
 }
 
@@ -2427,13 +2427,14 @@ static const float *dense_visit(const Mg &mg, const MgLevel &F, const TR *r, con
 // and the two post-smoothings alternate between the level's x1 and x3 buffers.
 // With no bit set the launches are those of the V-cycle: all restrictions
 // top-down, then all post-smoothings bottom-up, results in x3.
-static const float *coarse_cycle(const Mg &mg, int l, const SolveState *gate, cudaStream_t s)
+static const float *coarse_cycle(const Mg &mg, int l, const SolveState *gate, cudaStream_t s, bool steps)
 {
     const int L = mg.nlev;
     const MgLevel &F = mg.lev[l];
     if (l == L - 1) return F.x3; // exact column solve, written by the restriction from level l - 1
     const float *fused = nullptr;
-    if (mg.fuse_level > 0 && l == mg.fuse_level && launch_fused(mg, l, gate, s, &fused)) return fused;
+    const int dense = steps ? 0 : mg.dense_level;
+    if (!dense && mg.fuse_level > 0 && l == mg.fuse_level && launch_fused(mg, l, gate, s, &fused)) return fused;
     const MgLevel &C = mg.lev[l + 1];
     const bool last = l + 1 == L - 1;
     const int reps = (mg.wmask >> l) & 1 ? 2 : 1;
@@ -2442,10 +2443,10 @@ static const float *coarse_cycle(const Mg &mg, int l, const SolveState *gate, cu
         MgLevel Fi = F;
         Fi.x1 = cur; // the iterate whose residual is restricted and which the post-smoother corrects
         MgLevel Cr = C;
-        if (l + 1 == mg.dense_level) Cr.x3 = const_cast<float *>(dense_visit<float>(mg, Fi, F.r, gate, s, false));
+        if (l + 1 == dense) Cr.x3 = const_cast<float *>(dense_visit<float>(mg, Fi, F.r, gate, s, false));
         else {
             launch_restrict_pre<float>(Fi, F.r, C, l + 1, last ? C.x3 : C.x1, last ? 1.0f : mg.omega, gate, s);
-            Cr.x3 = const_cast<float *>(coarse_cycle(mg, l + 1, gate, s));
+            Cr.x3 = const_cast<float *>(coarse_cycle(mg, l + 1, gate, s, steps));
         }
         launch_post<float, float>(Fi, l, F.r, Cr, other, mg.omega, mg.cscale, gate, mg.use_tma, mg.err, s);
         std::swap(cur, other);
@@ -2456,10 +2457,11 @@ static const float *coarse_cycle(const Mg &mg, int l, const SolveState *gate, cu
 // out = V-cycle(in); in/out are outer Krylov vectors of type V on the fine level.
 // Launches: pre(0), restrict+pre(1..L-1) (exact solve on the last), post(L-2..0),
 // with the repeated coarse corrections of the levels in mg.wmask (coarse_cycle).
+// steps: every level step by step, although the coarse part has been tabulated.
 // Without fine pre-smoothing (mg.pre0 == 0) pre(0) is not launched, level 1
 // restricts `in` itself, and the finest post-smoother reads the zero x1.
 template <typename V>
-void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStream_t s)
+void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStream_t s, bool steps)
 {
     const int L = mg.nlev;
     const float w = mg.omega;
@@ -2469,17 +2471,17 @@ void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStr
     const MgLevel &C = mg.lev[1];
     const bool last = L == 2;
     MgLevel Cr = C;
-    if (mg.dense_level == 1) Cr.x3 = const_cast<float *>(dense_visit<V>(mg, F, in, gate, s, !mg.pre0));
+    if (!steps && mg.dense_level == 1) Cr.x3 = const_cast<float *>(dense_visit<V>(mg, F, in, gate, s, !mg.pre0));
     else {
         launch_restrict_pre<V>(F, in, C, 1, last ? C.x3 : C.x1, last ? 1.0f : w, gate, s, !mg.pre0);
-        Cr.x3 = const_cast<float *>(coarse_cycle(mg, 1, gate, s));
+        Cr.x3 = const_cast<float *>(coarse_cycle(mg, 1, gate, s, steps));
     }
     launch_post<V, V>(F, 0, in, Cr, out, w, mg.cscale, gate, mg.use_tma, mg.err, s,
                       mg.pre0 ? nullptr : mg.coef0h, !mg.pre0);
 }
 
-template void mg_apply<double>(const Mg &, const double *, double *, const SolveState *, cudaStream_t);
-template void mg_apply<float>(const Mg &, const float *, float *, const SolveState *, cudaStream_t);
+template void mg_apply<double>(const Mg &, const double *, double *, const SolveState *, cudaStream_t, bool);
+template void mg_apply<float>(const Mg &, const float *, float *, const SolveState *, cudaStream_t, bool);
 
 // ---- the bounded wait of the tensor-copy kernels, made to run out ----
 // An mbarrier that expects one arrival that never comes (no copy is issued to

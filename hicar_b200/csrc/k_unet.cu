@@ -38,7 +38,8 @@ static const int CSPEC[NCONV][3] = { // cin, cout, level
     {16, 16, 0}, {16, 32, 1}, {32, 32, 2}, {32, 32, 2}, {32, 16, 1}, {16, 16, 0}, {16, 16, 0}};
 
 enum { RS_POOL = 0, RS_UP = 1, RS_POOL_BWD = 2, RS_UP_BWD = 3 };
-constexpr int UNET_RED = 296; // partial-sum blocks of the reductions
+constexpr int UNET_RED = 296; // partial-sum blocks of the loss reductions
+constexpr int RMS_BLOCKS = 148 * 4;
 
 }  // namespace hw
 
@@ -57,7 +58,8 @@ struct hicarw_unet {
     uint4 *dO = nullptr, *dD0 = nullptr, *dU0 = nullptr, *dD1 = nullptr, *dU1 = nullptr, *dF2 = nullptr,
           *dE2 = nullptr, *dP2 = nullptr, *dE1 = nullptr, *dP1 = nullptr, *dE0 = nullptr;
     const uint4 *x_in = nullptr; // input of the last forward pass
-    double *red = nullptr;       // UNET_RED partial sums
+    double *red = nullptr;       // RMS_BLOCKS partial sums
+    unsigned int *ticket = nullptr;
     float *scal = nullptr;       // [0] rms, [1] 1/rms, [2] loss
     int *err = nullptr;
     std::vector<void *> allocs;
@@ -161,31 +163,19 @@ __device__ __forceinline__ void block_partial(double acc, double *part)
     }
 }
 
-// sum of squares of the interior of r -> per-block partials
-__global__ void __launch_bounds__(256) unet_sumsq_kernel(const double *__restrict__ r, VecView vw, Dims d,
-                                                         double *__restrict__ part, const SolveState *gate)
+// rms and 1/rms of the interior of r into scal[0], scal[1] (the last CTA)
+__global__ void __launch_bounds__(256) unet_rms_kernel(const double *__restrict__ r, VecView vw, Dims d, double *part,
+                                                       unsigned int *ticket, float *scal, const SolveState *gate)
 {
     if (ugated(gate)) return;
-    const long long n = (long long)d.nx * d.ny * d.nz;
-    double acc = 0.0;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(q % d.nx);
-        const long long t = q / d.nx;
-        const int k = (int)(t % d.nz), j = (int)(t / d.nz);
-        const double v = r[vw.at(i + 1, k + 1, j + 1)];
-        acc += v * v;
+    double acc[1] = {0.0}, tot[1];
+    const int lines = d.ny * d.nz;
+    for (int l = blockIdx.x; l < lines; l += gridDim.x) {
+        const double *row = r + vw.at(1, l % d.nz + 1, l / d.nz + 1);
+        for (int i = threadIdx.x; i < d.nx; i += 256) acc[0] += row[i] * row[i];
     }
-    block_partial(acc, part);
-}
-
-// rms and 1/rms of r (scal[0], scal[1]) from the partials
-__global__ void unet_rms_kernel(const double *__restrict__ part, int nb, long long n, float *scal,
-                                const SolveState *gate)
-{
-    if (ugated(gate)) return;
-    double s = 0.0;
-    for (int b = 0; b < nb; b++) s += part[b];
-    const double rms = sqrt(s / (double)n);
+    if (!grid_reduce<1>(acc, part, ticket, tot) || threadIdx.x != 0) return;
+    const double rms = sqrt(tot[0] / ((double)d.nx * d.ny * d.nz));
     scal[0] = (float)rms;
     scal[1] = rms > 0.0 ? (float)(1.0 / rms) : 0.0f;
 }
@@ -270,8 +260,9 @@ __global__ void __launch_bounds__(256) unet_loss_kernel(const float *__restrict_
 __global__ void unet_loss_final_kernel(const double *__restrict__ part, int nb, long long n, float w, float *scal)
 {
     double s = 0.0;
-    for (int b = 0; b < nb; b++) s += part[b];
-    scal[2] = (float)(w * s / (double)n);
+    for (int b = threadIdx.x; b < nb; b += 32) s += part[b];
+    s = warp_sum(s);
+    if (threadIdx.x == 0) scal[2] = (float)(w * s / (double)n);
 }
 
 // Stencil offsets (dk, dj, di) of coefficients A..O of the probed operator
@@ -465,7 +456,7 @@ static int unet_backward(hicarw_unet *n, const float *T, float w, cudaStream_t s
 {
     const long long nvox = (long long)n->nx[0] * n->ny[0] * n->nz;
     unet_loss_kernel<<<UNET_RED, 256, 0, s>>>(n->O0, T, n->nx[0], n->ny[0], n->nz, w, n->dO, adim(n, 0, 16), n->red);
-    unet_loss_final_kernel<<<1, 1, 0, s>>>(n->red, UNET_RED, nvox, w, n->scal);
+    unet_loss_final_kernel<<<1, 32, 0, s>>>(n->red, UNET_RED, nvox, w, n->scal);
     count_launch(2);
     return unet_backward_chain(n, s);
 }
@@ -479,7 +470,7 @@ static int unet_backward_residual(hicarw_unet *n, const float *coef, const float
     unet_step_kernel<<<g, 256, 0, s>>>(n->O0, coef, n->tz, nvox);
     interior_stencil_kernel<<<g, 256, 0, s>>>(coef, n->tz, n->tr, nx, ny, nz, 0);
     unet_resid_kernel<<<UNET_RED, 256, 0, s>>>(n->tr, rhat, nvox, n->red);
-    unet_loss_final_kernel<<<1, 1, 0, s>>>(n->red, UNET_RED, nvox, w, n->scal);
+    unet_loss_final_kernel<<<1, 32, 0, s>>>(n->red, UNET_RED, nvox, w, n->scal);
     interior_stencil_kernel<<<g, 256, 0, s>>>(coef, n->tr, n->tz, nx, ny, nz, 1);
     unet_resid_grad_kernel<<<g, 256, 0, s>>>(n->tz, coef, 2.0f * w / (float)nvox, nx, ny, nz, n->dO, adim(n, 0, 16));
     count_launch(6);
@@ -492,21 +483,19 @@ static VecView plain_view(const Dims &d) { return VecView{d.mx, (long long)d.mx 
 static void unet_rms(hicarw_unet *n, const Dims &d, const double *r, VecView vw, const SolveState *gate, cudaStream_t s)
 {
     const long long nvox = (long long)d.nx * d.ny * d.nz;
-    {
-        ProfScope ps_("unet_rms", (double)nvox * 8.0, s);
-        unet_sumsq_kernel<<<UNET_RED, 256, 0, s>>>(r, vw, d, n->red, gate);
-    }
-    unet_rms_kernel<<<1, 1, 0, s>>>(n->red, UNET_RED, nvox, n->scal, gate);
-    count_launch(2);
+    ProfScope ps_("unet_rms", (double)nvox * 8.0, s);
+    unet_rms_kernel<<<RMS_BLOCKS, 256, 0, s>>>(r, vw, d, n->red, n->ticket, n->scal, gate);
+    count_launch(1);
 }
 
 // z = M(r) for solver vectors in the given view
+// have_rms: n->scal holds the rms of r already
 static int unet_apply(hicarw_unet *n, const OpCtx &c, const double *r, double *z, VecView vw, const SolveState *gate,
-                      cudaStream_t s)
+                      cudaStream_t s, bool have_rms = false)
 {
     const Dims &d = c.d;
     const long long nvox = (long long)d.nx * d.ny * d.nz;
-    unet_rms(n, d, r, vw, gate, s);
+    if (!have_rms) unet_rms(n, d, r, vw, gate, s);
     {
         ProfScope ps_("unet_features", (double)nvox * (8.0 + 32.0), s);
         feat_r_kernel<<<ew_grid(nvox), 256, 0, s>>>(r, vw, d, n->X0, adim(n, 0, 16), n->scal, gate);
@@ -529,10 +518,14 @@ int unet_prepare_operator(hicarw_unet *n, const OpCtx &c, cudaStream_t s)
     return 0;
 }
 
-int unet_precond(hicarw_unet *n, const OpCtx &c, const double *in, double *out, const SolveState *gate, cudaStream_t s)
+int unet_precond(hicarw_unet *n, const OpCtx &c, const double *in, double *out, const SolveState *gate, cudaStream_t s,
+                 bool have_rms)
 {
-    return unet_apply(n, c, in, out, padded_view(c.d), gate, s);
+    return unet_apply(n, c, in, out, padded_view(c.d), gate, s, have_rms);
 }
+
+// where the rms of the next input is expected (rms, 1 / rms)
+float *unet_scale(hicarw_unet *n) { return n->scal; }
 
 bool unet_matches(const hicarw_unet *n, const Dims &d)
 {
@@ -607,7 +600,8 @@ extern "C" int hicarw_unet_create(int nx, int ny, int nz, unsigned long long see
     T(&n->U0, 0, 16);
     T(&n->D0, 0, 16);
     A((void **)&n->O0, (size_t)nx * ny * nz * 4);
-    A((void **)&n->red, UNET_RED * 8);
+    A((void **)&n->red, RMS_BLOCKS * 8);
+    A((void **)&n->ticket, 4);
     A((void **)&n->scal, 16);
     A((void **)&n->err, 4);
     if (bad) {

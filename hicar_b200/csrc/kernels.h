@@ -84,6 +84,14 @@ void launch_spmv_sigma(const OpCtx &c, const V *phat, V *v, const V *rhat, Solve
 template <typename V>
 void launch_spmv_dot5(const OpCtx &c, const V *shat, V *t, const V *s, const V *rhat, SolveState *stt, double *hist,
                       const RedBuf &rb, cudaStream_t st);
+// composite learned preconditioner: res = r - A z with its interior rms in scal; au = A u and
+// theta = <res, au> / <au, au>; z += theta u and (w not null) w = A z
+void launch_mgl_residual(const OpCtx &c, const double *z, const double *r, double *res, float *scal, SolveState *stt,
+                         const RedBuf &rb, const SolveState *gate, cudaStream_t st);
+void launch_mgl_step(const OpCtx &c, const double *u, const double *res, double *au, SolveState *stt, const RedBuf &rb,
+                     const SolveState *gate, cudaStream_t st);
+void launch_mgl_add(const Dims &d, const double *u, double *z, const SolveState *stt, const double *r, const double *res,
+                    const double *au, double *w, const SolveState *gate, cudaStream_t st);
 template <typename V, typename X>
 void launch_update_xrp(const Dims &d, X *x, const V *phat, const V *shat, V *r, const V *s, const V *t, V *p,
                        const V *v, const SolveState *stt, cudaStream_t st);

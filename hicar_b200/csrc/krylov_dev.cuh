@@ -280,8 +280,8 @@ namespace hw {
 // columns i = 0 and i = mx - 1 (a scalar row, done by the strip's first lane
 // and by the lane of the last group).  Work items (j, strip, level chunk) are
 // ordered j fastest, so that warps running at the same time share the x rows
-// j +- 1 through L2.  f4(o, y[4]) receives a group's four values at the
-// offset of its first element, f1(o, y) a scalar row.
+// j +- 1 through L2.  f4(o, y[4], interior) receives a group's four values at the
+// offset of its first element, f1(o, y, interior) a scalar row.
 constexpr int M4_KC = 16;
 
 __device__ __forceinline__ void ld4v(const float *__restrict__ p, float (&o)[4])
@@ -330,26 +330,26 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
         const long long oc = (long long)j * PL + XO;                // column i = 0 at k = 0
         const bool first = live && g == 0, lastg = live && g == G - 1;
         const int nv = RAG && lastg ? d.nx - 4 * (G - 1) : 4; // interior columns of the group
-        auto put = [&](long long o, const double (&y)[4]) {
-            if (!RAG || nv == 4) f4(o, y);
+        auto put = [&](long long o, const double (&y)[4], bool in) {
+            if (!RAG || nv == 4) f4(o, y, in);
             else {
 #pragma unroll
                 for (int e = 0; e < 3; e++)
-                    if (e < nv) f1(o + e, y[e]);
+                    if (e < nv) f1(o + e, y[e], in);
             }
         };
         // lateral columns i = 0 and i = mx - 1: identity rows
         if (first)
-            for (int k = k0; k <= k1; k++) f1(oc + k * P, (double)x[oc + k * P]);
+            for (int k = k0; k <= k1; k++) f1(oc + k * P, (double)x[oc + k * P], false);
         if (lastg)
-            for (int k = k0; k <= k1; k++) f1(oc + (d.mx - 1) + k * P, (double)x[oc + (d.mx - 1) + k * P]);
+            for (int k = k0; k <= k1; k++) f1(oc + (d.mx - 1) + k * P, (double)x[oc + (d.mx - 1) + k * P], false);
         if (j == 0 || j == d.my - 1) { // lateral j rows: identity (warp-uniform)
             if (live)
                 for (int k = k0; k <= k1; k++) {
                     V xv[4];
                     ld4v(x + ob + k * P, xv);
                     const double y[4] = {(double)xv[0], (double)xv[1], (double)xv[2], (double)xv[3]};
-                    put(ob + k * P, y);
+                    put(ob + k * P, y, false);
                 }
             continue;
         }
@@ -429,7 +429,7 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
                         y[e] = v;
                     }
                 }
-                put(o, y);
+                put(o, y, interior);
             }
 #pragma unroll
             for (int e = 0; e < 4; e++) {

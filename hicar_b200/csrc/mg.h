@@ -48,7 +48,7 @@ void mg_free(Mg &mg);
 int mg_refresh(Mg &mg, cudaStream_t s); // after a change of omega, cscale or wmask: 1 when the cycle's launches changed
 long long mg_tma_posts(); // post-smoother launches enqueued through the tensor-copy kernel
 template <typename V>
-void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStream_t s);
+void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStream_t s, bool steps = false);
 // one bounded mbarrier wait that nothing completes, limit_ns long; sets *err on time-out
 void mg_wait_probe(int *err, uint64_t limit_ns, cudaStream_t s);
 template <typename V>
