@@ -22,10 +22,17 @@
 // Weight gradient: dW_tap[CIN x COUT] = sum over cells of X(v + tap)^T dY(v):
 // the reduction runs over cells (the MMA's K), both operands MN-major straight
 // from the same line images (8 cells x 8 channels = one 128-byte core matrix).
-// Rows of one M=128 operand are 16 consecutive (line, channel group) blocks at
-// the fixed 2080-byte line stride, so one descriptor covers several taps; the
-// three x-shifts are three accumulators.  Each persistent CTA accumulates all of
-// its tiles in TMEM and adds its partial sums to the FP32 gradient at the end.
+// A tile is TJ lines of dY (N = TJ cout) and the 3 (TJ + 2) input lines around
+// them: rows of one M=128 operand are 16 consecutive (level, line, channel group)
+// blocks at the fixed 2080-byte line stride, so one descriptor covers many taps;
+// the three x-shifts are separate accumulators.  Of the line pairs in a product
+// those within one line of each other are kept.  Each persistent CTA accumulates
+// all of its tiles in TMEM, sums its pairs in shared memory and adds them to the
+// FP32 gradient with 16-byte atomics.
+// What bounds it: reading the A operand (4 KB an MMA), so several dY lines share
+// it (16 MMAs per 128-cell line of 16 channels instead of 48), and the atomics of
+// 148 CTAs.  128x128x32 (and its halves), a launch: 16 -> 16 97 -> 53 us, 32 -> 32
+// 107 -> 58 us, 16 -> 32 95 -> 56 us, 32 -> 16 91 -> 53 us.
 #include <cuda_bf16.h>
 #include <limits.h>
 #include <stdio.h>
@@ -332,35 +339,36 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
 template <int CIN, int COUT>
 struct WgCfg {
     static constexpr int GI = CIN / 8, GO = COUT / 8;
-    static constexpr int NB = 9 * GI;          // (line, channel group) blocks of one x-shift
-    static constexpr int NMC = (NB + 15) / 16; // M = 128 row chunks
-    static constexpr int XR = NMC * 16 * LG;   // input lines + slack read by the last chunk
-    static constexpr int YR = GO * YG;
+    static constexpr int TJ = CIN == 16 ? (COUT == 16 ? 3 : 2) : COUT == 16 ? 2 : 1; // dY lines of a tile (tensor memory)
+    static constexpr int NL = TJ + 2;            // input lines in j
+    static constexpr int NB = 3 * NL * GI;       // (level, line, channel group) blocks of one x-shift
+    static constexpr int NMC = (NB + 15) / 16;   // M = 128 row chunks
+    static constexpr int N = TJ * COUT;
+    static constexpr int XR = NMC * 16 * LG;     // input lines + slack read by the last chunk
+    static constexpr int YR = TJ * GO * YG;
     static constexpr int STAGE = XR + YR;
-    static constexpr int NACC = 3 * NMC;
-    static constexpr int NEED = NACC * COUT;
+    static constexpr int NEED = 3 * NMC * N;
     static constexpr int NCOL = NEED <= 32 ? 32 : NEED <= 64 ? 64 : NEED <= 128 ? 128 : NEED <= 256 ? 256 : 512;
     static constexpr int SMEM = 2 * STAGE + 64;
     static_assert(NEED <= 512, "tensor memory columns");
     static_assert(SMEM <= 232448, "shared memory");
+    static_assert(27 * CIN * COUT * 4 <= 2 * STAGE, "the CTA's sums fit where the stages were");
 };
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
 {
     using C = WgCfg<CIN, COUT>;
+    constexpr int TJ = C::TJ, NL = C::NL;
     extern __shared__ __align__(128) uint8_t sm[];
-    uint8_t *stg0 = sm, *stg1 = sm + C::STAGE;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + 2 * C::STAGE);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 3);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + 2 * C::STAGE); // copies of stage 0, 1; MMAs of stage 0, 1
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 4);
     const int tid = threadIdx.x, warp = tid >> 5;
     const ActDims dx = a.dx, dy = a.ddy;
-    const int ntx = (dx.nx + TILE - 1) / TILE;
-    const int ntiles = ntx * dx.nz * dx.ny;
+    const int ntx = (dx.nx + TILE - 1) / TILE, njb = (dx.ny + TJ - 1) / TJ;
+    const int ntiles = ntx * dx.nz * njb;
     if (tid == 0) {
-        tc::mbar_init(&bars[0], 1);
-        tc::mbar_init(&bars[1], 1);
-        tc::mbar_init(&bars[2], 1);
+        for (int q = 0; q < 4; q++) tc::mbar_init(&bars[q], 1);
         tc::mbar_fence_init();
     }
     if (warp == 0) tc::tmem_alloc(tslot, C::NCOL);
@@ -371,29 +379,29 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
     const char *xb = reinterpret_cast<const char *>(a.x);
     const char *yb = reinterpret_cast<const char *>(a.dy);
 
-    // called by all lanes of warp 0 (see the forward kernel)
+    // called by all lanes of warp 0.  Lines past the last block's end: the zero
+    // halo lines, so that the products of a short block's missing lines are zero.
     auto issue = [&](int tile, int s) {
-        const int tx = tile % ntx, r = tile / ntx, k = r % dx.nz, j = r / dx.nz;
+        const int tx = tile % ntx, r = tile / ntx, k = r % dx.nz, j0 = r / dx.nz * TJ;
         const int lane = tid & 31;
-        uint8_t *dst = s ? stg1 : stg0;
-        if (lane == 0) tc::mbar_expect_tx(&bars[s], 9 * C::GI * LG + C::YR);
+        uint8_t *dst = sm + s * C::STAGE;
+        if (lane == 0) tc::mbar_expect_tx(&bars[s], C::NB * LG + C::YR);
         __syncwarp();
-        for (int q = lane; q < 9 * C::GI + C::GO; q += 32) {
-            if (q < 9 * C::GI) {
-                const int sl = q / C::GI, g = q % C::GI;
-                const long long L = (long long)(j + sl / 3) * (dx.nz + 2) + (k + sl % 3);
-                tc::bulk_g2s(dst + (sl * C::GI + g) * LG, xb + ((L * C::GI + g) * dx.PX + (long long)tx * TILE) * 16,
-                             LG, &bars[s]);
+        for (int q = lane; q < C::NB + TJ * C::GO; q += 32) {
+            if (q < C::NB) {
+                const int g = q % C::GI, l = q / C::GI % NL, kl = q / (C::GI * NL);
+                const long long L = (long long)min(j0 + l, dx.ny + 1) * (dx.nz + 2) + (k + kl);
+                tc::bulk_g2s(dst + q * LG, xb + ((L * C::GI + g) * dx.PX + (long long)tx * TILE) * 16, LG, &bars[s]);
             } else {
-                const int g = q - 9 * C::GI;
-                const long long L0 = (long long)(j + 1) * (dy.nz + 2) + (k + 1);
-                tc::bulk_g2s(dst + C::XR + g * YG, yb + ((L0 * C::GO + g) * dy.PX + (long long)tx * TILE + 1) * 16,
-                             YG, &bars[s]);
+                const int p = q - C::NB, g = p % C::GO, o = p / C::GO;
+                const long long L = (long long)(min(j0 + o, dy.ny) + 1) * (dy.nz + 2) + (k + 1);
+                tc::bulk_g2s(dst + C::XR + p * YG, yb + ((L * C::GO + g) * dy.PX + (long long)tx * TILE + 1) * 16, YG,
+                             &bars[s]);
             }
         }
     };
 
-    constexpr uint32_t IDESC = tc::idesc_bf16(128, COUT, 1, 1);
+    constexpr uint32_t IDESC = tc::idesc_bf16(128, C::N, 1, 1);
     float db[COUT];
 #pragma unroll
     for (int c = 0; c < COUT; c++) db[c] = 0.0f;
@@ -402,10 +410,9 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
     if (warp == 0 && tile < ntiles) issue(tile, 0);
     for (; tile < ntiles; tile += gridDim.x, it++) {
         const int s = it & 1;
-        if (warp == 0 && tile + (int)gridDim.x < ntiles) issue(tile + gridDim.x, s ^ 1);
         const bool got = tc::mbar_wait(&bars[s], (it >> 1) & 1);
         if (!__syncthreads_and(got)) { ok = false; break; }
-        const uint8_t *st = s ? stg1 : stg0;
+        const uint8_t *st = sm + s * C::STAGE;
         if (tid == 0) {
             tc::fence_after();
             const uint64_t a0 = tc::sdesc(tc::smem_u32(st), 128, LG);
@@ -414,7 +421,7 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
             for (int dil = 0; dil < 3; dil++)
 #pragma unroll
                 for (int mc = 0; mc < C::NMC; mc++) {
-                    const uint32_t d = tmem + (uint32_t)((dil * C::NMC + mc) * COUT);
+                    const uint32_t d = tmem + (uint32_t)((dil * C::NMC + mc) * C::N);
 #pragma unroll
                     for (int kc = 0; kc < TILE / 16; kc++) {
                         const uint64_t ad = a0 + (uint64_t)((mc * 16 * LG + dil * 16 + kc * 256) >> 4);
@@ -422,39 +429,74 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
                         tc::mma_bf16(d, ad, bd, IDESC, (it > 0 || kc > 0) ? 1u : 0u);
                     }
                 }
-            tc::mma_commit(&bars[2]);
+            tc::mma_commit(&bars[2 + s]);
         }
-        // bias gradient: this thread's cell row of dy
+        // bias gradient: this thread's cell of the dy lines
 #pragma unroll
-        for (int g = 0; g < C::GO; g++) {
+        for (int p = 0; p < TJ * C::GO; p++) {
             float f[8];
-            unpack8(*reinterpret_cast<const uint4 *>(st + C::XR + g * YG + tid * 16), f);
+            unpack8(*reinterpret_cast<const uint4 *>(st + C::XR + p * YG + tid * 16), f);
 #pragma unroll
-            for (int e = 0; e < 8; e++) db[g * 8 + e] += f[e];
+            for (int e = 0; e < 8; e++) db[p % C::GO * 8 + e] += f[e];
         }
-        const bool done = tc::mbar_wait(&bars[2], it & 1);
-        if (!__syncthreads_and(done)) { ok = false; break; }
-        tc::fence_before();
-        __syncthreads();
+        // the other stage's MMAs (the tile before) end while these run: the next tile's copies into it
+        if (it > 0) {
+            const bool done = tc::mbar_wait(&bars[2 + (s ^ 1)], ((it - 1) >> 1) & 1);
+            if (!__syncthreads_and(done)) { ok = false; break; }
+        }
+        if (warp == 0 && tile + (int)gridDim.x < ntiles) issue(tile + gridDim.x, s ^ 1);
+    }
+    if (ok && it > 0) {
+        const bool done = tc::mbar_wait(&bars[2 + ((it - 1) & 1)], ((it - 1) >> 1) & 1);
+        ok = __syncthreads_and(done) != 0;
     }
     if (ok && it > 0) {
         tc::fence_after();
-        for (int dil = 0; dil < 3; dil++)
-            for (int mc = 0; mc < C::NMC; mc++)
+        // the products (input line l) x (dy line o) with l - o = dj + 1 belong to the tap dj: summed over o in
+        // shared memory, one o at a time (each sum is then touched by one thread), then added to the gradient
+        float *sum = reinterpret_cast<float *>(sm);
 #pragma unroll
-                for (int q = 0; q < COUT / 16; q++) {
-                    float v[16];
-                    tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) +
-                                      (uint32_t)((dil * C::NMC + mc) * COUT + q * 16),
-                                  v);
-                    const int b = mc * 16 + tid / 8;
-                    if (b < C::NB) {
-                        const int sl = b / C::GI, g = b % C::GI, ci = g * 8 + (tid & 7), t = sl * 3 + dil;
-                        float *dst = a.dw + ((long long)t * CIN + ci) * COUT + q * 16;
+        for (int o = 0; o < TJ; o++) {
+            for (int dil = 0; dil < 3; dil++)
+                for (int mc = 0; mc < C::NMC; mc++)
 #pragma unroll
-                        for (int e = 0; e < 16; e++) atomicAdd(dst + e, v[e]);
+                    for (int q = 0; q < COUT / 16; q++) {
+                        float v[16];
+                        tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) +
+                                          (uint32_t)((dil * C::NMC + mc) * C::N + o * COUT + q * 16),
+                                      v);
+                        const int b = mc * 16 + tid / 8, g = b % C::GI, l = b / C::GI % NL, kl = b / (C::GI * NL);
+                        if (b < C::NB && l >= o && l <= o + 2) {
+                            const int t = (l - o) * 9 + kl * 3 + dil;
+                            float4 *dst = reinterpret_cast<float4 *>(sum + (t * CIN + g * 8 + (tid & 7)) * COUT + q * 16);
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                float4 x = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+                                if (o > 0) {
+                                    const float4 y = dst[e];
+                                    x = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+                                }
+                                dst[e] = x;
+                            }
+                        }
                     }
-                }
+            __syncthreads();
+        }
+        // CTAs start at different places, so that they do not queue for the same addresses
+        constexpr int Q = 27 * CIN * COUT / 4;
+        const int q0 = (int)((long long)Q * blockIdx.x / gridDim.x);
+        const bool vec = ((uintptr_t)a.dw & 15) == 0;
+        for (int p = tid; p < Q; p += 128) {
+            const int q = q0 + p < Q ? q0 + p : q0 + p - Q;
+            const float4 x = reinterpret_cast<const float4 *>(sum)[q];
+            if (vec) atomicAdd(reinterpret_cast<float4 *>(a.dw) + q, x);
+            else {
+                atomicAdd(a.dw + 4 * q, x.x);
+                atomicAdd(a.dw + 4 * q + 1, x.y);
+                atomicAdd(a.dw + 4 * q + 2, x.z);
+                atomicAdd(a.dw + 4 * q + 3, x.w);
+            }
+        }
 #pragma unroll
         for (int c = 0; c < COUT; c++) {
             float x = db[c];
@@ -464,8 +506,8 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
     }
     if (!ok && tid == 0) {
         atomicExch(a.err, 1);
-        tc::mbar_wait(&bars[0], 0, 100000000ull);
-        tc::mbar_wait(&bars[1], 0, 100000000ull);
+        // bounded waits for the copies and MMAs this CTA may still have in flight
+        for (int q = 0; q < 4; q++) tc::mbar_wait(&bars[q], (uint32_t)((q & 1) == (it & 1) ? it >> 1 : (it - 1) >> 1) & 1, 100000000ull);
     }
     tc::fence_before();
     __syncthreads();
@@ -582,7 +624,8 @@ static int launch_wgrad(const WgradArgs &a, cudaStream_t s)
             return -1;
         attr = true;
     }
-    const long long ntiles = (long long)((a.dx.nx + TILE - 1) / TILE) * a.dx.nz * a.dx.ny;
+    const long long ntiles = (long long)((a.dx.nx + TILE - 1) / TILE) * a.dx.nz * ((a.dx.ny + C::TJ - 1) / C::TJ);
+    if (ntiles > INT_MAX) return -2;
     const int grid = (int)(ntiles < sm_count() ? ntiles : sm_count()); // 1 CTA per SM (TMEM / smem)
     if (grid <= 0) return 0;
     char name[32];

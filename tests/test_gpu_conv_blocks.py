@@ -33,3 +33,32 @@ def test_blocks_against_fp64(lib, cin, cout, nx, ny, nz):
     o = out.float()
     o[1:-1, 1:-1, :, 1:nx + 1] = 0
     assert not bool(o.any())
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 16)])
+@pytest.mark.parametrize("nx,ny,nz", [(1, 1, 1), (128, 2, 1), (129, 3, 2), (40, 4, 5), (20, 331, 3)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_weight_gradient_blocks_against_fp64(lib, cin, cout, nx, ny, nz, shift):
+    """dY lines in ones, twos or threes with a remainder, added to what the gradient
+    holds, also where it is not 16-byte aligned (shift); 1e-4 of the largest
+    value, as in the kernel's other test."""
+    import ctypes as C
+    from hicar_b200 import _capi, learned as L
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    g = torch.Generator().manual_seed(3 * nx + ny + nz)
+    bf = lambda t: t.to(torch.bfloat16).double()  # noqa: E731
+    x, dy = bf(torch.randn((cin, ny, nz, nx), generator=g)), bf(torch.randn((cout, ny, nz, nx), generator=g))
+    wt = torch.zeros((cout, cin, 3, 3, 3), dtype=torch.float64, requires_grad=True)
+    (F.conv3d(x[None], wt, padding=1)[0] * dy).sum().backward()
+    ref = wt.grad.permute(2, 3, 4, 1, 0).reshape(27, cin, cout)
+    buf = torch.ones(27 * cin * cout + 4, device="cuda")
+    dw, db = buf[shift:shift + 27 * cin * cout], torch.zeros(cout, device="cuda")
+    xa, ya = L.to_act(x), L.to_act(dy)
+    rc = _capi.load().hicarw_nn_conv3_wgrad(cin, cout, nx, ny, nz, C.c_void_p(xa.data_ptr()), C.c_void_p(ya.data_ptr()),
+                                            C.c_void_p(dw.data_ptr()), C.c_void_p(db.data_ptr()), None)
+    assert rc == 0
+    got = dw.double().cpu().reshape(27, cin, cout) - 1.0
+    assert float((got - ref).abs().max()) <= 1e-4 * max(float(ref.abs().max()), 1.0)
+    rb = dy.sum((1, 2, 3))
+    assert float((db.double().cpu() - rb).abs().max()) <= 1e-4 * float(rb.abs().max().clamp(min=1.0))
