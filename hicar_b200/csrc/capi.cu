@@ -1570,7 +1570,15 @@ extern "C" int hicarw_calc_alpha(hicarw_handle *h, const float *froude, float *a
     api_entry();
     if (!h || !froude || !alpha || halo < 0 || 2 * halo >= h->d.nx || 2 * halo >= h->d.ny || device_only(mem_kind))
         return HICARW_ERR_ARG;
-    launch_calc_alpha(h->d, froude, alpha, halo, (cudaStream_t)stream);
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc;
+    float *out = alpha; // edge cells read other cells' Froude numbers: not over their own input
+    if (froude == alpha) {
+        if ((rc = ensure_work(h)) != 0) return rc;
+        out = h->swork;
+    }
+    launch_calc_alpha(h->d, froude, out, halo, s);
+    if (out != alpha) CK(cudaMemcpyAsync(alpha, out, n_cell(h->d) * 4, cudaMemcpyDeviceToDevice, s));
     CK(cudaGetLastError());
     return HICARW_OK;
 }
@@ -1783,10 +1791,12 @@ extern "C" int hicarw_smooth_alpha(hicarw_handle *h, float *alpha, int window, i
     int rc;
     if ((rc = ensure_work(h)) != 0) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    float *in = alpha, *out = h->swork;
     for (int p = 0; p < nsmooths; p++) {
-        CK(cudaMemcpyAsync(h->swork, alpha, n_cell(h->d) * 4, cudaMemcpyDeviceToDevice, s));
-        launch_smooth_xy(h->d, h->swork, alpha, window, s);
+        launch_smooth_xy(h->d, in, out, window, s);
+        std::swap(in, out);
     }
+    if (in != alpha) CK(cudaMemcpyAsync(alpha, in, n_cell(h->d) * 4, cudaMemcpyDeviceToDevice, s));
     CK(cudaGetLastError());
     return HICARW_OK;
 }

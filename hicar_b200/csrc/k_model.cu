@@ -687,22 +687,32 @@ __global__ void w_real_kernel(Dims d, Metrics m, const float *__restrict__ u, co
     w_real[cidx(d, i, k, j)] = w_real_at(d, m, u, v, w_grid, i, k, j);
 }
 
-// calc_idealized_wgrid (wind.F90:940-998): one thread per column
+// calc_idealized_wgrid (wind.F90:940-998): one thread per WG_LEVELS levels of a
+// column, each computing the level above its last one again, so that the grid
+// has a few threads per column instead of one (256x256 columns left half of the
+// chip idle).
+constexpr int WG_LEVELS = 8;
 __global__ void idealized_wgrid_kernel(Dims d, Metrics m, const float *__restrict__ u, const float *__restrict__ v,
                                        const float *__restrict__ w_real_field, float *__restrict__ w)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    int j = blockIdx.y + 1;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.z + 1, k0 = blockIdx.y * WG_LEVELS + 1;
     if (i > d.nx) return;
-    float cur = w_real_field[cidx(d, i, 1, j)] - w_real_at(d, m, u, v, nullptr, i, 1, j);
-    for (int k = 1; k <= d.nz - 1; k++) {
-        const long long c = cidx(d, i, k, j), cp = cidx(d, i, k + 1, j);
+    float cur = w_real_field[cidx(d, i, k0, j)] - w_real_at(d, m, u, v, nullptr, i, k0, j);
+#pragma unroll
+    for (int q = 0; q < WG_LEVELS; q++) {
+        const int k = k0 + q;
+        if (k > d.nz) break;
+        const long long c = cidx(d, i, k, j);
+        if (k == d.nz) {
+            w[c] = 0.0f;
+            break;
+        }
+        const long long cp = cidx(d, i, k + 1, j);
         const float nxt = w_real_field[cp] - w_real_at(d, m, u, v, nullptr, i, k + 1, j);
         float wk = (cur * m.adz[cp] + nxt * m.adz[c]) / (m.adz[c] + m.adz[cp]);
         w[c] = wk / m.jw[c];
         cur = nxt;
     }
-    w[cidx(d, i, d.nz, j)] = 0.0f;
 }
 
 // calc_w (wind.F90:201-248): upward integration of the horizontal divergence per column
@@ -753,30 +763,39 @@ __device__ __forceinline__ float dry_stability(float th_top, float th_bot, float
     return STAB_GRAVITY * (th_top - th_bot) / ((z_top - z_bot) * (th_top + th_bot) / 2.0f);
 }
 
-__global__ void update_stability_kernel(Dims d, const float *__restrict__ u, const float *__restrict__ v,
-                                        const float *__restrict__ z, const float *__restrict__ theta,
-                                        const float *__restrict__ fterr, int nsect, int froude_mode,
-                                        float *__restrict__ froude, float *__restrict__ blk_ri)
+// A CTA takes STAB_X columns; its first row of threads finds each column's bulk
+// Richardson number, then all rows share the levels.  (One thread per column
+// walked all levels before, five dependent loads each.)
+constexpr int STAB_X = 32, STAB_Y = 8;
+__global__ void __launch_bounds__(STAB_X *STAB_Y) update_stability_kernel(
+    Dims d, const float *__restrict__ u, const float *__restrict__ v, const float *__restrict__ z,
+    const float *__restrict__ theta, const float *__restrict__ fterr, int nsect, int froude_mode,
+    float *__restrict__ froude, float *__restrict__ blk_ri)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
-    if (i > d.nx) return;
+    __shared__ float s_ri[STAB_X];
+    const int i = blockIdx.x * STAB_X + threadIdx.x + 1, j = blockIdx.y + 1;
     const long long ncell = (long long)d.nx * d.ny * d.nz;
-    int rk = d.nz; // Ri_k_max (:1444-1454)
-    for (int k = 2; k <= d.nz; k++)
-        if (z[cidx(d, i, k, j)] - z[cidx(d, i, 1, j)] > 100.0f) {
-            rk = max(2, k - 1);
-            break;
-        }
-    const float us = (u[uidx(d, i, 5, j)] + u[uidx(d, i + 1, 5, j)]) / 2.0f; // u_shear(:, kms, :) (:1462-1465)
-    const float vs = (v[cidx(d, i, 5, j)] + v[cidx(d, i, 5, j + 1)]) / 2.0f;
-    const float th_b = theta[cidx(d, i, 1, j)], th_t = theta[cidx(d, i, rk, j)];
-    const float z_b = z[cidx(d, i, 1, j)], z_t = z[cidx(d, i, rk, j)];
-    // calc_Ri of the column's bulk stability (:1482-1495)
-    const float stab = dry_stability(th_t, th_b, z_t, z_b, false, 0.0f);
-    const float dz = z_t - z_b, a = us / dz, b = vs / dz;
-    const float den = a * a + b * b;
-    const float ri = den == 0.0f ? 10.0f : stab / den;
-    for (int k = 1; k <= d.nz; k++) {
+    if (threadIdx.y == 0 && i <= d.nx) {
+        int rk = d.nz; // Ri_k_max (:1444-1454)
+        const float z_b = z[cidx(d, i, 1, j)];
+        for (int k = 2; k <= d.nz; k++)
+            if (z[cidx(d, i, k, j)] - z_b > 100.0f) {
+                rk = max(2, k - 1);
+                break;
+            }
+        const float us = (u[uidx(d, i, 5, j)] + u[uidx(d, i + 1, 5, j)]) / 2.0f; // u_shear(:, kms, :) (:1462-1465)
+        const float vs = (v[cidx(d, i, 5, j)] + v[cidx(d, i, 5, j + 1)]) / 2.0f;
+        const float z_t = z[cidx(d, i, rk, j)];
+        // calc_Ri of the column's bulk stability (:1482-1495)
+        const float stab = dry_stability(theta[cidx(d, i, rk, j)], theta[cidx(d, i, 1, j)], z_t, z_b, false, 0.0f);
+        const float dz = z_t - z_b, a = us / dz, b = vs / dz;
+        const float den = a * a + b * b;
+        s_ri[threadIdx.x] = den == 0.0f ? 10.0f : stab / den;
+    }
+    __syncthreads();
+    if (i > d.nx) return;
+    const float ri = s_ri[threadIdx.x], th_b = theta[cidx(d, i, 1, j)];
+    for (int k = threadIdx.y + 1; k <= d.nz; k += STAB_Y) {
         const long long o = cidx(d, i, k, j);
         blk_ri[o] = k < d.nz ? ri : 10.0f;
         float fr = 0.1f;
@@ -803,46 +822,29 @@ void launch_update_stability(const Dims &d, const float *u, const float *v, cons
                              const float *fterr, int nsect, int froude_mode, float *froude, float *blk_ri,
                              cudaStream_t st)
 {
-    dim3 b(128), g((d.nx + 127) / 128, d.ny);
+    dim3 b(STAB_X, STAB_Y), g((d.nx + STAB_X - 1) / STAB_X, d.ny);
     update_stability_kernel<<<g, b, 0, st>>>(d, u, v, z, theta, fterr, nsect, froude_mode, froude, blk_ri);
     count_launch(1);
 }
 
-// calc_alpha (wind.F90:1102-1173), elementwise part; (1/Fr)**4 as (t*t)*(t*t)
-__global__ void calc_alpha_kernel(Dims d, const float *__restrict__ froude, float *__restrict__ alpha)
+// calc_alpha (wind.F90:1102-1173); (1/Fr)**4 as (t*t)*(t*t).  The reference then
+// copies the h outermost rows and columns, south, west, north, east, from the
+// first ones inside; together these take every cell's value from the nearest cell
+// of the tile, which is where its Froude number is read here.
+__global__ void calc_alpha_kernel(Dims d, const float *__restrict__ froude, float *__restrict__ alpha, int h)
 {
-    const long long n = (long long)d.nx * d.nz * d.ny;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const float t = 1.0f / froude[q];
-        const float t2 = t * t;
-        const float p = t2 * t2;
-        const float mx = p > 0.00001f ? p : 0.00001f;
-        float a = 1.0f - 0.5f * mx * (sqrtf(1.0f + 4.0f / mx) - 1.0f);
-        a = sqrtf(a > 0.00001f ? a : 0.00001f);
-        a = a > 0.2f ? a : 0.2f;
-        a = a < 2.0f ? a : 2.0f;
-        const int k = (int)((q / d.nx) % d.nz) + 1;
-        alpha[q] = k == d.nz ? 0.2f : a;
-    }
-}
-
-// one of the four boundary copies of calc_alpha: side 0 south (j <= h), 1 west
-// (i <= h), 2 north (j > ny - h), 3 east (i > nx - h); whole columns
-__global__ void alpha_edge_kernel(Dims d, float *__restrict__ alpha, int h, int side)
-{
-    const int ni = (side == 1 || side == 3) ? h : d.nx, nj = (side == 0 || side == 2) ? h : d.ny;
-    const long long n = (long long)ni * nj * d.nz;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        int a = (int)(q % ni) + 1;
-        long long r = q / ni;
-        int k = (int)(r % d.nz) + 1, b = (int)(r / d.nz) + 1;
-        int i = a, j = b, is = a, js = b;
-        if (side == 0) js = h + 1;
-        else if (side == 1) is = h + 1;
-        else if (side == 2) { j = d.ny - h + b; js = d.ny - h; }
-        else { i = d.nx - h + a; is = d.nx - h; }
-        alpha[cidx(d, i, k, j)] = alpha[cidx(d, is, k, js)];
-    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, j = blockIdx.z + 1;
+    if (i > d.nx) return;
+    const int is = min(max(i, h + 1), d.nx - h), js = min(max(j, h + 1), d.ny - h);
+    const float t = 1.0f / froude[cidx(d, is, k, js)];
+    const float t2 = t * t;
+    const float p = t2 * t2;
+    const float mx = p > 0.00001f ? p : 0.00001f;
+    float a = 1.0f - 0.5f * mx * (sqrtf(1.0f + 4.0f / mx) - 1.0f);
+    a = sqrtf(a > 0.00001f ? a : 0.00001f);
+    a = a > 0.2f ? a : 0.2f;
+    a = a < 2.0f ? a : 2.0f;
+    alpha[cidx(d, i, k, j)] = k == d.nz ? 0.2f : a;
 }
 
 // one pass of smooth_array_3d, ydim = 3 (array_utilities.F90:322-397): x-y box
@@ -876,7 +878,7 @@ void launch_w_real(const Dims &d, const Metrics &m, const float *u, const float 
 void launch_idealized_wgrid(const Dims &d, const Metrics &m, const float *u, const float *v, const float *w_real_field,
                             float *w, cudaStream_t st)
 {
-    dim3 b(64), g((d.nx + 63) / 64, d.ny);
+    dim3 b(128), g((d.nx + 127) / 128, (d.nz + WG_LEVELS - 1) / WG_LEVELS, d.ny);
     idealized_wgrid_kernel<<<g, b, 0, st>>>(d, m, u, v, w_real_field, w);
     count_launch(1);
 }
@@ -891,14 +893,8 @@ void launch_calc_w(const Dims &d, const Metrics &m, const float *div, const floa
 
 void launch_calc_alpha(const Dims &d, const float *froude, float *alpha, int halo, cudaStream_t st)
 {
-    const long long n = (long long)d.nx * d.nz * d.ny;
-    calc_alpha_kernel<<<(int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16), 256, 0, st>>>(d, froude, alpha);
+    calc_alpha_kernel<<<dim3((d.nx + 127) / 128, d.nz, d.ny), 128, 0, st>>>(d, froude, alpha, halo);
     count_launch(1);
-    if (halo > 0)
-        for (int side = 0; side < 4; side++) {
-            alpha_edge_kernel<<<148, 256, 0, st>>>(d, alpha, halo, side);
-            count_launch(1);
-        }
 }
 
 void launch_smooth_xy(const Dims &d, const float *in, float *out, int w, cudaStream_t st)

@@ -1,0 +1,50 @@
+"""GPU tests of the per-step kernels where their tiles end: update_stability in
+columns of 32 and levels of 8, the w predictor in levels of 8, calc_alpha's edge
+cells (also over its own input), against the oracle, bit for bit."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from hicar_b200 import _capi, cases
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(5, 6, 5), (31, 5, 8), (32, 5, 9), (33, 7, 17), (129, 6, 16)])
+@pytest.mark.parametrize("halo", [0, 1, 2])
+def test_per_step_kernels(lib, oracle_mod, nx, ny, nz, halo):
+    from hicar_b200 import wind, wind_iterative as wi
+    from hicar_b200.domain import DeviceDomain
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    wi.finalize_iter_winds()
+    case = cases.build_case(nx, ny, nz, seed=nx + halo, n_hills=3)
+    dom = DeviceDomain.from_case(case, "cuda")
+    wi.init_iter_winds(dom, wi.WindOptions())
+    s = oracle_mod.OracleSolver(case.domain)
+    rng = np.random.default_rng(nz)
+    new = lambda: torch.empty((ny, nz, nx), device="cuda")  # noqa: E731
+    # the w predictor
+    w_real = rng.standard_normal((ny, nz, nx)).astype(np.float32)
+    wind.calc_idealized_wgrid(dom, torch.from_numpy(w_real).cuda())
+    np.testing.assert_array_equal(dom.w_dqdt.cpu().numpy(), s.idealized_wgrid(case.u, case.v, w_real))
+    # the bulk Richardson number (the Froude number's sector may differ within an ulp: its other test)
+    theta, ft = cases.stability_inputs(case, seed=1, nsect=4)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (case.domain.z, theta, ft)]
+    froude, ri = new(), new()
+    wind.update_stability(dom, dev[0], dev[1], froude, ri, dev[2])
+    fr_ref, ri_ref = s.update_stability(case.u, case.v, case.domain.z, theta, ft)
+    np.testing.assert_array_equal(ri.cpu().numpy(), ri_ref)
+    assert np.mean(froude.cpu().numpy() != fr_ref) < 0.01
+    # alpha, into another array and over its input
+    lib_ = _capi.load()
+    fr = torch.from_numpy(fr_ref).cuda()
+    out = new()
+    h = wi.handle(dom.nest_indx)
+    want = s.calc_alpha(fr_ref, halo)
+    for dst in (out, fr):
+        _capi.check(lib_.hicarw_calc_alpha(h, C.c_void_p(fr.data_ptr()), C.c_void_p(dst.data_ptr()), halo, 0, None), h)
+        np.testing.assert_array_equal(dst.cpu().numpy(), want)
+    wi.finalize_iter_winds()
