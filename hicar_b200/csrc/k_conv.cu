@@ -153,6 +153,58 @@ __device__ __forceinline__ void issue_taps(int nj, uint64_t a0, uint64_t b0, uin
         }
 }
 
+// Bias, skip, ReLU, mask and the stores of one cell of one output line: v its
+// sums, ex its skip (or else mask) values fetched ahead, at its act unit.
+template <int COUT>
+__device__ __forceinline__ void conv_store(const ConvArgs &a, float (&v)[COUT], const float (&bias)[COUT],
+                                           const uint4 (&ex)[COUT / 8], long long at, int i, int k, int j)
+{
+    constexpr int GO = COUT / 8;
+    const ActDims &dd = a.dout;
+#pragma unroll
+    for (int c = 0; c < COUT; c++) v[c] += bias[c];
+    if (a.skip) {
+#pragma unroll
+        for (int g = 0; g < GO; g++) {
+            float f[8];
+            unpack8(ex[g], f);
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[g * 8 + e] += f[e];
+        }
+    }
+    if (a.relu) {
+#pragma unroll
+        for (int c = 0; c < COUT; c++) v[c] = fmaxf(v[c], 0.0f);
+    }
+    if (a.mask) {
+#pragma unroll
+        for (int g = 0; g < GO; g++) {
+            float f[8];
+            unpack8(a.skip ? a.mask[at + g * dd.PX] : ex[g], f);
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[g * 8 + e] = f[e] > 0.0f ? v[g * 8 + e] : 0.0f;
+        }
+    }
+    if (a.out) {
+#pragma unroll
+        for (int g = 0; g < GO; g++) a.out[at + g * dd.PX] = pack8(v + g * 8);
+    }
+    if (a.out0) a.out0[((long long)j * dd.nz + k) * dd.nx + i] = v[0];
+}
+
+// The skip (or else mask) values of a thread's cell in the output lines of a block's level.
+template <int COUT, int TJ>
+__device__ __forceinline__ void conv_extra(const ConvArgs &a, uint4 (&ex)[TJ][COUT / 8], long long base, long long js, int nj,
+                                           bool live)
+{
+    const uint4 *extra = a.skip ? a.skip : a.mask;
+#pragma unroll
+    for (int o = 0; o < TJ; o++)
+#pragma unroll
+        for (int g = 0; g < COUT / 8; g++)
+            ex[o][g] = extra && live && o < nj ? extra[base + o * js + g * a.dout.PX] : make_uint4(0, 0, 0, 0);
+}
+
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, ConvSplit p)
 {
@@ -268,13 +320,8 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
                 const int slot = n % SLOTS;
                 const long long base = act_unit(dd, i, k, b.j0, 0);
                 // what the epilogue reads, fetched while the accumulators are still being summed
-                const uint4 *extra = a.skip ? a.skip : a.mask;
                 uint4 ex[TJ][C::GO];
-#pragma unroll
-                for (int o = 0; o < TJ; o++)
-#pragma unroll
-                    for (int g = 0; g < C::GO; g++)
-                        ex[o][g] = extra && live && o < b.nj ? extra[base + o * js + g * dd.PX] : make_uint4(0, 0, 0, 0);
+                conv_extra<COUT, TJ>(a, ex, base, js, b.nj, live);
                 wait(&tfull[slot], n / SLOTS);
                 tc::fence_after();
 #pragma unroll
@@ -291,42 +338,196 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
                     for (int q = 0; q < COUT / 16; q++) {
                         tc::tmem_ld_wait(r[q]);
 #pragma unroll
-                        for (int e = 0; e < 16; e++) v[q * 16 + e] = __uint_as_float(r[q][e]) + bias[q * 16 + e];
+                        for (int e = 0; e < 16; e++) v[q * 16 + e] = __uint_as_float(r[q][e]);
                     }
                     if (o == b.nj - 1) { // the slot is read out
                         tc::fence_before();
                         __syncwarp();
                         if (lane == 0) tc::mbar_arrive(&tempty[slot]);
                     }
-                    if (!live) continue;
-                    const long long at = base + o * js;
-                    if (a.skip) {
+                    if (live) conv_store<COUT>(a, v, bias, ex[o], base + o * js, i, k, b.j0 + o);
+                }
+            }
+        }
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, C::NCOL);
+}
+
+// ---------------------------------------------------------------------------
+// The same for 16 output channels with all nine taps (dj, dk) merged in N: the
+// accumulators of an output line's three levels in the making lie side by side
+// (column (3 o + slot) 16, slots rotating with the level), so one MMA of a line
+// and x-shift feeds up to three output lines times three levels (N = 144): three
+// MMAs per line and level instead of nine, for an operand read that costs as much
+// each.  The rotation of the slots is in the weights (three images).  Every
+// product accumulates; a slot is read out and zeroed before the next level's
+// products, which the CTA next to it on the SM covers.  Levels outside the block
+// that a block's first and last input levels also feed are zeroed without being
+// stored.
+// 16 -> 16 at 512x512x48 (B200): 0.342 -> 0.183 ms (0.68 of measured HBM, 0.57 of
+// measured BF16); 32 -> 16 at 256x256x48: 0.093 ms.
+// ---------------------------------------------------------------------------
+template <int CIN>
+struct Fwd9Cfg {
+    static constexpr int COUT = 16, GI = CIN / 8, GO = 2, TJ = 4, NL = TJ + 2;
+    static constexpr int ROWS = 9 * COUT;                  // weight rows of one (rotation, x-shift, channel group)
+    static constexpr int WB = 9 * GI * ROWS * 16;          // three images
+    static constexpr int STAGE = NL * GI * SG;
+    static constexpr int NCOL = 256, NS = 2;
+    static constexpr int SMEM = up128(WB) + NS * STAGE + 256;
+    static constexpr int PER_SM = SMEM <= 113 * 1024 ? 2 : 1;
+    static_assert(SMEM <= 232448, "shared memory");
+};
+
+template <int CIN>
+__global__ void __launch_bounds__(CONV_THREADS) conv3_fwd9_kernel(ConvArgs a, ConvSplit p)
+{
+    using C = Fwd9Cfg<CIN>;
+    constexpr int NS = C::NS, TJ = C::TJ, COUT = C::COUT;
+    if (conv_gated(a.gate)) return;
+    extern __shared__ __align__(128) uint8_t sm[];
+    uint8_t *wsm = sm, *stg = sm + up128(C::WB) + SGO;
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + up128(C::WB) + NS * C::STAGE + 128), *empty = full + NS,
+             *summed = empty + NS, *drained = summed + 1;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(drained + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const ActDims di = a.din, dd = a.dout;
+    if (tid == 0) {
+        for (int q = 0; q < NS; q++) {
+            tc::mbar_init(&full[q], 1);
+            tc::mbar_init(&empty[q], 1);
+        }
+        tc::mbar_init(summed, 1);
+        tc::mbar_init(drained, 4);
+        tc::mbar_fence_init();
+    }
+    if (warp == 0) tc::tmem_alloc(tslot, C::NCOL);
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = *tslot;
+    bool ok = true;
+    auto wait = [&](uint64_t *bar, int use) { // the use-th completion (from 0); on time-out: no more waits
+        if (ok && !tc::mbar_wait(bar, use & 1)) {
+            if (lane == 0) atomicExch(a.err, 1);
+            ok = false;
+        }
+    };
+
+    if (warp == 4) { // ---- copies (as conv3_fwd_kernel) ----
+        const char *inb = reinterpret_cast<const char *>(a.in);
+        int it = 0;
+        for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+            const ConvBlock b = conv_block(di, p, TJ, u);
+            for (int kk = b.lo; kk <= b.hi; kk++, it++) {
+                const int s = it % NS;
+                if (it >= NS) wait(&empty[s], it / NS - 1);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const int n = (b.nj + 2) * C::GI;
+                if (lane == 0) tc::mbar_expect_tx(&full[s], n * LG + (it == 0 ? C::WB : 0));
+                __syncwarp();
+                if (it == 0 && lane == 31) tc::bulk_g2s(wsm, a.w, C::WB, &full[s]);
+                for (int q = lane; q < n; q += 32) {
+                    const int l = q / C::GI, g = q % C::GI; // input line j0 - 1 + l, level kk
+                    const long long L = (long long)(b.j0 + l) * (di.nz + 2) + (kk + 1);
+                    tc::bulk_g2s(stg + s * C::STAGE + q * SG, inb + ((L * C::GI + g) * di.PX + (long long)b.tx * TILE) * 16,
+                                 LG, &full[s]);
+                }
+            }
+            if (!ok) break;
+        }
+        // nothing in flight at the end: the last stages landed and were read
+        for (int q = it > NS ? it - NS : 0; q < it; q++) {
+            if (!tc::mbar_wait(&full[q % NS], (q / NS) & 1) && lane == 0) atomicExch(a.err, 1);
+            wait(&empty[q % NS], q / NS);
+        }
+    } else if (warp == 5) { // ---- MMAs, one thread ----
+        if (lane == 0) {
+            const uint64_t b0 = tc::sdesc(tc::smem_u32(wsm), C::ROWS * 16, 128);
+            int it = 0; // input level; its rotation (the slot of output level kk - 1) is it % 3
+            for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+                const ConvBlock b = conv_block(di, p, TJ, u);
+                for (int kk = b.lo; kk <= b.hi; kk++, it++) {
+                    const int s = it % NS;
+                    wait(&full[s], it / NS);
+                    wait(drained, it); // completion 0: all columns zeroed at the start
+                    if (!ok) continue;
+                    tc::fence_after();
+                    const uint64_t a0 = tc::sdesc(tc::smem_u32(stg + s * C::STAGE), SG, 128);
+                    const uint64_t br = b0 + (uint64_t)((it % 3 * 3 * C::GI * C::ROWS * 16) >> 4);
 #pragma unroll
-                        for (int g = 0; g < C::GO; g++) {
-                            float f[8];
-                            unpack8(ex[o][g], f);
+                    for (int dil = 0; dil < 3; dil++)
 #pragma unroll
-                            for (int e = 0; e < 8; e++) v[g * 8 + e] += f[e];
+                        for (int c = 0; c < C::GI / 2; c++) {
+                            const uint64_t bt = br + (uint64_t)(((dil * C::GI + 2 * c) * C::ROWS * 16) >> 4);
+#pragma unroll
+                            for (int l = 0; l < C::NL; l++) {
+                                if (l >= b.nj + 2) break;
+                                const int o0 = l - 2 > 0 ? l - 2 : 0, o1 = min(l, b.nj - 1);
+                                const uint64_t ad = a0 + (uint64_t)(((l * C::GI + 2 * c) * SG + dil * 16) >> 4);
+                                tc::mma_bf16(tmem + o0 * 3 * COUT, ad, bt + (uint64_t)((o0 - (l - 2)) * 3 * COUT),
+                                             tc::idesc_bf16(128, 0, 0, 0) | ((uint32_t)((o1 - o0 + 1) * 3 * COUT / 8) << 17), 1u);
+                            }
                         }
-                    }
-                    if (a.relu) {
+                    tc::mma_commit(&empty[s]);
+                    tc::mma_commit(summed);
+                }
+            }
+        }
+        __syncwarp();
+    } else { // ---- epilogue: thread = cell of the x-tile ----
+        const uint32_t lanes = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll
-                        for (int c = 0; c < COUT; c++) v[c] = fmaxf(v[c], 0.0f);
-                    }
-                    if (a.mask) {
+        for (int q = 0; q < 3 * TJ; q++) tc::tmem_zero16(lanes + q * COUT);
+        tc::tmem_st_wait();
+        auto hand_back = [&]() {
+            tc::fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(drained);
+        };
+        hand_back();
+        float bias[COUT];
 #pragma unroll
-                        for (int g = 0; g < C::GO; g++) {
-                            float f[8];
-                            unpack8(a.skip ? a.mask[at + g * dd.PX] : ex[o][g], f);
+        for (int c = 0; c < COUT; c++) bias[c] = a.bias ? __ldg(a.bias + c) : 0.0f;
+        const long long js = (long long)(dd.nz + 2) * C::GO * dd.PX; // from one line to the next in j
+        int it = 0;
+        for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+            const ConvBlock b = conv_block(di, p, TJ, u);
+            const int i = b.tx * TILE + tid;
+            const bool live = i < di.nx;
+            for (int kk = b.lo; kk <= b.hi; kk++, it++) {
+                // output level kk - 1 is complete after input level kk, and after the last one also kk, if it is the grid's last
+                const int last = kk == b.hi ? 3 : 1;
+                uint4 ex[TJ][C::GO];
+                conv_extra<COUT, TJ>(a, ex, act_unit(dd, i, kk - 1, b.j0, 0), js, b.nj, live && kk > b.k0);
+                wait(summed, it);
+                tc::fence_after();
+                for (int t = 0; t < last; t++) {
+                    const int k = kk - 1 + t, slot = (it + t) % 3;
+                    const bool store = k >= b.k0 && k < b.k0 + b.nk;
+                    uint32_t r[TJ][16];
 #pragma unroll
-                            for (int e = 0; e < 8; e++) v[g * 8 + e] = f[e] > 0.0f ? v[g * 8 + e] : 0.0f;
-                        }
-                    }
-                    if (a.out) {
+                    for (int o = 0; o < TJ; o++) tc::tmem_ld16_async(lanes + (uint32_t)((3 * o + slot) * COUT), r[o]);
 #pragma unroll
-                        for (int g = 0; g < C::GO; g++) a.out[at + g * dd.PX] = pack8(v + g * 8);
+                    for (int o = 0; o < TJ; o++) tc::tmem_ld_wait(r[o]);
+#pragma unroll
+                    for (int o = 0; o < TJ; o++) tc::tmem_zero16(lanes + (uint32_t)((3 * o + slot) * COUT));
+                    tc::tmem_st_wait();
+                    if (t == last - 1) hand_back();
+                    if (!store || !live) continue;
+                    const long long base = act_unit(dd, i, k, b.j0, 0);
+                    if (t > 0) conv_extra<COUT, TJ>(a, ex, base, js, b.nj, live);
+#pragma unroll
+                    for (int o = 0; o < TJ; o++) {
+                        if (o >= b.nj) break;
+                        float v[COUT];
+#pragma unroll
+                        for (int e = 0; e < 16; e++) v[e] = __uint_as_float(r[o][e]);
+                        conv_store<COUT>(a, v, bias, ex[o], base + o * js, i, k, b.j0 + o);
                     }
-                    if (a.out0) a.out0[((long long)(b.j0 + o) * dd.nz + k) * dd.nx + i] = v[0];
                 }
             }
         }
@@ -515,45 +716,59 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// Element (t, ci, co) of the weight image of a conv cin -> cout: per (dk, di) and
-// group of 8 input channels a column of 3 cout rows of 16 bytes, the taps dj = 1,
-// 0, -1 below one another (the order of the output lines that they feed).
-__device__ __forceinline__ int wimage_at(int t, int ci, int co, int cin, int cout)
+// Weight image of a conv cin -> cout, BF16.  cout = 32: per (dk, di) and group of 8
+// input channels a column of 3 cout rows of 16 bytes, the taps dj = 1, 0, -1 below
+// one another (the order of the output lines that they feed).  cout = 16: per
+// rotation, di and group a column of 9 cout rows, the taps dj = 1, 0, -1 and below
+// each the three slots, slot s of rotation q holding the tap dk that feeds it.
+static bool merged9(int cout) { return cout == 16; }
+
+__device__ __forceinline__ void wimage_put(__nv_bfloat16 *img, int t, int ci, int co, int cin, int cout, int nine, float w)
 {
-    return ((t % 9 * (cin / 8) + ci / 8) * 3 * cout + (2 - t / 9) * cout + co) * 8 + (ci & 7);
+    const __nv_bfloat16 v = __float2bfloat16_rn(w);
+    const int tj = t / 9, tk = t / 3 % 3, ti = t % 3, g = ci / 8, e = ci & 7, G = cin / 8;
+    if (!nine) {
+        img[(((tk * 3 + ti) * G + g) * 3 * cout + (2 - tj) * cout + co) * 8 + e] = v;
+        return;
+    }
+    for (int q = 0; q < 3; q++) { // rotation q: slot q holds output level kk - 1 (tap dk = 1), the next ones kk and kk + 1
+        const int slot = (q + 2 - tk) % 3;
+        img[(((q * 3 + ti) * G + g) * 9 * cout + ((2 - tj) * 3 + slot) * cout + co) * 8 + e] = v;
+    }
 }
 
-__global__ void conv_pack_fwd_kernel(const float *__restrict__ W, int cin, int cout, __nv_bfloat16 *__restrict__ img)
+__global__ void conv_pack_fwd_kernel(const float *__restrict__ W, int cin, int cout, int nine, __nv_bfloat16 *__restrict__ img)
 {
     const int n = 27 * cin * cout;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         const int t = q / (cin * cout), r = q % (cin * cout), ci = r / cout, co = r % cout;
-        img[wimage_at(t, ci, co, cin, cout)] = __float2bfloat16_rn(W[q]);
+        wimage_put(img, t, ci, co, cin, cout, nine, W[q]);
     }
 }
 
 // image of the conv cout -> cin whose output is the data gradient:
 // W'[t'][ci' = co][co' = ci] = W[26 - t'][ci][co]
-__global__ void conv_pack_bwd_kernel(const float *__restrict__ W, int cin, int cout, __nv_bfloat16 *__restrict__ img)
+__global__ void conv_pack_bwd_kernel(const float *__restrict__ W, int cin, int cout, int nine, __nv_bfloat16 *__restrict__ img)
 {
     const int n = 27 * cin * cout;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         const int t = q / (cin * cout), r = q % (cin * cout), ci = r / cout, co = r % cout;
-        img[wimage_at(26 - t, co, ci, cout, cin)] = __float2bfloat16_rn(W[q]);
+        wimage_put(img, 26 - t, co, ci, cout, cin, nine, W[q]);
     }
 }
 
-size_t conv_wimage_bytes(int cin, int cout) { return (size_t)27 * cin * cout * 2; }
+// room for the image of either direction
+size_t conv_wimage_bytes(int cin, int cout) { return (size_t)27 * cin * cout * 2 * 3; }
 
 void conv_pack_fwd(const float *W, int cin, int cout, uint4 *img, cudaStream_t s)
 {
-    conv_pack_fwd_kernel<<<(27 * cin * cout + 255) / 256, 256, 0, s>>>(W, cin, cout, (__nv_bfloat16 *)img);
+    conv_pack_fwd_kernel<<<(27 * cin * cout + 255) / 256, 256, 0, s>>>(W, cin, cout, merged9(cout), (__nv_bfloat16 *)img);
     count_launch(1);
 }
 
 void conv_pack_bwd(const float *W, int cin, int cout, uint4 *img, cudaStream_t s)
 {
-    conv_pack_bwd_kernel<<<(27 * cin * cout + 255) / 256, 256, 0, s>>>(W, cin, cout, (__nv_bfloat16 *)img);
+    conv_pack_bwd_kernel<<<(27 * cin * cout + 255) / 256, 256, 0, s>>>(W, cin, cout, merged9(cin), (__nv_bfloat16 *)img);
     count_launch(1);
 }
 
@@ -590,25 +805,19 @@ static ConvSplit conv_split(const ActDims &d, int TJ, int resident)
 
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
-template <int CI, int CO>
-static int launch_fwd(const ConvArgs &a, cudaStream_t s)
+template <typename C>
+static int launch_fwd(void (*kernel)(ConvArgs, ConvSplit), int ci, int co, const ConvArgs &a, cudaStream_t s)
 {
-    using C = FwdCfg<CI, CO>;
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(conv3_fwd_kernel<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
-            cudaSuccess)
-            return -1;
-        attr = true;
-    }
+    static const bool attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) == cudaSuccess;
+    if (!attr) return -1;
     const ConvSplit p = conv_split(a.din, C::TJ, sm_count() * C::PER_SM);
     const int grid = std::min(p.units, sm_count() * C::PER_SM);
     if (grid <= 0) return 0;
     char name[32];
-    snprintf(name, sizeof(name), "conv3_fwd_%dx%d", CI, CO);
+    snprintf(name, sizeof(name), "conv3_fwd_%dx%d", ci, co);
     const double cells = (double)a.din.nx * a.din.ny * a.din.nz;
-    ProfScope ps_(name, cells * 2.0 * (CI + CO), s);
-    conv3_fwd_kernel<CI, CO><<<grid, CONV_THREADS, C::SMEM, s>>>(a, p);
+    ProfScope ps_(name, cells * 2.0 * (ci + co), s);
+    kernel<<<grid, CONV_THREADS, C::SMEM, s>>>(a, p);
     count_launch(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -648,10 +857,10 @@ int conv3_fwd(int cin, int cout, const ConvArgs &a, cudaStream_t s)
         a.din.nz != a.dout.nz || !a.in || !a.w || !a.err)
         return -2;
     if (!aligned16(a.in) || !aligned16(a.w) || !aligned16(a.out) || !aligned16(a.skip) || !aligned16(a.mask)) return -2;
-    if (cin == 16 && cout == 16) return launch_fwd<16, 16>(a, s);
-    if (cin == 16 && cout == 32) return launch_fwd<16, 32>(a, s);
-    if (cin == 32 && cout == 32) return launch_fwd<32, 32>(a, s);
-    if (cin == 32 && cout == 16) return launch_fwd<32, 16>(a, s);
+    if (cin == 16 && cout == 16) return launch_fwd<Fwd9Cfg<16>>(conv3_fwd9_kernel<16>, 16, 16, a, s);
+    if (cin == 16 && cout == 32) return launch_fwd<FwdCfg<16, 32>>(conv3_fwd_kernel<16, 32>, 16, 32, a, s);
+    if (cin == 32 && cout == 32) return launch_fwd<FwdCfg<32, 32>>(conv3_fwd_kernel<32, 32>, 32, 32, a, s);
+    if (cin == 32 && cout == 16) return launch_fwd<Fwd9Cfg<32>>(conv3_fwd9_kernel<32>, 32, 16, a, s);
     return -2;
 }
 

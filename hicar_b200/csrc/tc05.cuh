@@ -84,6 +84,16 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16])
                  : "memory");
 }
 
+// Zeros into 16 consecutive columns of this thread's TMEM lane; tmem_st_wait before they count.
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+                 "{%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+                 "r"(0u)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 // 16 consecutive FP32 columns of this thread's TMEM lane (warp w reads lanes 32(w%4)..+31).
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
 {
