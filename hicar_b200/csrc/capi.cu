@@ -460,8 +460,10 @@ static void enqueue_precond(hicarw_handle *h, const VT *in, VT *out, int sweeps,
 {
     OpCtx c = opctx(h);
     VT *Dinv = V<VT>(h, V_DINV), *pres = V<VT>(h, V_PRES);
-    launch_precond_scale<VT>(h->d, in, out, Dinv, gate, set_halt, s);
-    for (int sw = 2; sw <= sweeps; sw++) {
+    int done = 1;
+    if (sweeps >= 2 && launch_precond2<VT>(c, in, out, Dinv, gate, set_halt, s)) done = 2;
+    else launch_precond_scale<VT>(h->d, in, out, Dinv, gate, set_halt, s);
+    for (int sw = done + 1; sw <= sweeps; sw++) {
         launch_spmv<VT>(c, out, pres, gate, s);
         launch_rich<VT>(h->d, in, out, pres, Dinv, gate, s);
     }
@@ -474,8 +476,7 @@ static void enqueue_iteration(hicarw_handle *h, XT *x, int sweeps, cudaStream_t 
     RedBuf rb{h->partials, h->red_blocks};
     SolveState *st = h->st;
     VT *r = V<VT>(h, V_R), *rhat = V<VT>(h, V_RHAT), *p = V<VT>(h, V_P), *phat = V<VT>(h, V_PHAT), *v = V<VT>(h, V_V),
-       *sv = V<VT>(h, V_S), *shat = V<VT>(h, V_SHAT), *t = V<VT>(h, V_T), *Dinv = V<VT>(h, V_DINV),
-       *pres = V<VT>(h, V_PRES);
+       *sv = V<VT>(h, V_S), *shat = V<VT>(h, V_SHAT), *t = V<VT>(h, V_T), *Dinv = V<VT>(h, V_DINV);
     if (h->use_mg) { // multigrid-preconditioned BiCGStab (same recurrences, M = V-cycle)
         launch_iteration_begin(st, s);
         mg_apply<VT>(h->mg, p, phat, st, s);
@@ -488,11 +489,10 @@ static void enqueue_iteration(hicarw_handle *h, XT *x, int sweeps, cudaStream_t 
     }
     enqueue_precond<VT>(h, p, phat, sweeps, st, 1, s);                 // :649
     launch_spmv_sigma<VT>(c, phat, v, rhat, st, rb, s);                // :657-688
-    launch_s_precond<VT>(h->d, r, v, sv, shat, Dinv, st, s);           // :690 + sweep 1 of :695
-    for (int sw = 2; sw <= sweeps; sw++) {
-        launch_spmv<VT>(c, shat, pres, st, s);
-        launch_rich<VT>(h->d, sv, shat, pres, Dinv, st, s);
-    }
+    if (sweeps >= 2) {
+        launch_s_update<VT>(h->d, r, v, sv, st, s);                    // :690
+        enqueue_precond<VT>(h, sv, shat, sweeps, st, 0, s);            // :695
+    } else launch_s_precond<VT>(h->d, r, v, sv, shat, Dinv, st, s);    // :690 + :695
     launch_spmv_dot5<VT>(c, shat, t, sv, rhat, st, h->hist, rb, s);    // :703-750
     launch_update_xrp<VT, XT>(h->d, x, phat, shat, r, sv, t, p, v, st, s); // :755-783
 }

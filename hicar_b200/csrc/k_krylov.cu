@@ -680,6 +680,50 @@ void launch_precond_scale(const Dims &d, const V *in, V *out, const V *Dinv, Sol
     count_launch(1);
 }
 
+// Both sweeps of the two-sweep preconditioner in one pass (probed operator):
+// z = D^-1 in, out = z + D^-1 (in - A z), z formed as the marching rows load it.
+// Bound by HBM: 84 bytes per row (FP64) for 140 of the scaling, the operator and
+// the Richardson step one after another.  512x512x48, FP64:
+// 273 us for 351.
+template <typename V, bool RAG>
+__global__ void __launch_bounds__(ROWT, M4_CTAS_DOT5) precond2_m4_kernel(OpCtx c, const V *__restrict__ in,
+                                                                         V *__restrict__ out, const V *__restrict__ Dinv,
+                                                                         SolveState *gate, int set_halt)
+{
+    if (gated(gate)) {
+        if (set_halt && blockIdx.x == 0 && threadIdx.x == 0) gate->halt = 1;
+        return;
+    }
+    auto step = [](V b, V d, double y) {
+        const V z = d * b;
+        return z + d * (b - (V)y);
+    };
+    march4_rows_of<V, RAG>(
+        c, RowsOfProduct<V>{in, Dinv},
+        [&](long long o, const double (&y)[4], bool) {
+            V b[4], d[4];
+            ld4v(in + o, b);
+            ld4v(Dinv + o, d);
+#pragma unroll
+            for (int e = 0; e < 4; e++) b[e] = step(b[e], d[e], y[e]);
+            st4v(out + o, b);
+        },
+        [&](long long o, double y, bool) { out[o] = step(in[o], Dinv[o], y); });
+}
+
+template <typename V>
+bool launch_precond2(const OpCtx &c, const V *in, V *out, const V *Dinv, SolveState *gate, int set_halt, cudaStream_t st)
+{
+    if (spmv_kind(c) != SPMV_MARCH4) return false;
+    ProfScope ps_("precond2", coef_bytes(c.d) + rows(c.d) * 3.0 * sizeof(V), st);
+    OpCtx m = c;
+    auto *kernel = c.d.nx % 4 ? precond2_m4_kernel<V, true> : precond2_m4_kernel<V, false>;
+    const int g = march4_grid(kernel, m, 148 * 16);
+    kernel<<<g, ROWT, 0, st>>>(m, in, out, Dinv, gate, set_halt);
+    count_launch(1);
+    return true;
+}
+
 // s = r - alpha v (:690) fused with s^ = D^-1 s (sweep 1 of the second apply)
 template <typename V>
 __global__ void s_precond_kernel(long long n, const V *__restrict__ r, const V *__restrict__ v, V *__restrict__ s,
@@ -981,6 +1025,7 @@ void launch_convert(long long n, const A *in, B *out, cudaStream_t st)
 // ---- explicit instantiations ----
 #define INST_V(V)                                                                                                      \
     template void launch_spmv<V>(const OpCtx &, const V *, V *, const SolveState *, cudaStream_t);                    \
+    template bool launch_precond2<V>(const OpCtx &, const V *, V *, const V *, SolveState *, int, cudaStream_t);      \
     template void launch_precond_scale<V>(const Dims &, const V *, V *, const V *, SolveState *, int, cudaStream_t);  \
     template void launch_s_precond<V>(const Dims &, const V *, const V *, V *, V *, const V *, SolveState *,          \
                                       cudaStream_t);                                                                   \

@@ -69,6 +69,9 @@ void launch_spmv(const OpCtx &c, const V *x, V *y, const SolveState *gate, cudaS
 template <typename V>
 void launch_precond_scale(const Dims &d, const V *in, V *out, const V *Dinv, SolveState *gate, int set_halt,
                           cudaStream_t st);
+// sweeps 1 and 2 of the preconditioner in one pass; false (nothing launched) where the operator has no such form
+template <typename V>
+bool launch_precond2(const OpCtx &c, const V *in, V *out, const V *Dinv, SolveState *gate, int set_halt, cudaStream_t st);
 template <typename V>
 void launch_s_precond(const Dims &d, const V *r, const V *v, V *s, V *shat, const V *Dinv, SolveState *stt,
                       cudaStream_t st);

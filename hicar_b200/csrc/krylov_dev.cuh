@@ -311,8 +311,30 @@ __host__ __device__ __forceinline__ long long march4_items(const Dims &d, int KC
     return (long long)d.my * nsx * nkc;
 }
 
-template <typename V, bool RAG, typename F4, typename F1>
-__device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict__ x, F4 &&f4, F1 &&f1)
+// The vector as the marching rows read it: an array, or the product of two
+// (rounded to V as if it had been stored).
+template <typename V>
+struct RowsOf {
+    const V *__restrict__ x;
+    __device__ __forceinline__ void ld4(long long o, V (&v)[4]) const { ld4v(x + o, v); }
+    __device__ __forceinline__ V at(long long o) const { return x[o]; }
+};
+template <typename V>
+struct RowsOfProduct {
+    const V *__restrict__ x, *__restrict__ d;
+    __device__ __forceinline__ void ld4(long long o, V (&v)[4]) const
+    {
+        V e[4];
+        ld4v(x + o, v);
+        ld4v(d + o, e);
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = e[q] * v[q];
+    }
+    __device__ __forceinline__ V at(long long o) const { return d[o] * x[o]; }
+};
+
+template <typename V, bool RAG, typename LX, typename F4, typename F1>
+__device__ __forceinline__ void march4_rows_of(const OpCtx &c, const LX x, F4 &&f4, F1 &&f1)
 {
     const Dims &d = c.d;
     const int KC = march4_kc(c), G = (d.nx + 3) / 4, nsx = (G + 31) / 32, nkc = (d.mz + KC - 1) / KC;
@@ -340,14 +362,14 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
         };
         // lateral columns i = 0 and i = mx - 1: identity rows
         if (first)
-            for (int k = k0; k <= k1; k++) f1(oc + k * P, (double)x[oc + k * P], false);
+            for (int k = k0; k <= k1; k++) f1(oc + k * P, (double)x.at(oc + k * P), false);
         if (lastg)
-            for (int k = k0; k <= k1; k++) f1(oc + (d.mx - 1) + k * P, (double)x[oc + (d.mx - 1) + k * P], false);
+            for (int k = k0; k <= k1; k++) f1(oc + (d.mx - 1) + k * P, (double)x.at(oc + (d.mx - 1) + k * P), false);
         if (j == 0 || j == d.my - 1) { // lateral j rows: identity (warp-uniform)
             if (live)
                 for (int k = k0; k <= k1; k++) {
                     V xv[4];
-                    ld4v(x + ob + k * P, xv);
+                    x.ld4(ob + k * P, xv);
                     const double y[4] = {(double)xv[0], (double)xv[1], (double)xv[2], (double)xv[3]};
                     put(ob + k * P, y, false);
                 }
@@ -358,17 +380,17 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
         V c_m[4] = {}, c_0[4] = {}, s_m[4] = {}, s_0[4] = {}, n_m[4] = {}, n_0[4] = {};
         V w_m = 0, w_0 = 0, e_m = 0, e_0 = 0;
         if (live) {
-            ld4v(x + ob + k0 * P, c_0);
-            ld4v(x + ob - PL + k0 * P, s_0);
-            ld4v(x + ob + PL + k0 * P, n_0);
+            x.ld4(ob + k0 * P, c_0);
+            x.ld4(ob - PL + k0 * P, s_0);
+            x.ld4(ob + PL + k0 * P, n_0);
             if (k0 > 0) {
-                ld4v(x + ob + (k0 - 1) * P, c_m);
-                ld4v(x + ob - PL + (k0 - 1) * P, s_m);
-                ld4v(x + ob + PL + (k0 - 1) * P, n_m);
+                x.ld4(ob + (k0 - 1) * P, c_m);
+                x.ld4(ob - PL + (k0 - 1) * P, s_m);
+                x.ld4(ob + PL + (k0 - 1) * P, n_m);
             }
         }
-        if (west) { w_0 = x[ob - 1 + k0 * P]; if (k0 > 0) w_m = x[ob - 1 + (k0 - 1) * P]; }
-        if (east) { e_0 = x[ob + 4 + k0 * P]; if (k0 > 0) e_m = x[ob + 4 + (k0 - 1) * P]; }
+        if (west) { w_0 = x.at(ob - 1 + k0 * P); if (k0 > 0) w_m = x.at(ob - 1 + (k0 - 1) * P); }
+        if (east) { e_0 = x.at(ob + 4 + k0 * P); if (k0 > 0) e_m = x.at(ob + 4 + (k0 - 1) * P); }
         for (int k = k0; k <= k1; k++) {
             const long long o = ob + k * P;
             const bool interior = k >= 1 && k <= d.nz;
@@ -376,11 +398,11 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
             V w_p = 0, e_p = 0;
             float cf[15][4];
             if (live && k + 1 < d.mz) {
-                ld4v(x + o + P, c_p);
-                ld4v(x + o - PL + P, s_p);
-                ld4v(x + o + PL + P, n_p);
-                if (west) w_p = x[o - 1 + P];
-                if (east) e_p = x[o + 4 + P];
+                x.ld4(o + P, c_p);
+                x.ld4(o - PL + P, s_p);
+                x.ld4(o + PL + P, n_p);
+                if (west) w_p = x.at(o - 1 + P);
+                if (east) e_p = x.at(o + 4 + P);
             }
             if (live && interior) {
 #pragma unroll
@@ -441,6 +463,12 @@ __device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict_
             e_m = e_0; e_0 = e_p;
         }
     }
+}
+
+template <typename V, bool RAG, typename F4, typename F1>
+__device__ __forceinline__ void march4_rows(const OpCtx &c, const V *__restrict__ x, F4 &&f4, F1 &&f1)
+{
+    march4_rows_of<V, RAG>(c, RowsOf<V>{x}, f4, f1);
 }
 
 }  // namespace hw
