@@ -1027,11 +1027,14 @@ __global__ void __launch_bounds__(MG_THREADS, 3) restrict_pre_kernel(
 // waited first (B200): 64x64x20 1.81 -> 1.62 ms, 181x157x33 8.24 -> 7.29 ms,
 // 512x512x48 39.7 -> 37.0 ms; without the programmatic launch 1.67, 7.63, 38.7.
 // ---------------------------------------------------------------------------
-constexpr int SM_POST_U = 2;     // cells per thread loaded ahead (8 columns x 64 levels: all)
 constexpr int SM_RESTRICT_U = 3; // fine cells per thread loaded ahead (4 coarse columns x 48 levels: all)
 
-template <typename TR, typename TO, int TX, int TY, typename CT>
-__global__ void __launch_bounds__(MG_THREADS) post_small_kernel(Dims d, const CT *__restrict__ coef,
+// U: cells per thread loaded ahead, one where the tile has no more cells than the
+// CTA threads (four CTAs then fit on an SM instead of two), else two.  One on
+// every level: 64x64x20 1.62 -> 1.58 ms and 181x157x33 6.15 -> 5.92 ms a solve,
+// but 512x512x48 35.1 -> 35.6 ms, whose tiles of 8 columns x 48 levels take two.
+template <typename TR, typename TO, int TX, int TY, typename CT, int U>
+__global__ void __launch_bounds__(MG_THREADS, U == 1 ? 4 : 2) post_small_kernel(Dims d, const CT *__restrict__ coef,
                                                                 const float *__restrict__ cp,
                                                                 const float *__restrict__ minv, const TR *r,
                                                                 const float *x1, Dims dc, const float *xc, TO *out,
@@ -1048,7 +1051,7 @@ __global__ void __launch_bounds__(MG_THREADS) post_small_kernel(Dims d, const CT
         o = kidx(d, i, t / TC + 1, j);
         return t < n && i <= d.nx && j <= d.ny;
     };
-    float cv[SM_POST_U][15], vm[SM_POST_U], vp[SM_POST_U];
+    float cv[U][15], vm[U], vp[U];
     auto load = [&](int u, int t) {
         long long o;
         vm[u] = vp[u] = 0.0f;
@@ -1059,21 +1062,21 @@ __global__ void __launch_bounds__(MG_THREADS) post_small_kernel(Dims d, const CT
         }
     };
 #pragma unroll
-    for (int u = 0; u < SM_POST_U; u++) load(u, threadIdx.x + u * MG_THREADS);
+    for (int u = 0; u < U; u++) load(u, threadIdx.x + u * MG_THREADS);
     pdl_wait();
     if (gate && *(volatile const int *)&gate->stop && !gate->profile) return;
-    TR rv[SM_POST_U];
+    TR rv[U];
     auto load_r = [&](int u, int t) {
         long long o;
         rv[u] = offset(t, o) ? r[o] : (TR)0;
     };
 #pragma unroll
-    for (int u = 0; u < SM_POST_U; u++) load_r(u, threadIdx.x + u * MG_THREADS);
+    for (int u = 0; u < U; u++) load_r(u, threadIdx.x + u * MG_THREADS);
     stage_window_l2<SX, SY>(d, x1, dc, xc, i0 - 1, j0 - 1, s_x, cscale);
     __syncthreads();
-    for (int base = threadIdx.x; base < n; base += MG_THREADS * SM_POST_U) {
+    for (int base = threadIdx.x; base < n; base += MG_THREADS * U) {
 #pragma unroll
-        for (int u = 0; u < SM_POST_U; u++) {
+        for (int u = 0; u < U; u++) {
             const int t = base + u * MG_THREADS;
             if (base >= MG_THREADS) {
                 load(u, t);
@@ -1892,9 +1895,10 @@ static void post_t(const MgLevel &L, const CT *coef, const TR *r, const MgLevel 
     dim3 g((L.d.nx + TX - 1) / TX, (L.d.ny + TY - 1) / TY);
     size_t smem = ((size_t)4 * TX * TY * L.d.nz + (size_t)(TX + 2) * (TY + 2) * (L.d.nz + 2)) * sizeof(float);
     if constexpr (TX * TY <= 8) {
-        set_smem(post_small_kernel<TR, TO, TX, TY, CT>, smem);
-        launch_pdl(post_small_kernel<TR, TO, TX, TY, CT>, g, MG_THREADS, smem, s, L.d, coef, L.cp, L.minv, r, L.x1, C.d,
-                   C.x3, out, omega, cscale, gate);
+        auto *kernel = TX * TY * L.d.nz <= MG_THREADS ? post_small_kernel<TR, TO, TX, TY, CT, 1>
+                                                      : post_small_kernel<TR, TO, TX, TY, CT, 2>;
+        set_smem(kernel, smem);
+        launch_pdl(kernel, g, MG_THREADS, smem, s, L.d, coef, L.cp, L.minv, r, L.x1, C.d, C.x3, out, omega, cscale, gate);
     } else {
         set_smem(post_kernel<TR, TO, TX, TY, CT>, smem);
         post_kernel<TR, TO, TX, TY, CT><<<g, MG_THREADS, smem, s>>>(L.d, coef, L.cp, L.minv, r, L.x1, C.d, C.x3, out,
@@ -2112,10 +2116,8 @@ static void launch_restrict_pre(const MgLevel &F, const TR *r, const MgLevel &C,
             else restrict_t<TR, 8, 1, false>(F, r, C, out, omega, gate, s);
         } else if (nox) restrict_t<TR, 2, 2, true>(F, r, C, out, omega, gate, s);
         else restrict_t<TR, 2, 2, false>(F, r, C, out, omega, gate, s);
-    } else {
-        if (nox) restrict_t<TR, 16, 1, true>(F, r, C, out, omega, gate, s);
-        else restrict_t<TR, 16, 1, false>(F, r, C, out, omega, gate, s);
-    }
+    } else if (nox) restrict_t<TR, 16, 1, true>(F, r, C, out, omega, gate, s);
+    else restrict_t<TR, 16, 1, false>(F, r, C, out, omega, gate, s);
     count_launch(1);
 }
 
