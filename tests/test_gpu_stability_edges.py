@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(5, 6, 5), (31, 5, 8), (32, 5, 9), (33, 7, 17), (129, 6, 16)])
+@pytest.mark.parametrize("nx,ny,nz", [(5, 6, 5), (31, 5, 8), (32, 5, 9), (33, 17, 17), (129, 16, 16)])
 @pytest.mark.parametrize("halo", [0, 1, 2])
 def test_per_step_kernels(lib, oracle_mod, nx, ny, nz, halo):
     from hicar_b200 import wind, wind_iterative as wi
@@ -47,4 +47,9 @@ def test_per_step_kernels(lib, oracle_mod, nx, ny, nz, halo):
     for dst in (out, fr):
         _capi.check(lib_.hicarw_calc_alpha(h, C.c_void_p(fr.data_ptr()), C.c_void_p(dst.data_ptr()), halo, 0, None), h)
         np.testing.assert_array_equal(dst.cpu().numpy(), want)
+    # smoothing passes of every window kernel (marching rows in 16s, and the general one)
+    for window, passes in ((1, 1), (1, 2), (2, 3), (3, 1)):
+        a = torch.from_numpy(want).cuda()
+        _capi.check(lib_.hicarw_smooth_alpha(h, C.c_void_p(a.data_ptr()), window, passes, 0, None), h)
+        np.testing.assert_array_equal(a.cpu().numpy(), s.smooth_array(want, window, passes))
     wi.finalize_iter_winds()
