@@ -1284,10 +1284,14 @@ static int get_padded(hicarw_handle *h, const double *src, double *dst, int mem_
 
 // The q-th transfer vector of the handle.  Allocating and freeing these on every
 // call cost more than the work (an operator and a V-cycle at 384x320x40: 4.8 ms a
-// pass, 0.7 ms with them kept); they go with the handle.
+// pass, 1.3 ms with them kept); they go with the handle.  The allocation clears on
+// the default stream, which the caller's stream need not wait for: the one wait here.
 static int transfer_vector(hicarw_handle *h, int q, double **x)
 {
-    if (!h->xfer[q]) CK(dalloc((void **)&h->xfer[q], (size_t)h->d.npad * sizeof(double)));
+    if (!h->xfer[q]) {
+        CK(dalloc((void **)&h->xfer[q], (size_t)h->d.npad * sizeof(double)));
+        CK(cudaStreamSynchronize(cudaStreamLegacy));
+    }
     *x = h->xfer[q];
     return 0;
 }
@@ -1331,6 +1335,7 @@ extern "C" int hicarw_apply_precond(hicarw_handle *h, const double *x, double *y
     double *bx, *by, *bd, *bp;
     int rc;
     if ((rc = transfer_vector(h, 0, &bx)) != 0 || (rc = transfer_vector(h, 1, &by)) != 0) return rc;
+    if (sweeps > 0 && ((rc = transfer_vector(h, 2, &bd)) != 0 || (rc = transfer_vector(h, 3, &bp)) != 0)) return rc;
     rc = put_padded(h, x, bx, mem_kind, s);
     if (!rc && learned) rc = ensure_vectors(h, HICARW_KRYLOV_F64); // scratch of the composite
     if (!rc && learned && h->unet_dirty) {
@@ -1354,7 +1359,6 @@ extern "C" int hicarw_apply_precond(hicarw_handle *h, const double *x, double *y
             if (!rc && h->mg.err) CK(cudaMemcpyAsync(herr, h->mg.err, sizeof(int), cudaMemcpyDeviceToHost, s));
         }
     } else if (!rc) {
-        if ((rc = transfer_vector(h, 2, &bd)) != 0 || (rc = transfer_vector(h, 3, &bp)) != 0) return rc;
         launch_diag<double>(d, h->coef, h->dz_if, bd, h->operator_probed, s);
         OpCtx c = opctx(h);
         launch_precond_scale<double>(d, bx, by, bd, nullptr, 0, s);
