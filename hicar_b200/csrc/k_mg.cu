@@ -2218,12 +2218,13 @@ static cudaLaunchConfig_t fused_config(int cn, size_t smem, cudaStream_t s, cuda
 }
 
 // Decide at build time (outside any stream capture) whether and where the
-// coarse part is fused (HICARW_MG_FUSE=0 in the environment: never), and the
-// cluster size: 16 CTAs where the device can place such a cluster with this
-// shared memory, else 8, else no fusion.  Measured at 1024x1024x64 with W on
-// levels 2-4: fused from level 6 (16 x 16 columns) 8.63 solves/s against 8.56
-// with one launch per level; from level 5 (32 x 32) 8.30 against 8.37; one CTA
-// walking the chain from level 7 8.30.
+// step-by-step coarse part is fused (HICARW_MG_FUSE=0 in the environment: never;
+// a solve walks it only where the dense matrix does not apply), and the cluster
+// size: 16 CTAs where the device can place such a cluster with this shared
+// memory, else 8, else no fusion.  Measured at 1024x1024x64 with W on levels 2-4:
+// fused from level 6 (16 x 16 columns) 8.63 solves/s against 8.56 with one launch
+// per level; from level 5 (32 x 32) 8.30 against 8.37; one CTA walking the chain
+// from level 7 8.30.
 static void fused_setup(Mg &mg)
 {
     mg.fuse_level = 0;

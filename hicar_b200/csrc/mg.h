@@ -28,8 +28,8 @@ struct Mg {
     int use_tma = 2;     // post-smoothers of the wide levels: 2 tensor copies, recurrences on their own warp
                          // (post_tma2_kernel); 1 tensor copies, post_tma_kernel (HICARW_MG_TMA=1);
                          // 0 register-fed (HICARW_MG_TMA=0)
-    int fuse_level = 0;  // first level of the coarse part run by one thread-block cluster (0: every level its own
-                         // launches; HICARW_MG_FUSE=0 at build time)
+    int fuse_level = 0;  // first level of the step-by-step coarse part run by one thread-block cluster (0: every
+                         // level its own launches; HICARW_MG_FUSE=0 at build time)
     int cluster_n = 0;   // CTAs of that cluster
     int dense_level = 0; // level (>= 1) from which the cycle is one matrix-vector product (0: none)
     int dense_n = 0, dense_ld = 0;  // its unknowns and the matrix's row length

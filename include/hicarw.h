@@ -118,7 +118,8 @@ typedef struct hicarw_options {
     int replace_every;    /* FP32 Krylov vectors: the recurrence residual is replaced by the FP64 true
                              residual b - A x every replace_every iterations (rounded down to a multiple
                              of check_every; default 50) */
-    int check_every;      /* iterations between host reads of the device-side stop flag */
+    int check_every;      /* unit of replace_every (the loop itself runs on the device until its stop
+                             flag is set; the host reads the flag once per replace_every iterations) */
     int precond;          /* HICARW_PRECOND_* */
     int stall_iters;      /* stop a preconditioned solve whose residual has not dropped by 1% for
                              this many iterations and fall back to the reference solve (0 = off) */
@@ -233,7 +234,8 @@ int hicarw_apply_operator(hicarw_handle *h, const double *x, double *y, int mem_
  * wind_iterative.F90:1268-1315) with that many sweeps; sweeps == 0 applies one
  * multigrid V-cycle (probed operator only); sweeps < 0 applies the learned
  * preconditioner the options name (HICARW_PRECOND_LEARNED or _MG_LEARNED, with
- * the attached U-Net), else the V-cycle. */
+ * the attached U-Net), else the V-cycle (its steps one by one, without the
+ * tabulated coarse part that solves use). */
 int hicarw_apply_precond(hicarw_handle *h, const double *x, double *y, int sweeps, int mem_kind, void *stream);
 
 /* Solve A lambda = rhs for a caller-given right-hand side ((nx+2, nz+2, ny+2), FP64),
