@@ -693,14 +693,16 @@ __global__ void w_real_kernel(Dims d, Metrics m, const float *__restrict__ u, co
 // has a few threads per column instead of one (256x256 columns left half of the
 // chip idle).
 constexpr int WG_LEVELS = 8;
-__global__ void idealized_wgrid_kernel(Dims d, Metrics m, const float *__restrict__ u, const float *__restrict__ v,
-                                       const float *__restrict__ w_real_field, float *__restrict__ w)
+template <int LEVELS> // levels per thread; 0: the column
+__device__ __forceinline__ void idealized_wgrid_levels(const Dims &d, const Metrics &m, const float *u, const float *v,
+                                                       const float *w_real_field, float *w)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.z + 1, k0 = blockIdx.y * WG_LEVELS + 1;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.z + 1;
+    const int k0 = blockIdx.y * LEVELS + 1, n = LEVELS ? LEVELS : d.nz;
     if (i > d.nx) return;
     float cur = w_real_field[cidx(d, i, k0, j)] - w_real_at(d, m, u, v, nullptr, i, k0, j);
 #pragma unroll
-    for (int q = 0; q < WG_LEVELS; q++) {
+    for (int q = 0; q < n; q++) {
         const int k = k0 + q;
         if (k > d.nz) break;
         const long long c = cidx(d, i, k, j);
@@ -714,6 +716,20 @@ __global__ void idealized_wgrid_kernel(Dims d, Metrics m, const float *__restric
         w[c] = wk / m.jw[c];
         cur = nxt;
     }
+}
+
+__global__ void idealized_wgrid_kernel(Dims d, Metrics m, const float *__restrict__ u, const float *__restrict__ v,
+                                       const float *__restrict__ w_real_field, float *__restrict__ w)
+{
+    idealized_wgrid_levels<WG_LEVELS>(d, m, u, v, w_real_field, w);
+}
+
+// w over w_real: one thread per column, which reads a level before it writes the
+// one below (threads of other levels would read what it has written).
+__global__ void idealized_wgrid_inplace_kernel(Dims d, Metrics m, const float *__restrict__ u,
+                                               const float *__restrict__ v, float *w)
+{
+    idealized_wgrid_levels<0>(d, m, u, v, w, w);
 }
 
 // calc_w (wind.F90:201-248): upward integration of the horizontal divergence per column
@@ -768,10 +784,9 @@ __device__ __forceinline__ float dry_stability(float th_top, float th_bot, float
 // Richardson number, then all rows share the levels.  (One thread per column
 // walked all levels before, five dependent loads each.)
 constexpr int STAB_X = 32, STAB_Y = 8;
-__global__ void __launch_bounds__(STAB_X *STAB_Y) update_stability_kernel(
-    Dims d, const float *__restrict__ u, const float *__restrict__ v, const float *__restrict__ z,
-    const float *__restrict__ theta, const float *__restrict__ fterr, int nsect, int froude_mode,
-    float *__restrict__ froude, float *__restrict__ blk_ri)
+__device__ __forceinline__ void stability_columns(const Dims &d, const float *u, const float *v, const float *z,
+                                                  const float *theta, const float *fterr, int nsect, int froude_mode,
+                                                  float *froude, float *blk_ri)
 {
     __shared__ float s_ri[STAB_X];
     const int i = blockIdx.x * STAB_X + threadIdx.x + 1, j = blockIdx.y + 1;
@@ -796,9 +811,8 @@ __global__ void __launch_bounds__(STAB_X *STAB_Y) update_stability_kernel(
     __syncthreads();
     if (i > d.nx) return;
     const float ri = s_ri[threadIdx.x], th_b = theta[cidx(d, i, 1, j)];
-    for (int k = threadIdx.y + 1; k <= d.nz; k += STAB_Y) {
+    for (int k = threadIdx.y + 1; k <= d.nz; k += blockDim.y) {
         const long long o = cidx(d, i, k, j);
-        blk_ri[o] = k < d.nz ? ri : 10.0f;
         float fr = 0.1f;
         if (froude_mode && k < d.nz) { // (:1503-1560)
             const float um = (u[uidx(d, i, k, j)] + u[uidx(d, i + 1, k, j)]) / 2.0f;
@@ -815,16 +829,38 @@ __global__ void __launch_bounds__(STAB_X *STAB_Y) update_stability_kernel(
             const float fden = tf * bv;
             fr = fden == 0.0f ? 100.0f : ws / fden;
         }
+        blk_ri[o] = k < d.nz ? ri : 10.0f;
         froude[o] = fr;
     }
+}
+
+__global__ void __launch_bounds__(STAB_X *STAB_Y) update_stability_kernel(
+    Dims d, const float *__restrict__ u, const float *__restrict__ v, const float *__restrict__ z,
+    const float *__restrict__ theta, const float *__restrict__ fterr, int nsect, int froude_mode,
+    float *__restrict__ froude, float *__restrict__ blk_ri)
+{
+    stability_columns(d, u, v, z, theta, fterr, nsect, froude_mode, froude, blk_ri);
+}
+
+// froude or blk_ri over theta or z: launched with one row of threads, so that one
+// thread walks a column and reads a level before it writes the one below.
+__global__ void __launch_bounds__(STAB_X) update_stability_inplace_kernel(
+    Dims d, const float *__restrict__ u, const float *__restrict__ v, const float *z, const float *theta,
+    const float *__restrict__ fterr, int nsect, int froude_mode, float *froude, float *blk_ri)
+{
+    stability_columns(d, u, v, z, theta, fterr, nsect, froude_mode, froude, blk_ri);
 }
 
 void launch_update_stability(const Dims &d, const float *u, const float *v, const float *z, const float *theta,
                              const float *fterr, int nsect, int froude_mode, float *froude, float *blk_ri,
                              cudaStream_t st)
 {
-    dim3 b(STAB_X, STAB_Y), g((d.nx + STAB_X - 1) / STAB_X, d.ny);
-    update_stability_kernel<<<g, b, 0, st>>>(d, u, v, z, theta, fterr, nsect, froude_mode, froude, blk_ri);
+    const dim3 g((d.nx + STAB_X - 1) / STAB_X, d.ny);
+    if (froude == theta || froude == z || blk_ri == theta || blk_ri == z)
+        update_stability_inplace_kernel<<<g, STAB_X, 0, st>>>(d, u, v, z, theta, fterr, nsect, froude_mode, froude, blk_ri);
+    else
+        update_stability_kernel<<<g, dim3(STAB_X, STAB_Y), 0, st>>>(d, u, v, z, theta, fterr, nsect, froude_mode, froude,
+                                                                    blk_ri);
     count_launch(1);
 }
 
@@ -920,8 +956,11 @@ void launch_w_real(const Dims &d, const Metrics &m, const float *u, const float 
 void launch_idealized_wgrid(const Dims &d, const Metrics &m, const float *u, const float *v, const float *w_real_field,
                             float *w, cudaStream_t st)
 {
-    dim3 b(128), g((d.nx + 127) / 128, (d.nz + WG_LEVELS - 1) / WG_LEVELS, d.ny);
-    idealized_wgrid_kernel<<<g, b, 0, st>>>(d, m, u, v, w_real_field, w);
+    const int gx = (d.nx + 127) / 128;
+    if (w == w_real_field) idealized_wgrid_inplace_kernel<<<dim3(gx, 1, d.ny), 128, 0, st>>>(d, m, u, v, w);
+    else
+        idealized_wgrid_kernel<<<dim3(gx, (d.nz + WG_LEVELS - 1) / WG_LEVELS, d.ny), 128, 0, st>>>(d, m, u, v, w_real_field,
+                                                                                                  w);
     count_launch(1);
 }
 

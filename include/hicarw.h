@@ -369,7 +369,8 @@ long long hicarw_mg_tma_launches(void);
 int hicarw_calc_w_real(hicarw_handle *h, const float *u, const float *v, const float *w_grid, float *w_real,
                        int mem_kind, void *stream);
 /* calc_idealized_wgrid (wind.F90:940-998): the w_grid predictor w = stagger(w_real -
- * calc_w_real(u, v, 0)) / jacobian_w, zero on the top level (u, v: the dqdt winds). */
+ * calc_w_real(u, v, 0)) / jacobian_w, zero on the top level (u, v: the dqdt winds);
+ * w may be w_real. */
 int hicarw_calc_idealized_wgrid(hicarw_handle *h, const float *u, const float *v, const float *w_real, float *w,
                                 int mem_kind, void *stream);
 /* balance_uvw + calc_w (wind.F90:123-248): w from the horizontal divergence of u, v
@@ -385,7 +386,8 @@ int hicarw_balance_uvw(hicarw_handle *h, const float *u, const float *v, const f
  * froude_terrain (nx, nz, ny, nsect) with 5-degree sectors (nsect = 72 in HICAR;
  * domain%vars_4d froude_terrain).  froude is 0.1 and blk_ri 10 on the top level,
  * froude 0.1 everywhere when froude_mode == 0.  u, v are the dqdt winds, z the
- * mass-level heights, theta the potential temperature (nx, nz, ny); nz >= 5. */
+ * mass-level heights, theta the potential temperature (nx, nz, ny); nz >= 5; froude
+ * and blk_ri may be theta or z. */
 int hicarw_update_stability(hicarw_handle *h, const float *u, const float *v, const float *z, const float *theta,
                             const float *froude_terrain, int nsect, int froude_mode, float *froude, float *blk_ri,
                             int mem_kind, void *stream);

@@ -1,6 +1,6 @@
 """GPU tests of the per-step kernels where their tiles end: update_stability in
 columns of 32 and levels of 8, the w predictor in levels of 8, calc_alpha's edge
-cells (also over its own input), against the oracle, bit for bit."""
+cells (each also over its own input), against the oracle, bit for bit."""
 import ctypes as C
 
 import numpy as np
@@ -29,7 +29,11 @@ def test_per_step_kernels(lib, oracle_mod, nx, ny, nz, halo):
     # the w predictor
     w_real = rng.standard_normal((ny, nz, nx)).astype(np.float32)
     wind.calc_idealized_wgrid(dom, torch.from_numpy(w_real).cuda())
-    np.testing.assert_array_equal(dom.w_dqdt.cpu().numpy(), s.idealized_wgrid(case.u, case.v, w_real))
+    want = s.idealized_wgrid(case.u, case.v, w_real)
+    np.testing.assert_array_equal(dom.w_dqdt.cpu().numpy(), want)
+    dom.w_dqdt.copy_(torch.from_numpy(w_real))
+    wind.calc_idealized_wgrid(dom, dom.w_dqdt)
+    np.testing.assert_array_equal(dom.w_dqdt.cpu().numpy(), want)
     # the bulk Richardson number (the Froude number's sector may differ within an ulp: its other test)
     theta, ft = cases.stability_inputs(case, seed=1, nsect=4)
     dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (case.domain.z, theta, ft)]
@@ -38,6 +42,14 @@ def test_per_step_kernels(lib, oracle_mod, nx, ny, nz, halo):
     fr_ref, ri_ref = s.update_stability(case.u, case.v, case.domain.z, theta, ft)
     np.testing.assert_array_equal(ri.cpu().numpy(), ri_ref)
     assert np.mean(froude.cpu().numpy() != fr_ref) < 0.01
+    # the same over its inputs: each output in the place of theta or of the heights
+    for f_at, r_at in ((0, None), (1, None), (None, 0), (None, 1), (0, 1), (1, 0)):
+        ins, outs = [dev[0].clone(), dev[1].clone()], [new(), new()]
+        for q, at in enumerate((f_at, r_at)):
+            if at is not None:
+                outs[q] = ins[at]
+        wind.update_stability(dom, ins[0], ins[1], outs[0], outs[1], dev[2])
+        assert torch.equal(outs[0], froude) and torch.equal(outs[1], ri)
     # alpha, into another array and over its input
     lib_ = _capi.load()
     fr = torch.from_numpy(fr_ref).cuda()
