@@ -1574,15 +1574,7 @@ extern "C" int hicarw_calc_alpha(hicarw_handle *h, const float *froude, float *a
     api_entry();
     if (!h || !froude || !alpha || halo < 0 || 2 * halo >= h->d.nx || 2 * halo >= h->d.ny || device_only(mem_kind))
         return HICARW_ERR_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    int rc;
-    float *out = alpha; // edge cells read other cells' Froude numbers: not over their own input
-    if (froude == alpha) {
-        if ((rc = ensure_work(h)) != 0) return rc;
-        out = h->swork;
-    }
-    launch_calc_alpha(h->d, froude, out, halo, s);
-    if (out != alpha) CK(cudaMemcpyAsync(alpha, out, n_cell(h->d) * 4, cudaMemcpyDeviceToDevice, s));
+    launch_calc_alpha(h->d, froude, alpha, halo, (cudaStream_t)stream);
     CK(cudaGetLastError());
     return HICARW_OK;
 }

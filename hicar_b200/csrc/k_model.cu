@@ -868,7 +868,7 @@ void launch_update_stability(const Dims &d, const float *u, const float *v, cons
 // copies the h outermost rows and columns, south, west, north, east, from the
 // first ones inside; together these take every cell's value from the nearest cell
 // of the tile, which is where its Froude number is read here.
-__global__ void calc_alpha_kernel(Dims d, const float *__restrict__ froude, float *__restrict__ alpha, int h)
+__global__ void calc_alpha_kernel(Dims d, const float *froude, float *alpha, int h)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, j = blockIdx.z + 1;
     if (i > d.nx) return;
@@ -882,6 +882,15 @@ __global__ void calc_alpha_kernel(Dims d, const float *__restrict__ froude, floa
     a = a > 0.2f ? a : 0.2f;
     a = a < 2.0f ? a : 2.0f;
     alpha[cidx(d, i, k, j)] = k == d.nz ? 0.2f : a;
+}
+
+// the cells within h of the edge, from the nearest cell of the tile
+__global__ void alpha_edges_kernel(Dims d, float *alpha, int h)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, j = blockIdx.z + 1;
+    if (i > d.nx) return;
+    const int is = min(max(i, h + 1), d.nx - h), js = min(max(j, h + 1), d.ny - h);
+    if (is != i || js != j) alpha[cidx(d, i, k, j)] = alpha[cidx(d, is, k, js)];
 }
 
 // one pass of smooth_array_3d, ydim = 3 (array_utilities.F90:322-397): x-y box
@@ -974,8 +983,11 @@ void launch_calc_w(const Dims &d, const Metrics &m, const float *div, const floa
 
 void launch_calc_alpha(const Dims &d, const float *froude, float *alpha, int halo, cudaStream_t st)
 {
-    calc_alpha_kernel<<<dim3((d.nx + 127) / 128, d.nz, d.ny), 128, 0, st>>>(d, froude, alpha, halo);
-    count_launch(1);
+    const dim3 g((d.nx + 127) / 128, d.nz, d.ny);
+    const bool over = alpha == froude; // an edge cell may not read a Froude number that its own cell overwrites
+    calc_alpha_kernel<<<g, 128, 0, st>>>(d, froude, alpha, over ? 0 : halo);
+    if (over && halo > 0) alpha_edges_kernel<<<g, 128, 0, st>>>(d, alpha, halo);
+    count_launch(over && halo > 0 ? 2 : 1);
 }
 
 void launch_smooth_xy(const Dims &d, const float *in, float *out, int w, cudaStream_t st)

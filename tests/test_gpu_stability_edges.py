@@ -65,3 +65,25 @@ def test_per_step_kernels(lib, oracle_mod, nx, ny, nz, halo):
         _capi.check(lib_.hicarw_smooth_alpha(h, C.c_void_p(a.data_ptr()), window, passes, 0, None), h)
         np.testing.assert_array_equal(a.cpu().numpy(), s.smooth_array(want, window, passes))
     wi.finalize_iter_winds()
+
+
+def test_alpha_over_its_input_can_be_captured(lib, oracle_mod):
+    """calc_alpha written over its Froude numbers, as the first call on a handle inside a stream capture: nothing is allocated."""
+    from hicar_b200 import wind_iterative as wi
+    from hicar_b200.domain import DeviceDomain
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    wi.finalize_iter_winds()
+    case = cases.build_case(33, 17, 9, seed=5, n_hills=3)
+    dom = DeviceDomain.from_case(case, "cuda")
+    wi.init_iter_winds(dom, wi.WindOptions())
+    fr = np.exp(np.random.default_rng(5).uniform(-3.0, 3.0, case.w.shape)).astype(np.float32)
+    a = torch.from_numpy(fr).cuda()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        rc = _capi.load().hicarw_calc_alpha(wi.handle(dom.nest_indx), C.c_void_p(a.data_ptr()), C.c_void_p(a.data_ptr()), 2,
+                                            _capi.MEM_DEVICE, C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == _capi.HICARW_OK
+    graph.replay()
+    np.testing.assert_array_equal(a.cpu().numpy(), oracle_mod.OracleSolver(case.domain).calc_alpha(fr, 2))
+    wi.finalize_iter_winds()
