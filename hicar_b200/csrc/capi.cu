@@ -142,9 +142,20 @@ struct hicarw_handle {
     double *dist_buf = nullptr; // decomposed solve: device staging of host-side totals (5 values)
     int tune_mg_feed = -1; // multigrid post-smoother feed: 1 tensor copies, 0 register-fed, -1 the build's choice
     int use_mg = 0;       // preconditioner of the solve being enqueued
+    long long plan = 0;   // counts the changes after which launches captured from this handle no longer stand
     std::string err;
     long long launches_at_call = 0;
 };
+
+// The handle's loop graphs no longer stand; with plan, nor do launches that a
+// batch has captured from the handle: a buffer moved, or a value that they hold
+// changed.
+static void drop_graphs(hicarw_handle *h, bool plan = true)
+{
+    for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
+    h->graphs.clear();
+    if (plan) h->plan++;
+}
 
 static void set_err(hicarw_handle *h, const char *what, cudaError_t e)
 {
@@ -211,9 +222,12 @@ static int mg_ensure(hicarw_handle *h, cudaStream_t s)
             return HICARW_ERR_CUDA;
         }
         h->mg_dirty = 0;
+        drop_graphs(h);
         return 1;
     }
-    return mg_refresh(h->mg, s);
+    if (!mg_refresh(h->mg, s)) return 0;
+    drop_graphs(h);
+    return 1;
 }
 
 static Metrics metrics_of(const hicarw_handle *h)
@@ -271,8 +285,7 @@ static int ensure_vectors(hicarw_handle *h, int prec)
     }
     for (int q = 0; q < NVEC; q++) h->vec[q] = nv[q];
     h->vprec = prec;
-    for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-    h->graphs.clear();
+    drop_graphs(h);
     return 0;
 }
 
@@ -395,8 +408,7 @@ extern "C" int hicarw_finalize_iter_winds(hicarw_handle *h)
     api_entry();
     if (!h) return HICARW_ERR_ARG;
     cudaDeviceSynchronize();
-    for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-    h->graphs.clear();
+    drop_graphs(h);
     mg_free(h->mg);
     if (h->gst) cudaFree(h->gst);
     if (h->fg_host) cudaFreeHost(h->fg_host);
@@ -438,8 +450,7 @@ extern "C" int hicarw_set_options(hicarw_handle *h, const hicarw_options *opt)
     }
     int prec = solve_precision(h);
     int rc = ensure_vectors(h, prec);
-    for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-    h->graphs.clear();
+    drop_graphs(h);
     // V-cycle parameters are read when its launches are enqueued (the graphs were just dropped)
     const int pre0_was = h->mg.pre0;
     mg_params(h);
@@ -764,8 +775,7 @@ static int fgmres_prepare(hicarw_handle *h, int sweeps, FgmresCtx *f)
         CK(dalloc((void **)&h->fgZ, (size_t)m * d.npad * sizeof(double)));
         CK(dalloc((void **)&h->fgW, (size_t)d.npad * sizeof(double)));
         h->fg_m = m;
-        for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-        h->graphs.clear();
+        drop_graphs(h);
     }
     h->fg_pc.h = h;
     h->fg_pc.sweeps = sweeps;
@@ -1145,11 +1155,10 @@ extern "C" int hicarw_probe_finalize(hicarw_handle *h, float max_leak, void *str
 {
     api_entry();
     if (!h) return HICARW_ERR_ARG;
+    drop_graphs(h, !h->operator_probed);
     h->operator_probed = 1;
     h->structure_uploaded = 1;
     h->mg_dirty = h->unet_dirty = 1;
-    for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-    h->graphs.clear();
     if (h->opt.verbose)
         fprintf(stderr, "Projection operator calibrated by probing (A = 2*D o G); off-stencil leakage max |T| = %g\n",
                 (double)max_leak);
@@ -1237,11 +1246,10 @@ extern "C" int hicarw_set_coefs(hicarw_handle *h, const float *coefs, int probed
     if (!h || !coefs) return HICARW_ERR_ARG;
     const int rc = copy_coefs(h, const_cast<float *>(coefs), 0, mem_kind, (cudaStream_t)stream);
     if (rc) return rc;
+    drop_graphs(h, h->operator_probed != (probed ? 1 : 0));
     h->operator_probed = probed ? 1 : 0;
     h->structure_uploaded = 1;
     h->mg_dirty = h->unet_dirty = 1;
-    for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-    h->graphs.clear();
     return HICARW_OK;
 }
 
@@ -1515,8 +1523,7 @@ extern "C" int hicarw_set_learned_precond(hicarw_handle *h, hicarw_unet *n)
     }
     if (h->unet != n) {
         cudaDeviceSynchronize();
-        for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-        h->graphs.clear();
+        drop_graphs(h);
     }
     h->unet = n;
     h->unet_dirty = 1;
@@ -1587,8 +1594,7 @@ extern "C" int hicarw_dist_configure(hicarw_handle *h, int edges)
     api_entry();
     if (!h || edges < 0 || edges > 15) return HICARW_ERR_ARG;
     cudaDeviceSynchronize();
-    for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-    h->graphs.clear();
+    drop_graphs(h);
     h->edges = edges;
     if (!h->dist_buf) CK(dalloc((void **)&h->dist_buf, 8 * sizeof(double)));
     return HICARW_OK;
@@ -1741,8 +1747,7 @@ extern "C" int hicarw_set_kernel_tuning(hicarw_handle *h, int spmv_levels, int m
     api_entry();
     if (!h || spmv_levels < 0 || spmv_levels > 1024 || mg_post_feed < -1 || mg_post_feed > 1) return HICARW_ERR_ARG;
     cudaDeviceSynchronize();
-    for (auto &g : h->graphs) cudaGraphExecDestroy(g.second.exec);
-    h->graphs.clear();
+    drop_graphs(h);
     h->tune_kc = spmv_levels;
     h->tune_mg_feed = mg_post_feed;
     if (mg_post_feed >= 0) h->mg.use_tma = mg_post_feed ? 2 : 0;
@@ -1826,6 +1831,7 @@ struct hicarw_batch {
     cudaGraphExec_t exec = nullptr;
     long long nodes = 0;
     std::vector<hicarw_batch_item> built;
+    std::vector<long long> built_plan; // the handles' plans that exec was captured from
     int built_lanes = -1, built_chunk = -1, built_cold = -1;
     std::vector<FgmresCtx> fg; // launch contexts of the FGMRES subdomains
     int *counters = nullptr; // device: WHILE-body executions per subdomain
@@ -1884,6 +1890,7 @@ static bool same_items(const hicarw_batch *b, const hicarw_batch_item *items)
         const hicarw_batch_item &x = b->built[i], &y = items[i];
         if (x.alpha != y.alpha || x.div != y.div || x.density != y.density || x.u != y.u || x.v != y.v || x.w != y.w)
             return false;
+        if (b->built_plan[i] != b->hs[i]->plan) return false;
     }
     return true;
 }
@@ -1998,6 +2005,8 @@ static int batch_build(hicarw_batch *b, const hicarw_batch_item *items, int cold
     }
     b->nodes = nodes;
     b->built.assign(items, items + n);
+    b->built_plan.resize(n);
+    for (int i = 0; i < n; i++) b->built_plan[i] = b->hs[i]->plan;
     b->built_lanes = b->lanes;
     b->built_chunk = b->chunk;
     b->built_cold = cold;
@@ -2010,27 +2019,28 @@ static int batch_run(hicarw_batch *b, const hicarw_batch_item *items, int adv_de
 {
     const int n = (int)b->hs.size();
     int rc;
-    bool rebuild = !b->exec || !same_items(b, items) || b->built_lanes != b->lanes || b->built_chunk != b->chunk ||
-                   b->built_cold != cold;
+    bool rebuild = false;
     b->fg.resize(n);
     for (int i = 0; i < n; i++) {
         hicarw_handle *h = b->hs[i];
         h->launches_at_call = g_launches.load();
         select_precond(h, 1);
-        if (h->use_mg) {
-            if ((rc = mg_ensure(h, s)) < 0)
-                return batch_fail(HICARW_ERR_CUDA, "multigrid build of subdomain " + std::to_string(i) + ": " + h->err);
-            if (rc) rebuild = true;
-        }
+        // the batch's launches are FP64, whatever Krylov precision later options name for the handle's own solves
+        if ((rc = ensure_vectors(h, HICARW_KRYLOV_F64)) != 0)
+            return batch_fail(rc, "vectors of subdomain " + std::to_string(i) + ": " + h->err);
+        if (h->use_mg && (rc = mg_ensure(h, s)) < 0)
+            return batch_fail(HICARW_ERR_CUDA, "multigrid build of subdomain " + std::to_string(i) + ": " + h->err);
         if (h->opt.solver == HICARW_SOLVER_FGMRES) {
             const bool dirty = (h->use_learned || h->use_mglearned) && h->unet_dirty;
             FgmresCtx f;
             if ((rc = fgmres_ready(h, h->precond_n_sweeps, s, &f)) != 0)
                 return batch_fail(rc, "FGMRES set-up of subdomain " + std::to_string(i) + ": " + h->err);
-            if (dirty || b->fg[i].V != f.V || b->fg[i].m != f.m) rebuild = true;
+            if (dirty) rebuild = true;
             b->fg[i] = f;
         }
     }
+    rebuild = rebuild || !b->exec || !same_items(b, items) || b->built_lanes != b->lanes ||
+              b->built_chunk != b->chunk || b->built_cold != cold;
     if (rebuild) {
         BCK(cudaStreamSynchronize(s));
         if ((rc = batch_build(b, items, cold)) != 0) return rc;
@@ -2055,7 +2065,7 @@ static int batch_run(hicarw_batch *b, const hicarw_batch_item *items, int adv_de
     for (int i = 0; i < n; i++) { // a stalled or failed preconditioned solve: the reference solve decides
         hicarw_handle *h = b->hs[i];
         if (h->hst->status != 0 && (h->use_mg || h->use_learned)) {
-            if ((rc = zero_solution(h, s)) != 0 || (rc = bicgstab_solve(h, h->precond_n_sweeps, s, 0)) != 0)
+            if ((rc = zero_solution(h, s)) != 0 || (rc = bicgstab_solve(h, h->precond_n_sweeps, s, 0, HICARW_KRYLOV_F64)) != 0)
                 return batch_fail(rc, "fallback solve of subdomain " + std::to_string(i) + ": " + h->err);
             fell[i] = 1;
         }

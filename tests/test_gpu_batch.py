@@ -140,3 +140,45 @@ def test_batch_mixes_fgmres_and_learned_with_bicgstab():
             assert torch.equal(lam_b[i], lam)
     finally:
         bs.close()
+
+
+def test_batch_follows_options_changed_between_its_steps():
+    """The batch's graph is captured from its handles: after set_options, also when a
+    call on the handle itself came in between and took the change over (the coarse
+    matrix of 64x64x4 moves between levels 1 and 2, the vectors become FP32, the
+    residual history grows), a step equals that of a new batch with these options."""
+    from hicar_b200.batch import BatchSolver
+    from hicar_b200.wind_iterative import WindOptions
+    cs = [cases.build_case(64, 64, 4, seed=60, adv_den=True, n_hills=6), _cases()[0]]
+    base = dict(tol_rel=1e-6, wind_solver_iterations=300, precond=_capi.PRECOND_MG, stall_iters=50)
+    start = dict(base, mg_w_levels=(1,))
+    changes = [dict(base), dict(base, mg_omega=0.9), dict(start, krylov_precision=_capi.KRYLOV_F32_X64),
+               dict(start, wind_solver_iterations=4000), dict(start, solver=_capi.SOLVER_FGMRES, fgmres_restart=12), start]
+    lib = _capi.load()
+
+    def solve(bs):
+        assert all(s["status"] == 0 for s in bs.step())
+        return [bs.lambda_of(i).cpu() for i in range(bs.n)]
+
+    bs = BatchSolver(cs, options=WindOptions(**start))
+    try:
+        first = solve(bs)
+        for between in (True, False):
+            for kw in changes:
+                _capi.check(lib.hicarw_set_options(bs.handles[0], C.byref(WindOptions(**kw).to_c())), bs.handles[0])
+                if between:
+                    _single(bs, 0)
+                got = solve(bs)
+                ref = BatchSolver(cs, options=WindOptions(**start))
+                try:
+                    kw64 = {**kw, "krylov_precision": _capi.KRYLOV_F64}
+                    _capi.check(lib.hicarw_set_options(ref.handles[0], C.byref(WindOptions(**kw64).to_c())), ref.handles[0])
+                    want = solve(ref)
+                finally:
+                    ref.close()
+                for a, b in zip(got, want):
+                    assert torch.equal(a, b), (kw, between)
+        for a, b in zip(got, first):
+            assert torch.equal(a, b)
+    finally:
+        bs.close()
