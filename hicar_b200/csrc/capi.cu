@@ -212,9 +212,11 @@ static int mg_build_tuned(hicarw_handle *h, cudaStream_t s)
 
 // The V-cycle for the handle's present coefficients and options, built or
 // refreshed where it is not: 1 when anything was made again, 0 when it stood,
-// negative on failure.  Never inside a stream capture.
-static int mg_ensure(hicarw_handle *h, cudaStream_t s)
+// negative on failure.  dense: with the tabulated coarse part that solves use.
+// Never inside a stream capture.
+static int mg_ensure(hicarw_handle *h, cudaStream_t s, bool dense = true)
 {
+    int made = 0;
     if (h->mg_dirty || !h->mg.ready) {
         mg_params(h);
         if (mg_build_tuned(h, s) != 0) {
@@ -222,12 +224,11 @@ static int mg_ensure(hicarw_handle *h, cudaStream_t s)
             return HICARW_ERR_CUDA;
         }
         h->mg_dirty = 0;
-        drop_graphs(h);
-        return 1;
+        made = 1;
     }
-    if (!mg_refresh(h->mg, s)) return 0;
-    drop_graphs(h);
-    return 1;
+    if (dense && mg_refresh(h->mg, s)) made = 1;
+    if (made) drop_graphs(h);
+    return made;
 }
 
 static Metrics metrics_of(const hicarw_handle *h)
@@ -1353,7 +1354,7 @@ extern "C" int hicarw_apply_precond(hicarw_handle *h, const double *x, double *y
     int *herr = h->hflag;
     *herr = 0;
     if (!rc && sweeps <= 0) {
-        if (!(learned && h->opt.precond == HICARW_PRECOND_LEARNED)) rc = std::min(0, mg_ensure(h, s));
+        if (!(learned && h->opt.precond == HICARW_PRECOND_LEARNED)) rc = std::min(0, mg_ensure(h, s, false)); // step by step: no matrix
         if (!rc) {
             CK(cudaMemsetAsync(by, 0, (size_t)d.npad * 8, s));
             if (learned) CK(cudaMemsetAsync(h->vec[V_T], 0, (size_t)d.npad * 8, s));

@@ -1555,112 +1555,207 @@ __global__ void __launch_bounds__(DN_THREADS) dense_apply_kernel(const float *__
     if (lane == 0 && row < n) x[kidx(d, row % d.nx + 1, row / d.nx % d.nz + 1, row / (d.nx * d.nz) + 1)] = y;
 }
 
-// ---- tabulating the matrix: the cycle's steps on n right-hand sides at once,
-// FP64, vectors as [cell][right-hand side] (coalesced over the right-hand
-// sides), x = nullptr standing for zero and r = nullptr for the unit vectors ----
-__device__ __forceinline__ double table_at(const double *x, const Dims &d, int i, int k, int j, int n, int q)
+// ---- tabulating the matrix: a CTA runs the cycle on one unit vector ----
+// The n unit vectors are independent and the levels of one fit in shared memory
+// (FP64: about 24 bytes an unknown, 98 KB at n = 4096), so a tabulation is one
+// launch of n CTAs with no memory of its own beside the matrix.
+// What bounds it: the serial column recurrences and the L2 round trips for
+// coefficients and factors between CTA barriers, which other CTAs on the SM hide in
+// part.  The first solve on a new operator at 181x157x33 (n = 3960) takes 12.1 ms,
+// a next one 5.9; with all unit vectors advanced together by a launch per step, over
+// 510 MB of memory mapped and unmapped around it, it took 15.4 ms and now and then
+// 20 to 50, at 512x512x48 41.7 ms and up to 414 where it now takes 40.0.
+struct TableLevel {
+    Dims d;
+    unsigned inv_x, inv_z; // of the divisions by nx and nz (table_div)
+    const float *coef, *cp, *minv;
+    int x1, x3, r; // offsets of its vectors in shared memory (doubles); r: below the tabulated level
+};
+struct TableArgs {
+    TableLevel lev[MG_MAX_LEVELS]; // from the tabulated level down
+    int nlev, n, ld;
+    unsigned wmask;                // bit l: level l corrects twice (levels counted as in lev)
+    double omega, cscale;
+};
+// Threads of a CTA: TABLE_THREADS where at most two fit on an SM by shared memory,
+// else half as many (first solve on a new operator: 181x157x33, n = 3960, 128 threads
+// 14.6 ms, 256 12.1, 384 15.2; 512x512x48, n = 3072, 40.0, 40.1, 41.1; 64x64x20,
+// n = 1280, 2.7, 2.9, 3.6).
+constexpr int TABLE_THREADS = 256, TABLE_U = 8; // TABLE_U: levels of a column read ahead
+
+// a / d for a < 2^16, d <= 4096, m = 2^32 / d rounded up (0 for d = 1): the error of
+// m is below d / 2^32, that of the quotient below a d / 2^32 / d < 1 / d
+__host__ __device__ inline unsigned table_inverse(int d) { return d == 1 ? 0u : (unsigned)((0x100000000ull + d - 1) / d); }
+__device__ __forceinline__ int table_div(int a, unsigned m) { return m ? (int)__umulhi((unsigned)a, m) : a; }
+
+// the place of a cell
+__device__ __forceinline__ void table_cell(const TableLevel &L, int cell, int &i, int &k, int &j)
 {
-    return x && inside(d, i, k, j) ? x[(size_t)dense_index(d, i, k, j) * n + q] : 0.0;
+    const int row = table_div(cell, L.inv_x), q = table_div(row, L.inv_z);
+    i = cell - row * L.d.nx + 1;
+    k = row - q * L.d.nz + 1;
+    j = q + 1;
 }
 
-// rc = R^T (r - A x), one thread per (coarse cell, right-hand side)
-__global__ void table_restrict_kernel(Dims f, const float *__restrict__ coef, const double *__restrict__ r,
-                                      const double *__restrict__ x, Dims dc, double *__restrict__ rc, int n)
+__device__ __forceinline__ double table_at(const double *x, const Dims &d, int i, int k, int j)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x, cell = blockIdx.y;
-    if (q >= n) return;
-    const int I = cell % dc.nx + 1, row = cell / dc.nx, k = row % dc.nz + 1, J = row / dc.nz + 1;
-    double acc = 0.0;
-    for (int child = 0; child < 4; child++) {
+    return x && inside(d, i, k, j) ? x[dense_index(d, i, k, j)] : 0.0;
+}
+
+// rc = R^T (r - A x), r = nullptr: the unit vector q; four lanes per coarse cell,
+// one per child, added in the children's order
+__device__ __forceinline__ void table_restrict(const TableLevel &F, const double *r, int q, const double *x,
+                                               const TableLevel &C, double *rc)
+{
+    const Dims &f = F.d, &dc = C.d;
+    const int items = 4 * dc.nx * dc.ny * dc.nz;
+    for (int base = 0; base < items; base += blockDim.x) { // whole warps: the shuffles below
+        const int t = base + threadIdx.x, cell = t >> 2, child = t & 3;
+        int I, k, J;
+        table_cell(C, cell, I, k, J);
         const int i = 2 * I - 1 + (child & 1), j = 2 * J - 1 + (child >> 1);
-        if (i > f.nx || j > f.ny) continue;
-        const int fc = dense_index(f, i, k, j);
-        double y = r ? r[(size_t)fc * n + q] : (fc == q ? 1.0 : 0.0);
-        const long long o = kidx(f, i, k, j);
+        double y = 0.0;
+        if (t < items && i <= f.nx && j <= f.ny) {
+            const int fc = dense_index(f, i, k, j);
+            const long long o = kidx(f, i, k, j);
+            float cv[15];
+            load_coefs(F.coef, f.npad, o, cv);
+            y = r ? r[fc] : (fc == q ? 1.0 : 0.0);
 #pragma unroll
-        for (int s = 0; s < 15; s++)
-            y -= (double)coef[(long long)s * f.npad + o] * table_at(x, f, i + off_i(s), k + off_k(s), j + off_j(s), n, q);
-        acc += y;
-    }
-    rc[(size_t)cell * n + q] = acc;
-}
-
-// res = r - A x2 with x2 = x + cs P xc, one thread per (cell, right-hand side)
-__global__ void table_residual_kernel(Dims d, const float *__restrict__ coef, const double *__restrict__ r,
-                                      const double *__restrict__ x, Dims dc, const double *__restrict__ xc, double cs,
-                                      double *__restrict__ res, int n)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x, cell = blockIdx.y;
-    if (q >= n) return;
-    const int i = cell % d.nx + 1, row = cell / d.nx, k = row % d.nz + 1, j = row / d.nz + 1;
-    double y = r ? r[(size_t)cell * n + q] : (cell == q ? 1.0 : 0.0);
-    const long long o = kidx(d, i, k, j);
-#pragma unroll
-    for (int s = 0; s < 15; s++) {
-        const int ii = i + off_i(s), kk = k + off_k(s), jj = j + off_j(s);
-        if (!inside(d, ii, kk, jj)) continue;
-        y -= (double)coef[(long long)s * d.npad + o] *
-             (table_at(x, d, ii, kk, jj, n, q) + cs * table_at(xc, dc, (ii + 1) >> 1, kk, (jj + 1) >> 1, n, q));
-    }
-    res[(size_t)cell * n + q] = y;
-}
-
-// out = x2 + w T^-1 res (x2 as above, zero where x and xc are null), one thread
-// per (column, right-hand side); the operands of TABLE_U levels are read ahead
-constexpr int TABLE_U = 8;
-__global__ void table_columns_kernel(Dims d, const float *__restrict__ coef, const float *__restrict__ cp,
-                                     const float *__restrict__ minv, const double *__restrict__ res,
-                                     const double *__restrict__ x, Dims dc, const double *__restrict__ xc, double cs,
-                                     double omega, double *out, int n)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y % d.nx + 1, j = blockIdx.y / d.nx + 1;
-    if (q >= n) return;
-    double dp = 0.0;
-    for (int k0 = 1; k0 <= d.nz; k0 += TABLE_U) {
-        double rv[TABLE_U];
-        float cv[TABLE_U], mv[TABLE_U];
-#pragma unroll
-        for (int u = 0; u < TABLE_U; u++) {
-            const int k = k0 + u;
-            const bool in = k <= d.nz;
-            const int cell = dense_index(d, i, in ? k : d.nz, j);
-            const long long o = kidx(d, i, in ? k : d.nz, j);
-            rv[u] = res ? res[(size_t)cell * n + q] : (cell == q ? 1.0 : 0.0);
-            cv[u] = k > 1 ? coef[(long long)CC * d.npad + o] : 0.0f;
-            mv[u] = minv[o];
+            for (int s = 0; s < 15; s++)
+                y -= (double)cv[s] * table_at(x, f, i + off_i(s), k + off_k(s), j + off_j(s));
         }
-#pragma unroll
-        for (int u = 0; u < TABLE_U; u++)
-            if (k0 + u <= d.nz) {
-                dp = (rv[u] - (double)cv[u] * dp) * (double)mv[u];
-                out[(size_t)dense_index(d, i, k0 + u, j) * n + q] = dp;
-            }
-    }
-    double y = 0.0;
-    for (int k0 = d.nz; k0 >= 1; k0 -= TABLE_U) {
-        double rv[TABLE_U], bv[TABLE_U];
-        float pv[TABLE_U];
-#pragma unroll
-        for (int u = 0; u < TABLE_U; u++) {
-            const int k = max(k0 - u, 1);
-            rv[u] = out[(size_t)dense_index(d, i, k, j) * n + q];
-            pv[u] = cp[kidx(d, i, k, j)];
-            bv[u] = table_at(x, d, i, k, j, n, q) + cs * table_at(xc, dc, (i + 1) >> 1, k, (j + 1) >> 1, n, q);
-        }
-#pragma unroll
-        for (int u = 0; u < TABLE_U; u++)
-            if (k0 - u >= 1) {
-                y = rv[u] - (double)pv[u] * y;
-                out[(size_t)dense_index(d, i, k0 - u, j) * n + q] = bv[u] + omega * y;
-            }
+        const double y1 = __shfl_down_sync(0xffffffffu, y, 1), y2 = __shfl_down_sync(0xffffffffu, y, 2),
+                     y3 = __shfl_down_sync(0xffffffffu, y, 3);
+        if (t < items && child == 0) rc[cell] = ((y + y1) + y2) + y3; // a missing child adds zero
     }
 }
 
-// S = x rounded to FP32, rows padded to ld
-__global__ void table_store_kernel(const double *__restrict__ x, int n, int ld, float *__restrict__ S)
+// res = r - A x2 with x2 = x + cs P xc
+__device__ __forceinline__ void table_residual(const TableLevel &L, const double *r, int q, const double *x, const Dims &dc,
+                                               const double *xc, double cs, double *res)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y;
-    if (q < ld) S[(size_t)row * ld + q] = q < n ? (float)x[(size_t)row * n + q] : 0.0f;
+    const Dims &d = L.d;
+    for (int cell = threadIdx.x; cell < d.nx * d.ny * d.nz; cell += blockDim.x) {
+        int i, k, j;
+        table_cell(L, cell, i, k, j);
+        const long long o = kidx(d, i, k, j);
+        float cv[15];
+        load_coefs(L.coef, d.npad, o, cv);
+        double y = r ? r[cell] : (cell == q ? 1.0 : 0.0);
+#pragma unroll
+        for (int s = 0; s < 15; s++) {
+            const int ii = i + off_i(s), kk = k + off_k(s), jj = j + off_j(s);
+            if (!inside(d, ii, kk, jj)) continue;
+            y -= (double)cv[s] *
+                 (table_at(x, d, ii, kk, jj) + cs * table_at(xc, dc, (ii + 1) >> 1, kk, (jj + 1) >> 1));
+        }
+        res[cell] = y;
+    }
+}
+
+// out = x2 + w T^-1 res (x2 as above, zero where x and xc are null; res = nullptr:
+// the unit vector q; out may be res), one thread per column
+__device__ __forceinline__ void table_columns(const TableLevel &L, const double *res, int q, const double *x, const Dims &dc,
+                                              const double *xc, double cs, double omega, double *out)
+{
+    const Dims &d = L.d;
+    for (int c = threadIdx.x; c < d.nx * d.ny; c += blockDim.x) {
+        const int jj = table_div(c, L.inv_x), i = c - jj * d.nx + 1, j = jj + 1;
+        double dp = 0.0;
+        float cv[TABLE_U], mv[TABLE_U], pv[TABLE_U];
+        auto down = [&](int k0) { // the factors of the next TABLE_U levels
+#pragma unroll
+            for (int u = 0; u < TABLE_U; u++) {
+                const long long o = kidx(d, i, min(k0 + u, d.nz), j);
+                cv[u] = __ldg(L.coef + (long long)CC * d.npad + o);
+                mv[u] = __ldg(L.minv + o);
+            }
+        };
+        down(1);
+        for (int k0 = 1; k0 <= d.nz; k0 += TABLE_U) {
+            double rv[TABLE_U], cn[TABLE_U], mn[TABLE_U];
+#pragma unroll
+            for (int u = 0; u < TABLE_U; u++) {
+                const int cell = dense_index(d, i, min(k0 + u, d.nz), j);
+                rv[u] = res ? res[cell] : (cell == q ? 1.0 : 0.0);
+                cn[u] = k0 + u > 1 ? (double)cv[u] : 0.0;
+                mn[u] = (double)mv[u];
+            }
+            down(k0 + TABLE_U);
+#pragma unroll
+            for (int u = 0; u < TABLE_U; u++)
+                if (k0 + u <= d.nz) {
+                    dp = (rv[u] - cn[u] * dp) * mn[u];
+                    out[dense_index(d, i, k0 + u, j)] = dp;
+                }
+        }
+        double y = 0.0;
+        auto up = [&](int k0) {
+#pragma unroll
+            for (int u = 0; u < TABLE_U; u++) pv[u] = __ldg(L.cp + kidx(d, i, max(k0 - u, 1), j));
+        };
+        up(d.nz);
+        for (int k0 = d.nz; k0 >= 1; k0 -= TABLE_U) {
+            double rv[TABLE_U], bv[TABLE_U], pn[TABLE_U];
+#pragma unroll
+            for (int u = 0; u < TABLE_U; u++) {
+                const int k = max(k0 - u, 1);
+                rv[u] = out[dense_index(d, i, k, j)];
+                pn[u] = (double)pv[u];
+                bv[u] = table_at(x, d, i, k, j) + cs * table_at(xc, dc, (i + 1) >> 1, k, (j + 1) >> 1);
+            }
+            up(k0 - TABLE_U);
+#pragma unroll
+            for (int u = 0; u < TABLE_U; u++)
+                if (k0 - u >= 1) {
+                    y = rv[u] - pn[u] * y;
+                    out[dense_index(d, i, k0 - u, j)] = bv[u] + omega * y;
+                }
+        }
+    }
+}
+
+// Column q = blockIdx.x of the matrix: the cycle on the unit vector q, rounded to FP32.
+__global__ void __launch_bounds__(TABLE_THREADS) table_kernel(const __grid_constant__ TableArgs a, float *__restrict__ S)
+{
+    extern __shared__ double tab[];
+    const int q = blockIdx.x, last = a.nlev - 1;
+    unsigned flip = 0, again = 0; // bit l: level l's iterate is in x3; its second correction runs
+    auto cur = [&](int l) { return tab + ((flip >> l) & 1 ? a.lev[l].x3 : a.lev[l].x1); };
+    auto other = [&](int l) { return tab + ((flip >> l) & 1 ? a.lev[l].x1 : a.lev[l].x3); };
+    auto rhs = [&](int l) { return l ? tab + a.lev[l].r : nullptr; };
+    table_columns(a.lev[0], nullptr, q, nullptr, a.lev[0].d, nullptr, 0.0, last ? a.omega : 1.0, cur(0));
+    __syncthreads();
+    int l = 0;
+    bool descend = last > 0;
+    while (descend) {
+        while (l < last) { // down: restrict, pre-smooth from zero (the last level: solve)
+            const TableLevel &F = a.lev[l], &C = a.lev[l + 1];
+            table_restrict(F, rhs(l), q, cur(l), C, tab + C.r);
+            __syncthreads();
+            l++;
+            flip &= ~(1u << l);
+            again &= ~(1u << l);
+            table_columns(C, tab + C.r, q, nullptr, C.d, nullptr, 0.0, l == last ? 1.0 : a.omega, cur(l));
+            __syncthreads();
+        }
+        descend = false;
+        while (l > 0 && !descend) { // up: correct and post-smooth, to a level that corrects once more
+            const double *xc = cur(l);
+            const Dims &dc = a.lev[l].d;
+            l--;
+            table_residual(a.lev[l], rhs(l), q, cur(l), dc, xc, a.cscale, other(l));
+            __syncthreads();
+            table_columns(a.lev[l], other(l), q, cur(l), dc, xc, a.cscale, a.omega, other(l));
+            __syncthreads();
+            flip ^= 1u << l;
+            descend = ((a.wmask & ~again) >> l) & 1;
+            if (descend) again |= 1u << l;
+        }
+    }
+    const double *x = cur(0);
+    for (int row = threadIdx.x; row < a.n; row += blockDim.x) S[(size_t)row * a.ld + q] = (float)x[row];
 }
 
 // ---------------------------------------------------------------------------
@@ -1793,7 +1888,7 @@ int mg_build(Mg &mg, const Dims &fine, const float *fine_coef, cudaStream_t s)
         mg.coef0h = nullptr;
     }
     const cudaError_t e = cudaGetLastError();
-    dense_setup(mg, s);
+    mg.dense_stale = 1; // tabulated when a solve asks for it (mg_refresh)
     fused_setup(mg);
     mg.ready = 1;
     return e == cudaSuccess ? 0 : -1;
@@ -2294,60 +2389,39 @@ static bool launch_fused(const Mg &mg, int l, const SolveState *gate, cudaStream
 }
 
 // ---- dense coarse cycle: where it starts, tabulation, launches ----
-static dim3 table_grid(int n, int y) { return dim3((n + 127) / 128, y); }
-
-// The cycle of level l (its pre-smoothed iterate in x1) on the unit vectors;
-// returns the buffer that holds its result.
-static double *tabulate(const Mg &mg, int l, double *const *r, double *const *x1, double *const *x3, double *res, int n,
-                        cudaStream_t s)
-{
-    if (l == mg.nlev - 1) return x1[l];
-    const MgLevel &F = mg.lev[l], &C = mg.lev[l + 1];
-    const bool last = l + 1 == mg.nlev - 1;
-    const int cells = F.d.nx * F.d.ny * F.d.nz, ccells = C.d.nx * C.d.ny * C.d.nz;
-    double *cur = x1[l], *other = x3[l];
-    for (int rep = 0; rep < ((mg.wmask >> l) & 1 ? 2 : 1); rep++) {
-        table_restrict_kernel<<<table_grid(n, ccells), 128, 0, s>>>(F.d, F.coef, r[l], cur, C.d, r[l + 1], n);
-        table_columns_kernel<<<table_grid(n, C.d.nx * C.d.ny), 128, 0, s>>>(
-            C.d, C.coef, C.cp, C.minv, r[l + 1], nullptr, C.d, nullptr, 0.0, last ? 1.0 : (double)mg.omega, x1[l + 1], n);
-        const double *xc = tabulate(mg, l + 1, r, x1, x3, res, n, s);
-        table_residual_kernel<<<table_grid(n, cells), 128, 0, s>>>(F.d, F.coef, r[l], cur, C.d, xc, (double)mg.cscale,
-                                                                   res, n);
-        table_columns_kernel<<<table_grid(n, F.d.nx * F.d.ny), 128, 0, s>>>(F.d, F.coef, F.cp, F.minv, res, cur, C.d, xc,
-                                                                            (double)mg.cscale, (double)mg.omega, other, n);
-        count_launch(4);
-        std::swap(cur, other);
-    }
-    return cur;
-}
-
 // Tabulate the cycle from mg.dense_level down into mg.dense with the present
-// cycle parameters; false when there is no memory for it.
+// cycle parameters; false when a unit vector's levels do not fit in shared memory.
 static bool dense_fill(Mg &mg, cudaStream_t s)
 {
-    const int l0 = mg.dense_level, n = mg.dense_n;
-    double *r[MG_MAX_LEVELS] = {}, *x1[MG_MAX_LEVELS] = {}, *x3[MG_MAX_LEVELS] = {}, *buf = nullptr;
-    size_t total = 0;
-    auto size = [&](int l) { return (size_t)mg.lev[l].d.nx * mg.lev[l].d.ny * mg.lev[l].d.nz * n; };
-    for (int l = l0; l < mg.nlev; l++) total += size(l) * (l == l0 ? 2 : 3);
-    total += size(l0); // residuals
-    if (cudaMallocAsync((void **)&buf, total * sizeof(double), s) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+    const int l0 = mg.dense_level;
+    TableArgs a{};
+    size_t total = 0; // doubles
+    a.nlev = mg.nlev - l0;
+    a.n = mg.dense_n;
+    a.ld = mg.dense_ld;
+    a.wmask = (unsigned)mg.wmask >> l0;
+    a.omega = mg.omega;
+    a.cscale = mg.cscale;
+    for (int l = 0; l < a.nlev; l++) {
+        const MgLevel &L = mg.lev[l0 + l];
+        const size_t n = (size_t)L.d.nx * L.d.ny * L.d.nz;
+        TableLevel &t = a.lev[l];
+        t.d = L.d;
+        t.inv_x = table_inverse(L.d.nx);
+        t.inv_z = table_inverse(L.d.nz);
+        t.coef = L.coef;
+        t.cp = L.cp;
+        t.minv = L.minv;
+        t.x1 = (int)total;
+        t.x3 = (int)(total + n);
+        t.r = (int)(total + 2 * n);
+        total += n * (l ? 3 : 2);
     }
-    double *p = buf;
-    for (int l = l0; l < mg.nlev; l++) {
-        if (l > l0) { r[l] = p; p += size(l); }
-        x1[l] = p; p += size(l);
-        x3[l] = p; p += size(l);
-    }
-    const MgLevel &T = mg.lev[l0];
-    table_columns_kernel<<<table_grid(n, T.d.nx * T.d.ny), 128, 0, s>>>(
-        T.d, T.coef, T.cp, T.minv, nullptr, nullptr, T.d, nullptr, 0.0, l0 == mg.nlev - 1 ? 1.0 : (double)mg.omega, x1[l0], n);
-    const double *x = tabulate(mg, l0, r, x1, x3, p, n, s);
-    table_store_kernel<<<dim3((mg.dense_ld + 127) / 128, n), 128, 0, s>>>(x, n, mg.dense_ld, mg.dense);
-    count_launch(2);
-    cudaFreeAsync(buf, s);
+    const size_t smem = total * sizeof(double);
+    if (smem > (size_t)smem_optin()) return false;
+    set_smem(table_kernel, smem);
+    table_kernel<<<a.n, 3 * smem > (size_t)smem_per_sm() ? TABLE_THREADS : TABLE_THREADS / 2, smem, s>>>(a, mg.dense);
+    count_launch(1);
     mg.dense_omega = mg.omega;
     mg.dense_cscale = mg.cscale;
     mg.dense_wmask = mg.wmask;
@@ -2379,6 +2453,8 @@ static bool dense_setup(Mg &mg, cudaStream_t s)
             dense_free(mg);
             return false;
         }
+        // the padding of the rows and of the right-hand side stays zero
+        cudaMemsetAsync(mg.dense, 0, (size_t)mg.dense_n * mg.dense_ld * sizeof(float), s);
         cudaMemsetAsync(mg.dense_r, 0, mg.dense_ld * sizeof(float), s);
     }
     if (dense_fill(mg, s)) return true;
@@ -2386,14 +2462,16 @@ static bool dense_setup(Mg &mg, cudaStream_t s)
     return false;
 }
 
-// Before the launches of a cycle are enqueued: the dense matrix belongs to the
-// cycle's present parameters.  1: the launches changed, 0: they stand.
+// Before the launches of a solve's cycle are enqueued: the dense matrix belongs to
+// the present levels and parameters.  1: the launches changed, 0: they stand.
 int mg_refresh(Mg &mg, cudaStream_t s)
 {
-    if (!mg.ready || !mg.dense_level ||
-        (mg.dense_omega == mg.omega && mg.dense_cscale == mg.cscale && mg.dense_wmask == mg.wmask))
+    if (!mg.ready) return 0;
+    if (!mg.dense_stale && (!mg.dense_level || (mg.dense_omega == mg.omega && mg.dense_cscale == mg.cscale &&
+                                                mg.dense_wmask == mg.wmask)))
         return 0;
     dense_setup(mg, s); // the level may move with the repeats
+    mg.dense_stale = 0;
     return 1;
 }
 

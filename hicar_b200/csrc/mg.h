@@ -36,6 +36,7 @@ struct Mg {
     float *dense = nullptr, *dense_r = nullptr; // the matrix and the compact right-hand side of a visit
     float dense_omega = 0.0f, dense_cscale = 0.0f; // the parameters that the matrix was tabulated with
     int dense_wmask = 0;
+    int dense_stale = 0; // the levels have been built since
     int bf16 = 0;        // the finest level's smoother coefficients in BF16 (V(0,1) cycles; factors of the rounded
                          // tridiagonal)
     __nv_bfloat16 *coef0h = nullptr; // those coefficients (15 * npad)
@@ -45,7 +46,7 @@ struct Mg {
 
 int mg_build(Mg &mg, const Dims &fine, const float *fine_coef, cudaStream_t s);
 void mg_free(Mg &mg);
-int mg_refresh(Mg &mg, cudaStream_t s); // after a change of omega, cscale or wmask: 1 when the cycle's launches changed
+int mg_refresh(Mg &mg, cudaStream_t s); // before a solve, after a build or a change of omega, cscale or wmask: 1 when the cycle's launches changed
 long long mg_tma_posts(); // post-smoother launches enqueued through the tensor-copy kernel
 template <typename V>
 void mg_apply(const Mg &mg, const V *in, V *out, const SolveState *gate, cudaStream_t s, bool steps = false);

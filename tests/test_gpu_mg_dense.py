@@ -38,8 +38,21 @@ def _direction(h, x, **cycle):
     return y / np.linalg.norm(y)
 
 
-# dense level 1 with few, with an odd number of and with many unknowns; a lower level; rows of one aggregate
-@pytest.mark.parametrize("shape", [(6, 4, 3), (9, 7, 5), (32, 32, 8), (63, 65, 4), (33, 31, 9), (3, 40, 24), (70, 50, 33)])
+def _dense_level(h):
+    """The level that the profile's dense products name."""
+    cap = 64
+    names, ms, by, cnt = C.create_string_buffer(32 * cap), (C.c_double * cap)(), (C.c_double * cap)(), (C.c_int * cap)()
+    n = _capi.load().hicarw_profile_iteration(h, 1, names, ms, by, cnt, cap, None)
+    levels = [s for s in (names.raw[32 * q:32 * q + 32].split(b"\0")[0].decode() for q in range(n)) if "dense" in s]
+    assert len(levels) == 1, levels
+    return int(levels[0].replace("mg_dense_l", ""))
+
+
+# dense level 1 with few, with an odd number of and with many unknowns; a lower level; rows of one aggregate;
+# level 1 with 4096, 4092 and 3300 unknowns (dense with repeats only), with 3072 (the limit without) and 4224
+# (over both limits)
+@pytest.mark.parametrize("shape", [(6, 4, 3), (9, 7, 5), (32, 32, 8), (63, 65, 4), (33, 31, 9), (3, 40, 24), (70, 50, 33),
+                                   (64, 64, 4), (66, 62, 4), (66, 50, 4), (64, 48, 4)])
 def test_dense_coarse_cycle_against_the_restatement(shape):
     """Tolerance: the restatement runs the levels in FP32 as the per-level kernels
     do; 1e-5 is the bar of those kernels' own tests."""
@@ -65,6 +78,10 @@ def test_dense_coarse_cycle_against_the_restatement(shape):
         ref = mg_ref.VCycle(coefs, omega, scale, fine_presmooth=not skip, wlevels=wlev)(x[1:-1, 1:-1, 1:-1])
         ref = ref / np.linalg.norm(ref)
         got = y[1:-1, 1:-1, 1:-1]
+        sizes, level = (nx, ny), 0
+        while not level or sizes[0] * sizes[1] * nz > (4096 if level in wlev else 3072):
+            sizes, level = ((sizes[0] + 1) // 2, (sizes[1] + 1) // 2), level + 1
+        assert _dense_level(h) == level
         assert np.linalg.norm(got - np.sign((got * ref).sum()) * ref) < 1e-5, (omega, wlev)
         assert not y[0].any() and not y[-1].any() and not y[:, 0].any() and not y[:, :, -1].any()
         first = y if first is None else first
