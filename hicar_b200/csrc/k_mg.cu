@@ -664,10 +664,9 @@ __global__ void __launch_bounds__(pt::THREADS, 2)
 // post_tma_kernel.  Eight consumer warps read each cell's 15 neighbours of x2
 // = x1 + s P xc straight from the staged x1 and coarse rows (P is piecewise
 // constant over the 2 x 2 aggregates, so a neighbour's coarse cell is an index
-// shift; neighbours outside the interior count as zero), form the residuals,
-// release the stage as soon as their reads are done, and hand each chunk's
-// rows (residual, x2, cp, c, 1/m) to a recurrence warp through a ring of two
-// slots.  No CTA barrier is taken per chunk.  The recurrence warp owns the
+// shift; neighbours outside the interior count as zero), form the residuals, hand
+// each chunk's rows (residual, x2, cp, c, 1/m) to a recurrence warp through a ring
+// of two slots and release the stage.  No CTA barrier is taken per chunk.  The recurrence warp owns the
 // tile's column arrays: it runs the forward recurrence chunk by chunk and, at
 // the end of a tile, the backward one, writing each cell's result as soon as
 // it is known; the consumers go on with the next tile meanwhile.  NX1: the
@@ -923,8 +922,6 @@ __global__ void __launch_bounds__(pt2::THREADS, 2)
                 mv = ((const float *)(st + O_MINV))[warp * TX + lane];
                 ccv = k > 1 ? cv[CC] : 0.0f;
             }
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&empty[s]); // this warp's reads of the stage are done
             if (ok && it >= NR && !tc::mbar_wait(&rempty[q], ((it / NR) - 1) & 1)) {
                 atomicExch(err, 1);
                 ok = false;
@@ -935,8 +932,14 @@ __global__ void __launch_bounds__(pt2::THREADS, 2)
             rs[(2 * KC + warp) * TX + lane] = cpv;
             rs[(3 * KC + warp) * TX + lane] = ccv;
             rs[(4 * KC + warp) * TX + lane] = mv;
+            // Both releases after the stores, which need every value read from the stage: with the stage
+            // released straight after its loads were issued, a copy could overwrite it under them where other
+            // kernels shared the SM (a row of 32 columns wrong in 7 of 2000 cycles; the same speed)
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&rfull[q]);
+            if (lane == 0) {
+                tc::mbar_arrive(&rfull[q]);
+                tc::mbar_arrive(&empty[s]);
+            }
         }
     }
 }
