@@ -580,8 +580,7 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
     const char *xb = reinterpret_cast<const char *>(a.x);
     const char *yb = reinterpret_cast<const char *>(a.dy);
 
-    // called by all lanes of warp 0.  Lines past the last block's end: the zero
-    // halo lines, so that the products of a short block's missing lines are zero.
+    // called by all lanes of warp 0; lines past the last block's end: the zero halo lines
     auto issue = [&](int tile, int s) {
         const int tx = tile % ntx, r = tile / ntx, k = r % dx.nz, j0 = r / dx.nz * TJ;
         const int lane = tid & 31;
@@ -602,7 +601,10 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
         }
     };
 
-    constexpr uint32_t IDESC = tc::idesc_bf16(128, C::N, 1, 1);
+    // dY lines of a tile: those past a short last block's end take no part, since zero
+    // times an infinite input of the last line is not zero
+    const int whole = ntx * dx.nz * (njb - 1), rest = dx.ny - (njb - 1) * TJ; // tiles of whole blocks, the last block's lines
+    auto lines = [&](int tile) { return tile < whole ? TJ : rest; };
     float db[COUT];
 #pragma unroll
     for (int c = 0; c < COUT; c++) db[c] = 0.0f;
@@ -618,6 +620,7 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
             tc::fence_after();
             const uint64_t a0 = tc::sdesc(tc::smem_u32(st), 128, LG);
             const uint64_t b0 = tc::sdesc(tc::smem_u32(st) + C::XR, 128, YG);
+            const uint32_t idesc = tc::idesc_bf16(128, 0, 1, 1) | ((uint32_t)(lines(tile) * COUT / 8) << 17);
 #pragma unroll
             for (int dil = 0; dil < 3; dil++)
 #pragma unroll
@@ -627,7 +630,7 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
                     for (int kc = 0; kc < TILE / 16; kc++) {
                         const uint64_t ad = a0 + (uint64_t)((mc * 16 * LG + dil * 16 + kc * 256) >> 4);
                         const uint64_t bd = b0 + (uint64_t)((kc * 256) >> 4);
-                        tc::mma_bf16(d, ad, bd, IDESC, (it > 0 || kc > 0) ? 1u : 0u);
+                        tc::mma_bf16(d, ad, bd, idesc, (it > 0 || kc > 0) ? 1u : 0u);
                     }
                 }
             tc::mma_commit(&bars[2 + s]);
@@ -654,10 +657,13 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(WgradArgs a)
     if (ok && it > 0) {
         tc::fence_after();
         // the products (input line l) x (dy line o) with l - o = dj + 1 belong to the tap dj: summed over o in
-        // shared memory, one o at a time (each sum is then touched by one thread), then added to the gradient
+        // shared memory, one o at a time (each sum is then touched by one thread), then added to the gradient;
+        // the tiles run up in j, so the CTA's first one has touched all lines that any has
         float *sum = reinterpret_cast<float *>(sm);
+        const int used = lines(blockIdx.x);
 #pragma unroll
         for (int o = 0; o < TJ; o++) {
+            if (o >= used) break;
             for (int dil = 0; dil < 3; dil++)
                 for (int mc = 0; mc < C::NMC; mc++)
 #pragma unroll

@@ -62,3 +62,31 @@ def test_weight_gradient_blocks_against_fp64(lib, cin, cout, nx, ny, nz, shift):
     assert float((got - ref).abs().max()) <= 1e-4 * max(float(ref.abs().max()), 1.0)
     rb = dy.sum((1, 2, 3))
     assert float((db.double().cpu() - rb).abs().max()) <= 1e-4 * float(rb.abs().max().clamp(min=1.0))
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 16)])
+@pytest.mark.parametrize("ny", [1, 2, 4, 5, 331])
+def test_weight_gradient_keeps_an_infinite_input_to_its_taps(lib, cin, cout, ny):
+    """An infinite input in the last line, where the blocks of dY lines have a
+    remainder: it enters no product of the taps dj = -1, whose dY line would be the one
+    after the last; those gradients are as without it (1e-4 of the largest value)."""
+    import ctypes as C
+    from hicar_b200 import _capi, learned as L
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    nx, nz = 40, 3
+    g = torch.Generator().manual_seed(ny)
+    bf = lambda t: t.to(torch.bfloat16).double()  # noqa: E731
+    x, dy = bf(torch.randn((cin, ny, nz, nx), generator=g)), bf(torch.randn((cout, ny, nz, nx), generator=g))
+    wt = torch.zeros((cout, cin, 3, 3, 3), dtype=torch.float64, requires_grad=True)
+    (F.conv3d(x[None], wt, padding=1)[0] * dy).sum().backward()
+    ref = wt.grad.permute(2, 3, 4, 1, 0).reshape(27, cin, cout)[:9]
+    x[3, ny - 1, 1, 7] = float("inf")
+    dw, db = torch.zeros(27 * cin * cout, device="cuda"), torch.zeros(cout, device="cuda")
+    xa, ya = L.to_act(x), L.to_act(dy)
+    rc = _capi.load().hicarw_nn_conv3_wgrad(cin, cout, nx, ny, nz, C.c_void_p(xa.data_ptr()), C.c_void_p(ya.data_ptr()),
+                                            C.c_void_p(dw.data_ptr()), C.c_void_p(db.data_ptr()), None)
+    assert rc == 0
+    got = dw.double().cpu().reshape(27, cin, cout)
+    assert float((got[:9] - ref).abs().max()) <= 1e-4 * max(float(ref.abs().max()), 1.0)
+    assert not bool(torch.isfinite(got[13, 3]).any())
