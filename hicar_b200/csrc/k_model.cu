@@ -243,7 +243,8 @@ void launch_probe_record(const Dims &d, const float *T, float *coef, int ca, int
 // share a face with the cell (the other 12 record a response of zero: no
 // leakage).  One thread evaluates the 15 responses of its cell with the
 // statements of winds_kernel and divergence_kernel, the unit point's place
-// known at compile time, terms of untouched faces (exact zeros) left out.
+// known at compile time.  The flux of an untouched face is not evaluated: it is
+// zero, or NaN where the face's geometry is zero, infinite or undefined (idle).
 // What bounds it: the divisions (24 face responses of 8 each), not memory; the
 // 27 probes it replaces wrote and read back lambda, the winds and the
 // divergence in full each time.  At 256x256x48 the entry point takes 0.55 ms
@@ -283,8 +284,8 @@ __device__ __forceinline__ float face_response(const Face &f, int rj1, int ri1, 
     return f.inner ? u * f.jac * (f.a + f.b) / 2.0f : u * f.jac * f.a;
 }
 
-__global__ void calibrate_kernel(Dims d, Metrics m, const float *__restrict__ alpha, const float *__restrict__ rho,
-                                 int adv_den, float *__restrict__ coef)
+__global__ void __launch_bounds__(128, 8) calibrate_kernel(Dims d, Metrics m, const float *__restrict__ alpha,
+                                                          const float *__restrict__ rho, int adv_den, float *__restrict__ coef)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, j = blockIdx.z + 1;
     if (i > d.nx) return;
@@ -342,11 +343,11 @@ __global__ void calibrate_kernel(Dims d, Metrics m, const float *__restrict__ al
         return adv_den ? w * jw * rho_w : w * jw;
     };
     // 2 T from the horizontal sum and the w fluxes of levels k and k - 1
-    auto store = [&](int slot, bool in, float sum, float wk, float wm) {
+    auto response = [&](float sum, float wk, float wm) {
         float dv = mxy * sum / d.dx;
         if (k == 1) dv = dv + wk / (adz);
         else dv = dv + (wk - wm) / (adz);
-        coef[(long long)slot * d.npad + kidx(d, i, k, j)] = in ? 2.0f * (dv / jac) : 0.0f;
+        return 2.0f * (dv / jac);
     };
 #define U1(DK, DJ, DI) face_response<DK, DJ, DI>(u1, 0, 1, 0, 0, k, nz, dzk1, dzke, den, d.dx, adv_den)
 #define U0(DK, DJ, DI) face_response<DK, DJ, DI>(u0, 0, 0, 0, -1, k, nz, dzk1, dzke, den, d.dx, adv_den)
@@ -358,23 +359,54 @@ __global__ void calibrate_kernel(Dims d, Metrics m, const float *__restrict__ al
     const float wk_m = up ? w_response(k, -1.0f) : 0.0f, wm_m = dn ? w_response(k - 1, -1.0f) : 0.0f;
 #define OWN(DK) \
     (U1(DK, 0, 0) / u1.mf - U0(DK, 0, 0) / u0.mf + V1(DK, 0, 0) / v1.mf - V0(DK, 0, 0) / v0.mf)
-    store(CA, true, OWN(0), wk_m, wm_p);
-    store(CB, up, OWN(1), wk_p, 0.0f);
-    store(CC, dn, OWN(-1), 0.0f, wm_m);
+    const float own = response(OWN(0), wk_m, wm_p);
+    // The fluxes of no correction: 0 / x is 0 unless x is 0 or NaN, 0 * x unless x is infinite or NaN.  Which of them
+    // are undefined, and their sum; none is where `own` is finite, which has them all but the top level's.
+    constexpr int FU0 = 1, FU1 = 2, FV0 = 4, FV1 = 8, FWK = 16, FWM = 32, FSUM = 64;
+    int undefined = 0;
+    if (k == nz || !(fabsf(own) < INFINITY)) {
+        auto divides = [](float x) { return fabsf(x) > 0.0f; };
+        auto multiplies = [](float x) { return fabsf(x) < INFINITY; };
+        auto face = [&](const Face &f) {
+            return multiplies(f.half_mf) && multiplies(f.slope) && divides(f.jac) && divides(f.rho) && divides(f.mf) &&
+                   divides(k == nz ? dzke : k == 1 ? dzk1 : den) &&
+                   (!adv_den || (multiplies(f.jac) && multiplies(f.inner ? f.a + f.b : f.a)));
+        };
+        auto level = [&](int kk) {
+            const long long q = cidx(d, i, kk, j);
+            const float a = alpha[q], jw = m.jw[q];
+            if (kk == nz) return multiplies(jw) && (!adv_den || multiplies(rho[q])); // no correction there
+            const float rho_w = w_density(kk);
+            return multiplies(0.5f * (a * a)) && divides(m.dz_if[zidx(d, i, kk + 1, j)]) && divides(jw) &&
+                   divides(rho_w) && multiplies(jw) && (!adv_den || multiplies(rho_w));
+        };
+        undefined = (face(u0) ? 0 : FU0) | (face(u1) ? 0 : FU1) | (face(v0) ? 0 : FV0) | (face(v1) ? 0 : FV1) |
+                    (level(k) ? 0 : FWK) | (k == 1 || level(k - 1) ? 0 : FWM) |
+                    (multiplies(mxy) && divides(adz) && divides(jac) ? 0 : FSUM);
+    }
+    // idle: the fluxes that the response leaves out; a neighbour outside the grid leaves out all
+    auto store = [&](int slot, bool in, int idle, float value) {
+        coef[(long long)slot * d.npad + kidx(d, i, k, j)] = undefined & (in ? idle : ~0) ? NAN : in ? value : 0.0f;
+    };
+    store(CA, true, up ? 0 : FWK, own);
+    store(CB, up, FWM, response(OWN(1), wk_p, 0.0f));
+    store(CC, dn, FWK, response(OWN(-1), 0.0f, wm_m));
     // the neighbouring columns: the face they share with the cell
     const bool e = i < d.nx, w = i > 1, n = j < d.ny, s = j > 1;
-    store(CD, e, U1(0, 0, 1) / u1.mf, 0.0f, 0.0f);
-    store(CE, w, -(U0(0, 0, -1) / u0.mf), 0.0f, 0.0f);
-    store(CF, n, V1(0, 1, 0) / v1.mf, 0.0f, 0.0f);
-    store(CG, s, -(V0(0, -1, 0) / v0.mf), 0.0f, 0.0f);
-    store(CH, e && up, U1(1, 0, 1) / u1.mf, 0.0f, 0.0f);
-    store(CI, w && up, -(U0(1, 0, -1) / u0.mf), 0.0f, 0.0f);
-    store(CJ, e && dn, U1(-1, 0, 1) / u1.mf, 0.0f, 0.0f);
-    store(CK, w && dn, -(U0(-1, 0, -1) / u0.mf), 0.0f, 0.0f);
-    store(CL, n && up, V1(1, 1, 0) / v1.mf, 0.0f, 0.0f);
-    store(CM, s && up, -(V0(1, -1, 0) / v0.mf), 0.0f, 0.0f);
-    store(CN, n && dn, V1(-1, 1, 0) / v1.mf, 0.0f, 0.0f);
-    store(CO, s && dn, -(V0(-1, -1, 0) / v0.mf), 0.0f, 0.0f);
+    constexpr int LW = FWK | FWM, LE = FU0 | FV0 | FV1 | LW, LWE = FU1 | FV0 | FV1 | LW, LN = FU0 | FU1 | FV0 | LW,
+                  LS = FU0 | FU1 | FV1 | LW;
+    store(CD, e, LE, response(U1(0, 0, 1) / u1.mf, 0.0f, 0.0f));
+    store(CE, w, LWE, response(-(U0(0, 0, -1) / u0.mf), 0.0f, 0.0f));
+    store(CF, n, LN, response(V1(0, 1, 0) / v1.mf, 0.0f, 0.0f));
+    store(CG, s, LS, response(-(V0(0, -1, 0) / v0.mf), 0.0f, 0.0f));
+    store(CH, e && up, LE, response(U1(1, 0, 1) / u1.mf, 0.0f, 0.0f));
+    store(CI, w && up, LWE, response(-(U0(1, 0, -1) / u0.mf), 0.0f, 0.0f));
+    store(CJ, e && dn, LE, response(U1(-1, 0, 1) / u1.mf, 0.0f, 0.0f));
+    store(CK, w && dn, LWE, response(-(U0(-1, 0, -1) / u0.mf), 0.0f, 0.0f));
+    store(CL, n && up, LN, response(V1(1, 1, 0) / v1.mf, 0.0f, 0.0f));
+    store(CM, s && up, LS, response(-(V0(1, -1, 0) / v0.mf), 0.0f, 0.0f));
+    store(CN, n && dn, LN, response(V1(-1, 1, 0) / v1.mf, 0.0f, 0.0f));
+    store(CO, s && dn, LS, response(-(V0(-1, -1, 0) / v0.mf), 0.0f, 0.0f));
 #undef OWN
 #undef U1
 #undef U0

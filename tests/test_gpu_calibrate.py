@@ -58,6 +58,32 @@ def test_one_pass_calibration_equals_the_probe_hooks(shape, adv):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("field", ["density", "alpha", "jacobian_u", "jacobian_v", "jacobian_w", "jacobian", "dzdx_u",
+                                   "dzdy_v", "advection_dz", "mapfac_mx_u", "mapfac_my_u", "mapfac_mx_v", "mapfac_mxy"])
+@pytest.mark.parametrize("adv", [True, False])
+def test_undefined_geometry_reaches_the_same_coefficients(field, adv):
+    """Zeros, infinities and NaN at a few places of one input field: the same finite, infinite and undefined
+    coefficients as the probe hooks record."""
+    from hicar_b200 import wind, wind_iterative as wi
+    from hicar_b200.domain import DeviceDomain
+    case = cases.build_case(13, 11, 7, seed=12, adv_den=adv, n_hills=3, alpha="smooth")
+    dom = DeviceDomain.from_case(case, "cuda")
+    a = dom.density if field == "density" else dom.wind_alpha if field == "alpha" else dom.metrics[field]
+    flat, rng = a.view(-1), np.random.default_rng(len(field))
+    for value in (0.0, float("inf"), float("-inf"), float("nan")):
+        flat[torch.from_numpy(rng.integers(0, flat.numel(), 2)).cuda()] = value
+    if a.dim() == 3:  # the lowest and the highest level too
+        a[3, 0, 5], a[7, -1, 4] = 0.0, float("nan")
+    opt = wi.WindOptions(advect_density=adv)
+    wi.init_iter_winds(dom, opt)
+    leak = wind.calibrate_projection_operator(dom, opt)
+    one = _coefs(dom, host=False)
+    div = torch.empty((dom.ny, dom.nz, dom.nx), dtype=torch.float32, device="cuda")
+    leak_hooks = wind.calibrate_projection_operator(dom, opt, div, on_device=False)
+    np.testing.assert_array_equal(one, _coefs(dom, host=False))
+    assert leak == leak_hooks
+
+
 @pytest.mark.parametrize("shape", [(3, 3, 2), (130, 5, 3)])
 @pytest.mark.parametrize("host", [True, False])
 def test_coefficients_round_trip(shape, host):
