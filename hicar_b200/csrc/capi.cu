@@ -1152,18 +1152,24 @@ extern "C" int hicarw_probe_record(hicarw_handle *h, const float *Tfield, int ca
     return HICARW_OK;
 }
 
-extern "C" int hicarw_probe_finalize(hicarw_handle *h, float max_leak, void *stream)
+// the probed coefficients are in place: from now on they are the operator
+static int use_probed(hicarw_handle *h, cudaStream_t s)
 {
-    api_entry();
-    if (!h) return HICARW_ERR_ARG;
     drop_graphs(h, !h->operator_probed);
     h->operator_probed = 1;
     h->structure_uploaded = 1;
     h->mg_dirty = h->unet_dirty = 1;
+    return zero_solution(h, s); // :1243
+}
+
+extern "C" int hicarw_probe_finalize(hicarw_handle *h, float max_leak, void *stream)
+{
+    api_entry();
+    if (!h) return HICARW_ERR_ARG;
     if (h->opt.verbose)
         fprintf(stderr, "Projection operator calibrated by probing (A = 2*D o G); off-stencil leakage max |T| = %g\n",
                 (double)max_leak);
-    return zero_solution(h, (cudaStream_t)stream); // :1243
+    return use_probed(h, (cudaStream_t)stream);
 }
 
 extern "C" int hicarw_calibrate_projection_operator(hicarw_handle *h, const float *alpha, const float *density,
@@ -1188,10 +1194,11 @@ extern "C" int hicarw_calibrate_projection_operator(hicarw_handle *h, const floa
     launch_calibrate(d, metrics_of(h), h->alpha, rho, adv_den, h->coef, s);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
-    const float leak = 0.0f; // only stencil neighbours share a face with a cell
-    if (max_leak) *max_leak = leak;
+    if (max_leak) *max_leak = 0.0f; // no probe point off a cell's stencil shares a face with it
     (void)u; (void)v; (void)w;
-    return hicarw_probe_finalize(h, leak, stream);
+    if (h->opt.verbose)
+        fprintf(stderr, "Projection operator calibrated (A = 2*D o G, the responses of all probes in one pass)\n");
+    return use_probed(h, s);
 }
 
 // ---- extensions ----------------------------------------------------------

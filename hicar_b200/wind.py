@@ -31,9 +31,11 @@ def calibrate_projection_operator(domain: DeviceDomain, options: wi.WindOptions,
                                   on_device: bool = True) -> float:
     """Calibrate A = 2 D o G by the 27-colouring probe (wind.F90:1010-1099).
 
-    on_device=True runs all 27 probes inside the library (no host round trip);
+    on_device=True evaluates the responses of all 27 probes in one pass inside the
+    library (no host round trip; the leakage returned is 0 by construction);
     on_device=False drives the reference's probe hooks one by one, exactly as
-    wind.F90:1055-1067 does (``div`` is the probe's scratch divergence)."""
+    wind.F90:1055-1067 does, and measures the leakage (``div`` is the probe's
+    scratch divergence)."""
     lib = _capi.load()
     h = wi.handle(domain.nest_indx)
     adv = bool(options.advect_density)

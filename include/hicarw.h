@@ -209,8 +209,10 @@ int hicarw_probe_record(hicarw_handle *h, const float *Tfield, int ca, int cb, i
 int hicarw_probe_finalize(hicarw_handle *h, float max_leak, void *stream);                              /* :1235-1248 */
 
 /* calibrate_projection_operator(domain, options, div)  (wind.F90:1010-1099):
- * all 27 probes on the device, no host round trip; u, v, w are used as scratch
- * and restored, as the reference does. */
+ * the responses of all 27 probes in one pass on the device, no host round trip;
+ * u, v, w, in which the reference probes and which it restores, are not touched.
+ * *max_leak (optional) is 0: no probe point off a cell's stencil shares a face with
+ * it.  The probe hooks above measure the leakage. */
 int hicarw_calibrate_projection_operator(hicarw_handle *h, const float *alpha, const float *density,
                                          int adv_den, float *u, float *v, float *w, float *max_leak,
                                          int mem_kind, void *stream);

@@ -39,7 +39,7 @@ def _coefs(dom, host):
 # smallest extents (every face an outer one, nz = 2: no inner level), block edges, odd sizes
 @pytest.mark.parametrize("shape", [(3, 3, 2), (4, 5, 3), (129, 4, 2), (128, 7, 5), (37, 41, 9)])
 @pytest.mark.parametrize("adv", [True, False])
-def test_one_pass_calibration_equals_the_probe_hooks(shape, adv):
+def test_one_pass_calibration_equals_the_probe_hooks(shape, adv, capfd):
     from hicar_b200 import wind, wind_iterative as wi
     from hicar_b200.domain import DeviceDomain
     case = cases.build_case(*shape, seed=11, adv_den=adv, n_hills=3, alpha="smooth")
@@ -47,11 +47,13 @@ def test_one_pass_calibration_equals_the_probe_hooks(shape, adv):
     opt = wi.WindOptions(advect_density=adv)
     wi.init_iter_winds(dom, opt)
     leak = wind.calibrate_projection_operator(dom, opt)
+    assert "leakage" not in capfd.readouterr().err  # none is measured
     one = _coefs(dom, host=False)
     np.testing.assert_array_equal(one, _coefs(dom, host=True))
     winds = [a.clone() for a in (dom.u_dqdt, dom.v_dqdt, dom.w_dqdt)]
     div = torch.empty((dom.ny, dom.nz, dom.nx), dtype=torch.float32, device="cuda")
     leak_hooks = wind.calibrate_projection_operator(dom, opt, div, on_device=False)
+    assert "leakage max |T| = 0" in capfd.readouterr().err
     np.testing.assert_array_equal(one, _coefs(dom, host=False))
     assert leak == leak_hooks
     for a, b in zip(winds, (dom.u_dqdt, dom.v_dqdt, dom.w_dqdt)):

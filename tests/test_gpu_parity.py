@@ -97,11 +97,13 @@ def test_analytic_and_probed_coefs_bitexact(oracle_mod, case64):
     s = oracle_mod.OracleSolver(case64.domain)
     s.build_analytic(case64.alpha)
     assert np.array_equal(_coefs(dom), s.coefs())
-    leak = wind.calibrate_projection_operator(dom, opt, div)
     u, v, w = (np.ascontiguousarray(a).copy() for a in (case64.u, case64.v, case64.w))
     leak_ref = s.calibrate(True, u, v, w)
-    assert leak == leak_ref == 0.0
-    assert np.array_equal(_coefs(dom), s.coefs())
+    # the probe hooks one by one, which measure the leakage, and all probes in one pass
+    for on_device in (False, True):
+        leak = wind.calibrate_projection_operator(dom, opt, div, on_device=on_device)
+        assert leak == leak_ref == 0.0
+        assert np.array_equal(_coefs(dom), s.coefs())
 
 
 def test_probe_hooks_match_device_calibration(case64):
