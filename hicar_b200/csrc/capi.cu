@@ -1202,9 +1202,24 @@ extern "C" int hicarw_calibrate_projection_operator(hicarw_handle *h, const floa
 }
 
 // ---- extensions ----------------------------------------------------------
+// Whether a kernel may take a caller's device array as it is: aligned to its
+// elements and in this device's memory.  The copy calls take any address, another
+// device's memory too, so arrays of other kinds go through them.
+static bool kernel_takes(const void *p, size_t align)
+{
+    cudaPointerAttributes a;
+    int dev = -1;
+    if ((uintptr_t)p % align != 0) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeDevice && a.device == dev);
+}
+
 // The 15 coefficient arrays between the padded layout and the caller's
 // (15, ny, nz, nx): device arrays by one kernel (coalesced along i), host arrays
-// by one strided copy per coefficient.
+// and arrays that a kernel does not take by one strided copy per coefficient.
 __global__ void coefs_copy_kernel(Dims d, float *__restrict__ coef, float *__restrict__ user, int to_user)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, j = blockIdx.z + 1;
@@ -1220,7 +1235,8 @@ __global__ void coefs_copy_kernel(Dims d, float *__restrict__ coef, float *__res
 static int copy_coefs(hicarw_handle *h, float *user, int to_user, int mem_kind, cudaStream_t s)
 {
     const Dims &d = h->d;
-    if (mem_kind != HICARW_MEM_HOST) {
+    const bool host = mem_kind == HICARW_MEM_HOST;
+    if (!host && kernel_takes(user, sizeof(float))) {
         coefs_copy_kernel<<<dim3((d.nx + 127) / 128, d.nz, d.ny), 128, 0, s>>>(d, h->coef, user, to_user);
         count_launch(1);
         CK(cudaGetLastError());
@@ -1233,7 +1249,7 @@ static int copy_coefs(hicarw_handle *h, float *user, int to_user, int mem_kind, 
             p.srcPtr = to_user ? pad : usr;
             p.dstPtr = to_user ? usr : pad;
             p.extent = make_cudaExtent(sizeof(float) * d.nx, d.nz, d.ny);
-            p.kind = to_user ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+            p.kind = !host ? cudaMemcpyDeviceToDevice : to_user ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
             CK(cudaMemcpy3DAsync(&p, s));
         }
     }
@@ -1263,7 +1279,7 @@ extern "C" int hicarw_set_coefs(hicarw_handle *h, const float *coefs, int probed
 
 // A (nx+2, nz+2, ny+2) FP64 array of the caller into / out of a padded device
 // vector (its padding is not touched): device arrays by one kernel, host arrays
-// by a strided copy.
+// and arrays that a kernel does not take by a strided copy.
 __global__ void rows_copy_kernel(Dims d, const double *__restrict__ in, double *__restrict__ out, int to_padded)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y, j = blockIdx.z;
@@ -1284,17 +1300,19 @@ static int rows_copy(hicarw_handle *h, const double *in, double *out, int to_pad
 static int put_padded(hicarw_handle *h, const double *src, double *dst, int mem_kind, cudaStream_t s)
 {
     const Dims &d = h->d;
-    if (mem_kind != HICARW_MEM_HOST) return rows_copy(h, src, dst, 1, s);
+    const bool host = mem_kind == HICARW_MEM_HOST;
+    if (!host && kernel_takes(src, sizeof(double))) return rows_copy(h, src, dst, 1, s);
     CK(cudaMemcpy2DAsync(dst + XO, sizeof(double) * d.P, src, sizeof(double) * d.mx, sizeof(double) * d.mx,
-                         (size_t)d.mz * d.my, cudaMemcpyHostToDevice, s));
+                         (size_t)d.mz * d.my, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s));
     return 0;
 }
 static int get_padded(hicarw_handle *h, const double *src, double *dst, int mem_kind, cudaStream_t s)
 {
     const Dims &d = h->d;
-    if (mem_kind != HICARW_MEM_HOST) return rows_copy(h, src, dst, 0, s);
+    const bool host = mem_kind == HICARW_MEM_HOST;
+    if (!host && kernel_takes(dst, sizeof(double))) return rows_copy(h, src, dst, 0, s);
     CK(cudaMemcpy2DAsync(dst, sizeof(double) * d.mx, src + XO, sizeof(double) * d.P, sizeof(double) * d.mx,
-                         (size_t)d.mz * d.my, cudaMemcpyDeviceToHost, s));
+                         (size_t)d.mz * d.my, host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, s));
     return 0;
 }
 

@@ -102,3 +102,60 @@ def test_coefficients_round_trip(shape, host):
     _capi.check(lib.hicarw_set_coefs(h, C.c_void_p(src), 1, _capi.MEM_HOST if host else _capi.MEM_DEVICE, None), h)
     np.testing.assert_array_equal(_coefs(dom, host=True), a)
     np.testing.assert_array_equal(_coefs(dom, host=False), a)
+
+
+@pytest.mark.parametrize("shift", [1, 4])
+def test_copies_take_device_arrays_of_any_alignment(shift):
+    """Coefficients, vectors and lambda in device arrays that start `shift` bytes past an aligned address: as from
+    aligned ones."""
+    from hicar_b200 import wind, wind_iterative as wi
+    from hicar_b200.domain import DeviceDomain
+    case = cases.build_case(13, 9, 5, seed=4, adv_den=True, n_hills=3)
+    dom = DeviceDomain.from_case(case, "cuda")
+    wi.init_iter_winds(dom, wi.WindOptions(tol_rel=1e-8))
+    wind.calibrate_projection_operator(dom, wi.WindOptions())
+    h, lib = wi.handle(dom.nest_indx), _capi.load()
+
+    def shifted(like, fill):
+        raw = torch.zeros(like.numel() * like.element_size() + 16, dtype=torch.uint8, device="cuda")
+        part = raw[shift:shift + like.numel() * like.element_size()]
+        if fill:
+            part.copy_(like.reshape(-1).view(torch.uint8))
+        return part, C.c_void_p(part.data_ptr())
+
+    def call(name, *a):
+        rc = getattr(lib, name)(h, *a)
+        assert rc >= 0, lib.hicarw_last_error(h)
+
+    dev, rng = _capi.MEM_DEVICE, np.random.default_rng(9)
+    x = torch.from_numpy(rng.standard_normal((dom.ny + 2, dom.nz + 2, dom.nx + 2))).cuda()
+    xs, xp = shifted(x, True)
+    for sweeps in (None, 0, 2):
+        y = torch.empty_like(x)
+        ys, yp = shifted(y, False)
+        for src, dst in ((C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr())), (xp, yp)):
+            if sweeps is None:
+                call("hicarw_apply_operator", src, dst, dev, None)
+            else:
+                call("hicarw_apply_precond", src, dst, sweeps, dev, None)
+        assert torch.equal(ys, y.reshape(-1).view(torch.uint8))
+    lam, st = [], _capi.Stats()
+    for src, out in ((C.c_void_p(x.data_ptr()), torch.empty_like(x)), (xp, None)):
+        call("hicarw_reset_solution", None)
+        call("hicarw_solve_rhs", src, dev, None, C.byref(st))
+        if out is None:
+            part, op = shifted(x, False)
+            call("hicarw_get_lambda", op, dev, None)
+            lam.append(part)
+        else:
+            call("hicarw_get_lambda", C.c_void_p(out.data_ptr()), dev, None)
+            lam.append(out.reshape(-1).view(torch.uint8))
+    assert torch.equal(*lam)
+    coefs = torch.from_numpy(_coefs(dom, host=True)).cuda()
+    part, p = shifted(coefs, False)
+    call("hicarw_get_coefs", p, dev, None)
+    assert torch.equal(part, coefs.reshape(-1).view(torch.uint8))
+    other = coefs * 2
+    part, p = shifted(other, True)
+    call("hicarw_set_coefs", p, 1, dev, None)
+    np.testing.assert_array_equal(_coefs(dom, host=True), other.cpu().numpy())
