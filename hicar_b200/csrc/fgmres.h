@@ -38,7 +38,7 @@ struct FgmresCtx {
     void *pctx;
 };
 
-bool fgmres_init(); // once before the first launch (false: an attribute was refused)
+bool fgmres_init(); // before the launches of a solve, outside any capture (false: an attribute was refused)
 void fgmres_reset(GmresState *g, int m, double tol_rel, double tol_abs, int max_iters, double *hist, SolveState *mirror,
                   cudaStream_t s);
 void fgmres_set_profile(GmresState *g, int on, cudaStream_t s);

@@ -307,12 +307,12 @@ static int ew_blocks(long long n)
     return (int)(b < 148 * 8 ? b : 148 * 8);
 }
 
-// Attributes of the kernels, set outside any stream capture.
+// Attributes of the kernels, set outside any stream capture, for the current
+// device at each solve (a process may solve on several).
 bool fgmres_init()
 {
-    static const bool ok = cudaFuncSetAttribute(fgmres_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (FG_MAXM + 1) * FGT * (int)sizeof(double)) == cudaSuccess;
-    return ok;
+    return cudaFuncSetAttribute(fgmres_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (FG_MAXM + 1) * FGT * (int)sizeof(double)) == cudaSuccess;
 }
 
 void fgmres_reset(GmresState *g, int m, double tol_rel, double tol_abs, int max_iters, double *hist, SolveState *mirror,

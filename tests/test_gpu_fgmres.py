@@ -122,3 +122,48 @@ def test_fgmres_mg_iterations_and_restart_history(case):
     _capi.load().hicarw_get_history(h, hist.ctypes.data, n)
     assert hist[0] == pytest.approx(st_m["res0"])
     assert np.all(hist[1:] <= hist[:-1] * (1 + 1e-6))
+
+
+def test_long_restart_in_a_second_context(lib):
+    """A restart of 30 needs more than 48 KB of shared memory in the projection kernel, an attribute of the context
+    (a process's second device has one of its own): a solve in a second context equals that in the first."""
+    import ctypes as C
+    from hicar_b200.wind_iterative import WindOptions
+    lib = _capi.load()
+    nx, ny, nz = 24, 20, 12
+    case = cases.build_case(nx, ny, nz, seed=8, adv_den=True, n_hills=3)
+    d, keep = case.domain, []
+
+    def host(a):
+        keep.append(np.ascontiguousarray(a, np.float32))
+        return keep[-1].ctypes.data
+
+    def solve():
+        opt = WindOptions(windtype=0, tol_rel=1e-9, wind_solver_iterations=500, solver=_capi.SOLVER_FGMRES,
+                          precond=_capi.PRECOND_JACOBI, fgmres_restart=30).to_c()
+        g, h, leak, st = _capi.Grid(nx, ny, nz, d.dx, 1), C.c_void_p(), C.c_float(), _capi.Stats()
+        m = _capi.Metrics(*[host(getattr(d, n)) for n in _capi.METRIC_FIELDS])
+        _capi.check(lib.hicarw_init_iter_winds(C.byref(g), C.byref(opt), C.byref(m), _capi.MEM_HOST, None, C.byref(h)))
+        try:
+            _capi.check(lib.hicarw_calibrate_projection_operator(
+                h, host(case.alpha), host(d.density), 1, host(case.u), host(case.v), host(case.w), C.byref(leak),
+                _capi.MEM_HOST, None), h)
+            x = np.random.default_rng(1).standard_normal((ny + 2, nz + 2, nx + 2))
+            y = np.empty_like(x)
+            _capi.check(lib.hicarw_solve_rhs(h, x.ctypes.data, _capi.MEM_HOST, None, C.byref(st)), h)
+            _capi.check(lib.hicarw_get_lambda(h, y.ctypes.data, _capi.MEM_HOST, None), h)
+            return st.status, st.iterations, y
+        finally:
+            lib.hicarw_finalize_iter_winds(h)
+
+    first = solve()
+    assert first[0] == 0 and first[1] > 30
+    cu, ctx, old = C.CDLL("libcuda.so.1"), C.c_void_p(), C.c_void_p()
+    torch.cuda.synchronize()
+    assert cu.cuCtxGetCurrent(C.byref(old)) == 0 and cu.cuCtxCreate_v2(C.byref(ctx), 0, torch.cuda.current_device()) == 0
+    try:
+        second = solve()
+    finally:
+        cu.cuCtxDestroy_v2(ctx)
+        cu.cuCtxSetCurrent(old)
+    assert second[:2] == first[:2] and np.array_equal(second[2], first[2])
