@@ -137,11 +137,10 @@ def _timed_solve(wi, step, kw):
 def pick_cycle(wi, step, base: dict):
     """Two solves of the workload with each cycle of MG_CYCLES (the second one
     timed), then the fastest of them once more with FP32 Krylov vectors and
-    FP64 lambda, the faster of those with the finest level's smoother
-    coefficients in BF16 (cycles without fine pre-smoothing), and the fastest
-    so far with graphs of 4 iterations.  Returns
+    FP64 lambda, and the faster of those with the finest level's smoother
+    coefficients in BF16 (cycles without fine pre-smoothing).  Returns
     the options of the fastest candidate that converged with the multigrid
-    preconditioner (no fallback) and, for the FP32-vector one, whose FP64 true
+    preconditioner (no fallback) and, for the last two, whose FP64 true
     residual meets the tolerance; its name; and the table of times (ms; None
     for a candidate that was not accepted)."""
     table = {}
@@ -153,18 +152,14 @@ def pick_cycle(wi, step, base: dict):
     kw = {**base, **MG_CYCLES[best]}
     if good:
         best_ms = table[best]
-        # the same cycle with FP32 Krylov vectors and FP64 lambda, then with
-        # graphs of 4 iterations (fewer launched past convergence when few are needed)
-        trials = [("f32-vectors", {"krylov_precision": KRYLOV_F32_X64}, True)]
+        # the same cycle with FP32 Krylov vectors and FP64 lambda
+        trials = [("f32-vectors", {"krylov_precision": KRYLOV_F32_X64})]
         if kw.get("mg_skip_fine_presmooth"):  # BF16 coefficients of the finest level's post-smoother
-            trials.append(("bf16-smoother", {"mg_precision": 1}, True))
-        trials.append(("chunk4", {"check_every": 4}, False))
-        for tag, extra, accurate in trials:
+            trials.append(("bf16-smoother", {"mg_precision": 1}))
+        for tag, extra in trials:
             trial = {**kw, **extra}
             ms, st = _timed_solve(wi, step, trial)
-            ok = st["status"] == 0 and st["precond"] == 1
-            if accurate:
-                ok = ok and 0.0 <= st["true_res"] <= 1.01 * st["target"]
+            ok = st["status"] == 0 and st["precond"] == 1 and 0.0 <= st["true_res"] <= 1.01 * st["target"]
             table[best + "/" + tag] = ms if ok else None
             if ok and ms < best_ms:
                 best, kw, best_ms = best + "/" + tag, trial, ms
@@ -209,6 +204,34 @@ def solver_kwargs(name: str) -> dict:
 def solver_options(name: str):
     from hicar_b200 import wind_iterative as wi
     return wi.WindOptions(**solver_kwargs(name))
+
+
+# parts of the line that are tables or say at length what other keys say: in the file of the whole line only
+LONG_PARTS = (("roofline", "kernels"), ("config", "accuracy"), ("config", "learned_fgmres"),
+              ("config", "mg_cycle", "warmup_solve_ms"), ("config", "kernel_autotune"), ("batch96", "config"))
+
+
+def print_line(line: dict) -> None:
+    """The bench line on stdout, short enough to be read from the end of a log: without the long parts and
+    with seven digits.  build/bench_line.json (config.whole_line) holds it whole."""
+    path = os.path.join("build", "bench_line.json")
+    try:
+        os.makedirs(os.path.join(ROOT, "build"), exist_ok=True)
+        with open(os.path.join(ROOT, path), "w") as f:
+            json.dump(line, f, indent=1)
+    except OSError:
+        path = None
+
+    def short(x, at=()):
+        if isinstance(x, dict):
+            return {k: short(v, at + (k,)) for k, v in x.items() if at + (k,) not in LONG_PARTS}
+        if isinstance(x, (list, tuple)):
+            return [short(v, at) for v in x]
+        return float("%.7g" % x) if isinstance(x, float) else x
+
+    out = short(line)
+    out["config"]["whole_line"] = path
+    print(json.dumps(out), flush=True)
 
 
 class ClockSampler:
@@ -932,7 +955,7 @@ def run_ours(args, wl):
         line["batch96"] = {k: b[k] for k in ("value", "ms_per_step", "steps", "warmup", "config", "e2e", "clocks",
                                              "gpu_launches")}
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print_line(line)
     if dist:
         dist.barrier()
         dist.destroy_process_group()
@@ -1095,7 +1118,7 @@ def run_batch(args, wl):
         dist.init_process_group("nccl", timeout=datetime.timedelta(seconds=600))
     line = batch_measure(args, wl, rank, world, dist, local)
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print_line(line)
     if dist:
         dist.barrier()
         dist.destroy_process_group()

@@ -88,7 +88,7 @@ def test_no_candidate_converges(monkeypatch):
     assert opt.mg_w_levels == () and not opt.mg_skip_fine_presmooth
 
 
-def test_shorter_graphs_kept_when_faster(monkeypatch):
+def test_bf16_smoother_kept_when_faster(monkeypatch):
     import bench
     wi, applied = _setup(monkeypatch)
     inner = _fake_step(applied, 0.9, 9.5e-7)
@@ -96,11 +96,31 @@ def test_shorter_graphs_kept_when_faster(monkeypatch):
     def step():
         t0 = _Event.clock[0]
         st = inner()
-        if applied[-1].check_every == 4:        # fewer iterations launched past convergence
+        if applied[-1].mg_precision == 1:       # half the bytes of the finest level's coefficients
             _Event.clock[0] = t0 + 0.95 * (_Event.clock[0] - t0)
         return st
 
     opt, name, table = bench.pick_cycle(wi, step, bench.solver_kwargs("mg"))
-    assert name == "V01-W23/f32-vectors/chunk4"
-    assert opt.check_every == 4 and opt.krylov_precision == 2 and opt.mg_w_levels == (2, 3)
+    assert name == "V01-W23/f32-vectors/bf16-smoother"
+    assert opt.mg_precision == 1 and opt.krylov_precision == 2 and opt.mg_w_levels == (2, 3)
     assert table[name] < table["V01-W23/f32-vectors"] < table["V01-W23"]
+    assert set(table) == set(bench.MG_CYCLES) | {"V01-W23/f32-vectors", name}  # every trial can change the solve
+
+
+def test_line_is_short_and_its_tables_go_to_a_file(monkeypatch, tmp_path, capsys):
+    import json
+
+    import bench
+    monkeypatch.setattr(bench, "ROOT", str(tmp_path))
+    table = [{"bucket": {"nz": 20}, "tried": {"16/1": 1.23456789012}}] * 200
+    line = {"metric": "m", "value": 11.264580477912752, "steps": 20, "higher_is_better": True, "vs_baseline": None,
+            "config": {"workload": "w", "accuracy": {"x": 1.0}, "learned_fgmres": {}, "kernel_autotune": table,
+                       "mg_cycle": {"chosen": "V01", "warmup_solve_ms": {"V01": 1.5}}},
+            "roofline": {"kernel": "k", "frac": 0.8795682911123339, "kernels": table},
+            "batch96": {"value": 106.3, "config": {"kernel_autotune": table}}}
+    bench.print_line(line)
+    out = json.loads(capsys.readouterr().out)
+    assert out == {"metric": "m", "value": 11.26458, "steps": 20, "higher_is_better": True, "vs_baseline": None,
+                   "config": {"workload": "w", "mg_cycle": {"chosen": "V01"}, "whole_line": "build/bench_line.json"},
+                   "roofline": {"kernel": "k", "frac": 0.8795683}, "batch96": {"value": 106.3}}
+    assert json.loads((tmp_path / "build" / "bench_line.json").read_text()) == line
