@@ -17,7 +17,8 @@
 // What bounds it: an MMA with N <= 64 takes as long as reading its A operand (4
 // KB), so the taps are merged in N (13.5 MMAs per 128-cell tile and 16 input
 // channels instead of 27), and a line is fetched 1.5 times instead of 9.  B200,
-// 16 -> 16 channels at 512x512x48: 0.84 -> 0.34 ms; 32 -> 32 at 64x64x48: 91 -> 46 us.
+// 32 -> 32 channels at 64x64x48: 91 -> 46 us.  Convolutions to 16 channels merge
+// all nine taps of a line (conv3_fwd9_kernel).
 //
 // Weight gradient: dW_tap[CIN x COUT] = sum over cells of X(v + tap)^T dY(v):
 // the reduction runs over cells (the MMA's K), both operands MN-major straight
@@ -86,11 +87,11 @@ struct FwdCfg {
     static constexpr int SLOTS = 4;                 // accumulator levels: three in the making, one in the epilogue
     static constexpr int WB = 27 * GI * COUT * 16;  // weight image bytes
     static constexpr int STAGE = NL * GI * SG;      // one input level's line images
-    static constexpr int NCOL = SLOTS * TJ * COUT;  // 256 or 512
+    static constexpr int NCOL = SLOTS * TJ * COUT;  // all of the tensor memory
     static constexpr int NS = 3;                    // input levels in flight
     static constexpr int SMEM = up128(WB) + NS * STAGE + 256;
-    static constexpr int PER_SM = NCOL <= 256 && SMEM <= 113 * 1024 ? 2 : 1;
-    static_assert(CIN % 16 == 0 && COUT % 16 == 0 && NCOL <= 512 && 3 * COUT <= 256, "channel counts");
+    static constexpr int PER_SM = 1;
+    static_assert(CIN % 16 == 0 && COUT == 32 && NCOL == 512 && 3 * COUT <= 256, "channel counts");
     static_assert(SMEM <= 232448, "shared memory");
 };
 
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__(CONV_THREADS) conv3_fwd_kernel(ConvArgs a, Con
 // products, which the CTA next to it on the SM covers.  Levels outside the block
 // that a block's first and last input levels also feed are zeroed without being
 // stored.
-// 16 -> 16 at 512x512x48 (B200): 0.342 -> 0.183 ms (0.68 of measured HBM, 0.57 of
+// 16 -> 16 at 512x512x48 (B200), against the three-tap form above: 0.342 -> 0.183 ms (0.68 of measured HBM, 0.57 of
 // measured BF16); 32 -> 16 at 256x256x48: 0.093 ms.
 // ---------------------------------------------------------------------------
 template <int CIN>

@@ -1457,7 +1457,7 @@ __global__ void __launch_bounds__(MG_FUSE_THREADS) coarse_cycle_kernel(const __g
 // ---------------------------------------------------------------------------
 // Dense coarse cycle.  From a level of a few thousand unknowns down, the
 // cycle (its pre-smoothing, W repeats and post-smoothings included) is a fixed
-// linear map of that level's right-hand side, so the build tabulates it as one
+// linear map of that level's right-hand side, so it is tabulated as one
 // n x n matrix and a visit is one matrix-vector product: two short launches
 // (restriction, product) in the place of a chain of 8 to 44 dependent steps on
 // levels too small to hide a memory latency.  The columns are the cycle applied

@@ -219,6 +219,14 @@ int hicarw_calibrate_projection_operator(hicarw_handle *h, const float *alpha, c
 
 /* ---- extensions with no entry point of their own in the reference ---- */
 
+/* Device memory: what a call allocates stays with the handle until
+ * hicarw_finalize_iter_winds.  Beside the fields and the Krylov vectors: with the
+ * V-cycle its levels and, from the first solve on, the coarse matrix (n^2 FP32
+ * values of a level of n <= 3072 unknowns, 4096 where it corrects twice: up to 64
+ * MB a handle); with apply_operator two padded FP64 vectors, apply_precond two, or
+ * four with sweeps >= 1, solve_rhs one with FP32 Krylov vectors (four at most
+ * together; 0.56 GB each at 1024x1024x64). */
+
 /* Reset the warm-start lambda (x_sol) to zero, as probe_finalize does (:1243). */
 int hicarw_reset_solution(hicarw_handle *h, void *stream);
 
