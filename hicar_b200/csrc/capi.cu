@@ -1217,19 +1217,26 @@ static bool kernel_takes(const void *p, size_t align)
     return a.type == cudaMemoryTypeManaged || (a.type == cudaMemoryTypeDevice && a.device == dev);
 }
 
+// Rows of 128 columns over levels and lines, as many of each as a grid may have.
+static dim3 copy_grid(int nx, int nz, int ny) { return dim3((nx + 127) / 128, std::min(nz, 65535), std::min(ny, 65535)); }
+
 // The 15 coefficient arrays between the padded layout and the caller's
 // (15, ny, nz, nx): device arrays by one kernel (coalesced along i), host arrays
 // and arrays that a kernel does not take by one strided copy per coefficient.
 __global__ void coefs_copy_kernel(Dims d, float *__restrict__ coef, float *__restrict__ user, int to_user)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, k = blockIdx.y + 1, j = blockIdx.z + 1;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (i > d.nx) return;
-    const long long n = (long long)d.nx * d.nz * d.ny, o = kidx(d, i, k, j), c = cidx(d, i, k, j);
-    float v[NCOEF];
+    const long long n = (long long)d.nx * d.nz * d.ny;
+    for (int j = blockIdx.z + 1; j <= d.ny; j += gridDim.z)
+        for (int k = blockIdx.y + 1; k <= d.nz; k += gridDim.y) {
+            const long long o = kidx(d, i, k, j), c = cidx(d, i, k, j);
+            float v[NCOEF];
 #pragma unroll
-    for (int q = 0; q < NCOEF; q++) v[q] = to_user ? coef[q * d.npad + o] : user[q * n + c];
+            for (int q = 0; q < NCOEF; q++) v[q] = to_user ? coef[q * d.npad + o] : user[q * n + c];
 #pragma unroll
-    for (int q = 0; q < NCOEF; q++) (to_user ? user[q * n + c] : coef[q * d.npad + o]) = v[q];
+            for (int q = 0; q < NCOEF; q++) (to_user ? user[q * n + c] : coef[q * d.npad + o]) = v[q];
+        }
 }
 
 static int copy_coefs(hicarw_handle *h, float *user, int to_user, int mem_kind, cudaStream_t s)
@@ -1237,7 +1244,7 @@ static int copy_coefs(hicarw_handle *h, float *user, int to_user, int mem_kind, 
     const Dims &d = h->d;
     const bool host = mem_kind == HICARW_MEM_HOST;
     if (!host && kernel_takes(user, sizeof(float))) {
-        coefs_copy_kernel<<<dim3((d.nx + 127) / 128, d.nz, d.ny), 128, 0, s>>>(d, h->coef, user, to_user);
+        coefs_copy_kernel<<<copy_grid(d.nx, d.nz, d.ny), 128, 0, s>>>(d, h->coef, user, to_user);
         count_launch(1);
         CK(cudaGetLastError());
     } else {
@@ -1282,17 +1289,20 @@ extern "C" int hicarw_set_coefs(hicarw_handle *h, const float *coefs, int probed
 // and arrays that a kernel does not take by a strided copy.
 __global__ void rows_copy_kernel(Dims d, const double *__restrict__ in, double *__restrict__ out, int to_padded)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y, j = blockIdx.z;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.mx) return;
-    const long long o = kidx(d, i, k, j), c = ((long long)j * d.mz + k) * d.mx + i;
-    if (to_padded) out[o] = in[c];
-    else out[c] = in[o];
+    for (int j = blockIdx.z; j < d.my; j += gridDim.z)
+        for (int k = blockIdx.y; k < d.mz; k += gridDim.y) {
+            const long long o = kidx(d, i, k, j), c = ((long long)j * d.mz + k) * d.mx + i;
+            if (to_padded) out[o] = in[c];
+            else out[c] = in[o];
+        }
 }
 
 static int rows_copy(hicarw_handle *h, const double *in, double *out, int to_padded, cudaStream_t s)
 {
     const Dims &d = h->d;
-    rows_copy_kernel<<<dim3((d.mx + 127) / 128, d.mz, d.my), 128, 0, s>>>(d, in, out, to_padded);
+    rows_copy_kernel<<<copy_grid(d.mx, d.mz, d.my), 128, 0, s>>>(d, in, out, to_padded);
     count_launch(1);
     CK(cudaGetLastError());
     return 0;

@@ -159,3 +159,34 @@ def test_copies_take_device_arrays_of_any_alignment(shift):
     part, p = shifted(other, True)
     call("hicarw_set_coefs", p, 1, dev, None)
     np.testing.assert_array_equal(_coefs(dom, host=True), other.cpu().numpy())
+
+
+@pytest.mark.parametrize("ny", [65533, 65535])
+def test_copies_of_as_many_lines_as_a_grid_has(ny):
+    """Lambda, vectors and coefficients of the longest domain that a handle can be made for: with its two ghost lines
+    it has more than 65535."""
+    from hicar_b200 import wind_iterative as wi
+    nx, nz, lib, dev = 3, 2, _capi.load(), _capi.MEM_DEVICE
+    ones = lambda *s: torch.ones(s, device="cuda")  # noqa: E731
+    shape = {"jacobian_u": (ny, nz, nx + 1), "dzdx_u": (ny, nz, nx + 1), "jacobian_v": (ny + 1, nz, nx),
+             "dzdy_v": (ny + 1, nz, nx), "neighbor_terrain": (ny, nx), "mapfac_mx_u": (ny, nx + 1),
+             "mapfac_my_v": (ny + 1, nx), "mapfac_my_u": (ny, nx + 1), "mapfac_mx_v": (ny + 1, nx), "mapfac_mxy": (ny, nx)}
+    metrics = [ones(*shape.get(n, (ny, nz, nx))) for n in _capi.METRIC_FIELDS]
+    h, g = C.c_void_p(), _capi.Grid(nx, ny, nz, 250.0, 1)
+    m = _capi.Metrics(*[C.c_void_p(a.data_ptr()) for a in metrics])
+    _capi.check(lib.hicarw_init_iter_winds(C.byref(g), C.byref(wi.WindOptions().to_c()), C.byref(m), dev, None, C.byref(h)))
+    try:
+        coefs = torch.zeros((15, ny, nz, nx), device="cuda")
+        coefs[0] = torch.rand((ny, nz, nx), device="cuda") + 1
+        _capi.check(lib.hicarw_set_coefs(h, C.c_void_p(coefs.data_ptr()), 1, dev, None), h)
+        back = torch.empty_like(coefs)
+        _capi.check(lib.hicarw_get_coefs(h, C.c_void_p(back.data_ptr()), dev, None), h)
+        assert torch.equal(back, coefs)
+        x = torch.rand((ny + 2, nz + 2, nx + 2), dtype=torch.float64, device="cuda")
+        y = torch.empty_like(x)
+        _capi.check(lib.hicarw_apply_operator(h, C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()), dev, None), h)
+        assert torch.equal(y[1:-1, 1:-1, 1:-1], coefs[0].double() * x[1:-1, 1:-1, 1:-1])
+        _capi.check(lib.hicarw_get_lambda(h, C.c_void_p(y.data_ptr()), dev, None), h)
+        assert not bool(y.any())
+    finally:
+        lib.hicarw_finalize_iter_winds(h)
